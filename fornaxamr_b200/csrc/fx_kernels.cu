@@ -84,8 +84,9 @@ __device__ __forceinline__ void fx_recon_pair(const double (&q)[FxStencil<RECON>
         wl = fx_weno3_face(q[0], q[1], q[2], 0.5);
         wr = fx_weno3_face(q[1], q[2], q[3], -0.5);
     } else {
-        wl = q[1] + 0.5 * fx_mc_slope(q[0], q[1], q[2]);
-        wr = q[2] - 0.5 * fx_mc_slope(q[1], q[2], q[3]);
+        const double d0 = q[1] - q[0], d1 = q[2] - q[1], d2 = q[3] - q[2];
+        wl = q[1] + fx_mc_half(d0, d1);
+        wr = q[2] - fx_mc_half(d1, d2);
     }
 }
 
@@ -107,6 +108,40 @@ __device__ __forceinline__ double fx_stencil_load(const double *p)
         return *p;
     } else {
         return __ldg(p);
+    }
+}
+
+/* A face whose cheap checks did not pass (FxSuspect), evaluated again with
+ * the solver's checks themselves: reports the first that fails, if one does.
+ * Out of line: no sound state comes here.  q0: first stencil cell of
+ * variable 0; bnp: the face's normal field. */
+template <int RECON>
+__device__ __noinline__ void fx_face_recheck(FxErr *err, const double *q0, const double *bnp, int dir, int s,
+    double g, double gL, double gR, int b, int cR)
+{
+    constexpr int NS = FxStencil<RECON>::NS;
+    double WL[9], WR[9], pS[NS], pL, pR;
+    for (int lv = 0; lv < 9; ++lv) {
+        if (lv == FX_B1) {
+            WL[lv] = *bnp;
+            WR[lv] = *bnp;
+            continue;
+        }
+        const double *q = q0 + (size_t)fx_gmap(dir, lv) * kPlane;
+        double qs[NS];
+        for (int n = 0; n < NS; ++n) qs[n] = q[n * s];
+        fx_recon_pair<RECON>(qs, WL[lv], WR[lv]);
+    }
+    for (int n = 0; n < NS; ++n) {
+        pS[n] = fx_pressure(g, q0[(size_t)FX_RHO * kPlane + n * s], q0[(size_t)FX_EINT * kPlane + n * s]);
+    }
+    fx_recon_pair<RECON>(pS, pL, pR);
+    FxErrLocal le;
+    FxBrFree br;
+    FxFaceOut o;
+    fx_riemann_hlld_folded_br(WL, WR, pL, pR, gL, gR, *bnp, o, &le, b, cR, br);
+    if (le.code != 0) {
+        fx_fail(err, le.code, le.block, le.index);
     }
 }
 
@@ -238,18 +273,16 @@ __global__ void __launch_bounds__(TPB, MINB) k_flux(FxDev D, const int *__restri
     const size_t fbase = (size_t)b * FX_FLUX_COUNT(nv) + (size_t)dir * nv * FX_NCELLS;
     const size_t vbase = (size_t)b * FX_VR_COUNT + (size_t)dir * 3 * FX_NCELLS;
     if (MHD) {
-        const double bn = D.Bf[(size_t)b * FX_BF_COUNT + ((size_t)dir * FX_NSTAGES + bfslot) * FX_NFACES +
-            fx_face_idx(dir, i, j, k)];
+        const double *bnp = D.Bf + (size_t)b * FX_BF_COUNT + ((size_t)dir * FX_NSTAGES + bfslot) * FX_NFACES +
+            fx_face_idx(dir, i, j, k);
+        const double bn = *bnp;
+        FxSuspect suspect;
         WL[FX_B1] = bn;
         WR[FX_B1] = bn;
         FxFaceOut o;
         if constexpr (BRM == 0) {
-            FxErrLocal le;
             FxBrFree bf;
-            fx_riemann_hlld_folded_br(WL, WR, pL, pR, gL, gR, bn, o, &le, b, cR, bf);
-            if (le.code != 0) {
-                fx_fail(D.err, le.code, le.block, le.index);
-            }
+            fx_riemann_hlld_folded_br(WL, WR, pL, pR, gL, gR, bn, o, &suspect, b, cR, bf);
         } else {
             fx_riemann_hlld_folded_br(WL, WR, pL, pR, gL, gR, bn, o, D.err, b, cR, br);
             if constexpr (BRM == 1) {
@@ -269,6 +302,11 @@ __global__ void __launch_bounds__(TPB, MINB) k_flux(FxDev D, const int *__restri
         const size_t bvi = (size_t)b * FX_BV_COUNT + (size_t)dir * FX_NCELLS + cR;
         D.bv1[bvi] = o.bv1;
         D.bv2[bvi] = o.bv2;
+        if constexpr (BRM == 0) {
+            if (suspect.any) {
+                fx_face_recheck<RECON>(D.err, Wb + c0, bnp, dir, s, g, gL, gR, b, cR);
+            }
+        }
     } else {
         /* transverse velocity deltas of the theta limiter,
          * prj_flux_velocity_deltas (src/prj_flux.c:1967-2036) */
@@ -1517,7 +1555,7 @@ __global__ void __launch_bounds__(128) k_essprk_blend_cells(FxDev D, const int *
 static inline unsigned fx_blocks(int n, int tpb) { return (unsigned)((n + tpb - 1) / tpb); }
 
 /* launch shapes of the face kernel: {threads per CTA, min CTAs per SM} */
-static const int kFluxShapes[FX_FLUX_VARIANTS][2] = {{128, 4}, {128, 5}, {128, 6}, {256, 2}, {256, 3}, {64, 8}};
+static const int kFluxShapes[FX_FLUX_VARIANTS][2] = {{64, 9}, {64, 8}, {32, 18}, {128, 5}, {64, 12}, {256, 3}};
 
 template <bool MHD, bool FULL, int TPB, int MINB, int RECON = FX_RECON_MC>
 static void launch_flux_shape(const FxDev &D, const int *blist, int nlist, int ndir, int wslot,
@@ -1528,18 +1566,24 @@ static void launch_flux_shape(const FxDev &D, const int *blist, int nlist, int n
     k_flux<MHD, FULL, TPB, MINB, RECON><<<g, TPB, 0, s>>>(D, blist, wslot, bfslot);
 }
 
-/* the autotuner's launch shapes (threads per CTA, minimum CTAs per SM) */
+/* the autotuner's launch shapes (threads per CTA, minimum CTAs per SM).
+ * Microseconds per launch, MC / WENO-Z3 / hydro MC (512, 216, 216 blocks):
+ * 64 x 9  521 / 538 / 146    32 x 18  519 / 542 / 144    64 x 8  562 / 602 / 156
+ * 128 x 5 553 / 558 / 150    64 x 12  551 / 513 / 150    256 x 3 584 / 503 / 165
+ * 18 warps per SM at 96 registers suit MC; WENO-Z3 with its 54 divisions per
+ * face wants the 24 warps of 80 registers; small CTAs leave no half-empty
+ * SM behind a slow warp. */
 template <bool MHD, bool FULL, int RECON>
 static void launch_flux_shapes(const FxDev &D, const int *blist, int nlist, int ndir, int wslot,
     int bfslot, int variant, cudaStream_t s)
 {
     switch (variant) {
-    case 1: launch_flux_shape<MHD, FULL, 128, 5, RECON>(D, blist, nlist, ndir, wslot, bfslot, s); break;
-    case 2: launch_flux_shape<MHD, FULL, 128, 6, RECON>(D, blist, nlist, ndir, wslot, bfslot, s); break;
-    case 3: launch_flux_shape<MHD, FULL, 256, 2, RECON>(D, blist, nlist, ndir, wslot, bfslot, s); break;
-    case 4: launch_flux_shape<MHD, FULL, 256, 3, RECON>(D, blist, nlist, ndir, wslot, bfslot, s); break;
-    case 5: launch_flux_shape<MHD, FULL, 64, 8, RECON>(D, blist, nlist, ndir, wslot, bfslot, s); break;
-    default: launch_flux_shape<MHD, FULL, 128, 4, RECON>(D, blist, nlist, ndir, wslot, bfslot, s); break;
+    case 1: launch_flux_shape<MHD, FULL, 64, 8, RECON>(D, blist, nlist, ndir, wslot, bfslot, s); break;
+    case 2: launch_flux_shape<MHD, FULL, 32, 18, RECON>(D, blist, nlist, ndir, wslot, bfslot, s); break;
+    case 3: launch_flux_shape<MHD, FULL, 128, 5, RECON>(D, blist, nlist, ndir, wslot, bfslot, s); break;
+    case 4: launch_flux_shape<MHD, FULL, 64, 12, RECON>(D, blist, nlist, ndir, wslot, bfslot, s); break;
+    case 5: launch_flux_shape<MHD, FULL, 256, 3, RECON>(D, blist, nlist, ndir, wslot, bfslot, s); break;
+    default: launch_flux_shape<MHD, FULL, 64, 9, RECON>(D, blist, nlist, ndir, wslot, bfslot, s); break;
     }
 }
 
@@ -1551,6 +1595,22 @@ template <bool MHD, bool FULL>
 static void launch_flux_variant(const FxDev &D, const int *blist, int nlist, int ndir, int wslot,
     int bfslot, int variant, cudaStream_t s)
 {
+    if constexpr (FULL) {
+        /* the plain form's launches hold one block, 258 CTAs of 64: two per
+         * SM whatever the shape allows, so the one that does not spill */
+        if (D.recon == FX_RECON_WENO3) {
+            launch_flux_shape<MHD, true, 64, 8, FX_RECON_WENO3>(D, blist, nlist, ndir, wslot, bfslot, s);
+            return;
+        }
+#if FX_NG >= 4
+        if (D.recon == FX_RECON_WENO7) {
+            launch_flux_shape<MHD, true, 64, 8, FX_RECON_WENO7>(D, blist, nlist, ndir, wslot, bfslot, s);
+            return;
+        }
+#endif
+        launch_flux_shape<MHD, true, 64, 8, FX_RECON_MC>(D, blist, nlist, ndir, wslot, bfslot, s);
+        return;
+    }
     if (D.recon == FX_RECON_WENO3) {
         launch_flux_shapes<MHD, FULL, FX_RECON_WENO3>(D, blist, nlist, ndir, wslot, bfslot, variant, s);
         return;

@@ -22,7 +22,7 @@
 #ifdef __CUDACC__
 #define FX_HD __host__ __device__ __forceinline__
 #else
-#define FX_HD static inline
+#define FX_HD inline
 #endif
 
 #define FX_BS 16

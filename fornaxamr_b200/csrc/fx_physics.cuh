@@ -95,6 +95,113 @@ FX_HD void fx_fail(FxErrLocal *err, int code, int block, int index)
     err->index = first ? index : err->index;
 }
 
+/* The high word of a double: sign, exponent and the leading 20 bits. */
+FX_HD int fx_hi(double x)
+{
+#ifdef __CUDA_ARCH__
+    return __double2hiint(x);
+#else
+    long long b;
+    __builtin_memcpy(&b, &x, sizeof(b));
+    return (int)(b >> 32);
+#endif
+}
+
+/* positive, normal and finite, by one integer comparison */
+FX_HD bool fx_pos_normal(double x) { return (unsigned)(fx_hi(x) - 0x00100000) < 0x7fe00000u; }
+
+/* Collects whether any check of a face might fail.  A check costs the face
+ * kernel one to four FP64 operations, about thirty per face; here each is an
+ * integer comparison of high words that a failing value never passes and a
+ * sound state always does (a few more values do not pass: subnormals,
+ * nearly cancelled differences).  The rare face that does not pass is
+ * evaluated again with the checks themselves. */
+struct FxSuspect {
+    bool any = false;
+};
+
+/* |x| against 1e-14 (|a| + |b| + 1): x at least 2^-42 of the largest of |a|,
+ * |b| and 1 passes (3 * 1e-14 < 2^-44), unless that sum may overflow */
+FX_HD bool fx_may_cancel(double x, double a, double b)
+{
+    const int ha = fx_hi(a) & 0x7fffffff;
+    const int hb = fx_hi(b) & 0x7fffffff;
+    int m = ha > hb ? ha : hb;
+    m = m > 0x3ff00000 ? m : 0x3ff00000;
+    return (fx_hi(x) & 0x7fffffff) < m - (42 << 20) || m >= 0x7fd00000;
+}
+
+/* the solver's checks; E: FxErr, FxErrLocal (the checks themselves) or
+ * FxSuspect */
+template <class E>
+FX_HD void fx_check_state(E *err, double rho, double p, double gamma, int blk, int idx)
+{
+    if (rho <= 0.0) fx_fail(err, FX_ERR_HLLD_RHO, blk, idx);
+    if (p <= 0.0) fx_fail(err, FX_ERR_HLLD_P, blk, idx);
+    if (gamma <= 0.0) fx_fail(err, FX_ERR_HLLD_GAMMA, blk, idx);
+}
+
+FX_HD void fx_check_state(FxSuspect *err, double rho, double p, double gamma, int, int)
+{
+    err->any |= !fx_pos_normal(rho) || !fx_pos_normal(p) || !fx_pos_normal(gamma);
+}
+
+/* a negative discriminant beyond round-off */
+template <class E>
+FX_HD void fx_check_disc(E *err, double disc, double x, int blk, int idx)
+{
+    if (disc < -1.0e-12 * x * x) fx_fail(err, FX_ERR_HLLD_DISC, blk, idx);
+}
+
+FX_HD void fx_check_disc(FxSuspect *err, double, double, int, int) { err->any = true; }
+
+template <class E>
+FX_HD void fx_check_cf(E *err, double cf2, int blk, int idx)
+{
+    if (cf2 < 0.0 || !isfinite(cf2)) fx_fail(err, FX_ERR_HLLD_CF, blk, idx);
+}
+
+FX_HD void fx_check_cf(FxSuspect *err, double cf2, int, int)
+{
+    err->any |= (unsigned)fx_hi(cf2) >= 0x7ff00000u;
+}
+
+template <class E>
+FX_HD void fx_check_order(E *err, double SL, double SR, int blk, int idx)
+{
+    if (!(SL < SR)) fx_fail(err, FX_ERR_HLLD_ORDER, blk, idx);
+}
+
+FX_HD void fx_check_order(FxSuspect *err, double SL, double SR, int, int) { err->any |= !(SL < SR); }
+
+/* |x| <= 1e-14 (|a| + |b| + 1) */
+template <class E>
+FX_HD void fx_check_cancel(E *err, int code, double x, double a, double b, int blk, int idx)
+{
+    if (fabs(x) <= 1.0e-14 * (fabs(a) + fabs(b) + 1.0)) fx_fail(err, code, blk, idx);
+}
+
+FX_HD void fx_check_cancel(FxSuspect *err, int, double x, double a, double b, int, int)
+{
+    err->any |= fx_may_cancel(x, a, b);
+}
+
+template <class E>
+FX_HD void fx_check_star_rho(E *err, double rho, int blk, int idx)
+{
+    if (rho <= 0.0 || !isfinite(rho)) fx_fail(err, FX_ERR_HLLD_STARRHO, blk, idx);
+}
+
+FX_HD void fx_check_star_rho(FxSuspect *err, double rho, int, int) { err->any |= !fx_pos_normal(rho); }
+
+template <class E>
+FX_HD void fx_check_weights(E *err, double sum, int blk, int idx)
+{
+    if (sum <= 0.0) fx_fail(err, FX_ERR_HLLD_DSTAR, blk, idx);
+}
+
+FX_HD void fx_check_weights(FxSuspect *err, double sum, int, int) { err->any |= !fx_pos_normal(sum); }
+
 /* ------------------------------------------------------------------------ */
 /* Branch policies.  The solvers below take their data-dependent decisions  */
 /* (limiter candidate, wave-speed argument, fan region, upwind direction)   */
@@ -166,6 +273,27 @@ FX_HD double fx_mc_slope(double qm, double q0, double qp)
     mx = mx > c2 ? mx : c2;
     const double slope = sl > 0.0 ? mn : mx;
     return (sl * sr > 0.0) ? slope : 0.0;
+}
+
+/* 0.5 * fx_mc_slope from the two differences sl = q0 - qm, sr = qp - q0, the
+ * same double with 8 FP64 operations instead of 14 (the face kernel's time
+ * goes with its FP64 operations, and it takes 18 slopes per face):
+ * - the candidates are halved, sl, c1 / 2 and sr for 2 sl, c1 and 2 sr, so no
+ *   doubling and no final halving; scaling by 2 is exact here, since
+ *   sl * sr > 0 puts |c1| far above the subnormals;
+ * - with sl * sr > 0 the candidates have one sign, so the smallest magnitude
+ *   is the minimum of a positive triple and the maximum of a negative one:
+ *   one chain of two comparisons instead of two chains and their selection;
+ * - 0.5 * (sr - sl) is exact, so the addition to sl takes it in one FMA.
+ * Otherwise the slope is +0.0 whatever the candidates are.  (An infinite
+ * difference beside one of at least 2^1023 is the one input where the two
+ * differ.) */
+FX_HD double fx_mc_half(double sl, double sr)
+{
+    const double h1 = 0.5 * fma(0.5, sr - sl, sl);
+    double h = fabs(sl) < fabs(h1) ? sl : h1;
+    h = fabs(h) < fabs(sr) ? h : sr;
+    return (sl * sr > 0.0) ? h : 0.0;
 }
 
 /* fx_mc_slope with its selection through a policy: candidate 0, 1, 2 (c0,
@@ -493,8 +621,7 @@ FX_HD double fx_hlld_state_u(const FxHlldState &s, int v)
 /* prj_hlld_fill_flux, src/prj_riemann.c:96-115 (component v) */
 FX_HD double fx_hlld_state_f(const FxHlldState &s, int v)
 {
-    const double b2 = s.bx * s.bx + s.by * s.by + s.bz * s.bz;
-    const double pt = s.p + 0.5 * b2;
+    const double pt = s.pt; /* p + 0.5 (bx^2 + by^2 + bz^2), taken with the state */
     switch (v) {
     case 0: return s.rho * s.vx;
     case 1: return s.rho * s.vx * s.vx + pt - s.bx * s.bx;
@@ -527,9 +654,7 @@ FX_HD void fx_hlld_state_e(const double *w, double p, double gamma, double bn,
     s.p = p;
     s.gamma = gamma;
     s.ye = w[FX_YE];
-    if (s.rho <= 0.0) fx_fail(err, FX_ERR_HLLD_RHO, blk, idx);
-    if (s.p <= 0.0) fx_fail(err, FX_ERR_HLLD_P, blk, idx);
-    if (s.gamma <= 0.0) fx_fail(err, FX_ERR_HLLD_GAMMA, blk, idx);
+    fx_check_state(err, s.rho, s.p, s.gamma, blk, idx);
     const double kinetic = 0.5 * s.rho * (s.vx * s.vx + s.vy * s.vy + s.vz * s.vz);
     const double magnetic = 0.5 * (s.bx * s.bx + s.by * s.by + s.bz * s.bz);
     s.e = s.rho * w[FX_EINT] + kinetic + magnetic;
@@ -552,15 +677,11 @@ FX_HD double fx_hlld_fast_speed_br(const FxHlldState &s, E *err, int blk, int id
     const double b2_rho = fx_div(s.bx * s.bx + s.by * s.by + s.bz * s.bz, s.rho);
     double disc = (a2 + b2_rho) * (a2 + b2_rho) - 4.0 * a2 * bx2_rho;
     if (br.bit(k, disc < 0.0)) {
-        if (disc < -1.0e-12 * (a2 + b2_rho) * (a2 + b2_rho)) {
-            fx_fail(err, FX_ERR_HLLD_DISC, blk, idx);
-        }
+        fx_check_disc(err, disc, a2 + b2_rho, blk, idx);
         disc = 0.0;
     }
     const double cf2 = 0.5 * (a2 + b2_rho + sqrt(disc));
-    if (cf2 < 0.0 || !isfinite(cf2)) {
-        fx_fail(err, FX_ERR_HLLD_CF, blk, idx);
-    }
+    fx_check_cf(err, cf2, blk, idx);
     return sqrt(cf2);
 }
 
@@ -570,25 +691,21 @@ FX_HD double fx_hlld_fast_speed(const FxHlldState &s, FxErr *err, int blk, int i
     return fx_hlld_fast_speed_br(s, err, blk, idx, br, 0);
 }
 
-/* prj_hlld_outer_star, src/prj_riemann.c:185-232; the degenerate-denominator
- * branch is decision bit k */
+/* prj_hlld_outer_star, src/prj_riemann.c:185-232, with alpha = S - s.vx and
+ * ra = s.rho * alpha given; the degenerate-denominator branch is decision
+ * bit k */
 template <class BR, class E = FxErr>
-FX_HD void fx_hlld_outer_star_br(const FxHlldState &s, double S, double SM,
+FX_HD void fx_hlld_outer_star_br(const FxHlldState &s, double alpha, double ra, double S, double SM,
     double pt_star, FxHlldStar &st, E *err, int blk, int idx, BR &br, int k)
 {
-    const double alpha = S - s.vx;
     const double smdiff = S - SM;
-    if (fabs(smdiff) <= 1.0e-14 * (fabs(S) + fabs(SM) + 1.0)) {
-        fx_fail(err, FX_ERR_HLLD_OUTER, blk, idx);
-    }
-    st.rho = fx_div(s.rho * alpha, smdiff);
-    if (st.rho <= 0.0 || !isfinite(st.rho)) {
-        fx_fail(err, FX_ERR_HLLD_STARRHO, blk, idx);
-    }
+    fx_check_cancel(err, FX_ERR_HLLD_OUTER, smdiff, S, SM, blk, idx);
+    st.rho = fx_div(ra, smdiff);
+    fx_check_star_rho(err, st.rho, blk, idx);
     st.vx = SM;
     st.bx = s.bx;
     st.ye = s.ye;
-    const double denom = s.rho * alpha * smdiff - s.bx * s.bx;
+    const double denom = ra * smdiff - s.bx * s.bx;
     if (br.bit(k, fabs(denom) < FX_HLLD_SMALL * pt_star)) {
         st.vy = s.vy;
         st.vz = s.vz;
@@ -596,7 +713,7 @@ FX_HD void fx_hlld_outer_star_br(const FxHlldState &s, double S, double SM,
         st.bz = s.bz;
     } else {
         const double sm_diff_vx_over_denom = fx_div(SM - s.vx, denom);
-        const double mag_factor = fx_div(s.rho * alpha * alpha - s.bx * s.bx, denom);
+        const double mag_factor = fx_div(ra * alpha - s.bx * s.bx, denom);
         st.vy = s.vy - s.bx * s.by * sm_diff_vx_over_denom;
         st.vz = s.vz - s.bx * s.bz * sm_diff_vx_over_denom;
         st.by = s.by * mag_factor;
@@ -611,42 +728,8 @@ FX_HD void fx_hlld_outer_star(const FxHlldState &s, double S, double SM,
     double pt_star, FxHlldStar &st, FxErr *err, int blk, int idx)
 {
     FxBrFree br;
-    fx_hlld_outer_star_br(s, S, SM, pt_star, st, err, blk, idx, br, 0);
-}
-
-/* prj_hlld_double_star_one, src/prj_riemann.c:234-282 */
-FX_HD void fx_hlld_double_star(const FxHlldStar &left, const FxHlldStar &right,
-    double bx, bool right_side, FxHlldStar &ss, FxErr *err, int blk, int idx)
-{
-    const double sqrt_l = sqrt(left.rho);
-    const double sqrt_r = sqrt(right.rho);
-    if (sqrt_l + sqrt_r <= 0.0) {
-        fx_fail(err, FX_ERR_HLLD_DSTAR, blk, idx);
-    }
-    const double inv_sum = 1.0 / (sqrt_l + sqrt_r);
-    const double sign_bx = bx < 0.0 ? -1.0 : 1.0;
-    const double vy_ss = (sqrt_l * left.vy + sqrt_r * right.vy +
-        (right.by - left.by) * sign_bx) * inv_sum;
-    const double vz_ss = (sqrt_l * left.vz + sqrt_r * right.vz +
-        (right.bz - left.bz) * sign_bx) * inv_sum;
-    const double by_ss = (sqrt_l * right.by + sqrt_r * left.by +
-        sqrt_l * sqrt_r * (right.vy - left.vy) * sign_bx) * inv_sum;
-    const double bz_ss = (sqrt_l * right.bz + sqrt_r * left.bz +
-        sqrt_l * sqrt_r * (right.vz - left.vz) * sign_bx) * inv_sum;
-    const double vbdot_ss = (right_side ? right.vx : left.vx) * bx + vy_ss * by_ss + vz_ss * bz_ss;
-    if (!right_side) {
-        const double vbdot_l = left.vx * bx + left.vy * left.by + left.vz * left.bz;
-        ss = left;
-        ss.e = left.e - sqrt_l * sign_bx * (vbdot_l - vbdot_ss);
-    } else {
-        const double vbdot_r = right.vx * bx + right.vy * right.by + right.vz * right.bz;
-        ss = right;
-        ss.e = right.e + sqrt_r * sign_bx * (vbdot_r - vbdot_ss);
-    }
-    ss.vy = vy_ss;
-    ss.vz = vz_ss;
-    ss.by = by_ss;
-    ss.bz = bz_ss;
+    const double alpha = S - s.vx;
+    fx_hlld_outer_star_br(s, alpha, s.rho * alpha, S, SM, pt_star, st, err, blk, idx, br, 0);
 }
 
 /* Face outputs of the MHD solver: local-frame flux (9), face velocity (3)
@@ -669,110 +752,23 @@ FX_HD void fx_face_outputs(double vx, double vy, double vz,
     o.bv2 = bx * vy - by * vx;
 }
 
-/* prj_riemann_hlld, src/prj_riemann.c:321-440 */
-static __device__ __noinline__ void fx_riemann_hlld(const double *WL, const double *WR,
-    double pL, double pR, double gL, double gR, double bn, FxFaceOut &o,
-    FxErr *err, int blk, int idx)
-{
-    FxHlldState L, R;
-    fx_hlld_state(WL, pL, gL, bn, L, err, blk, idx);
-    fx_hlld_state(WR, pR, gR, bn, R, err, blk, idx);
-    const double cfL = fx_hlld_fast_speed(L, err, blk, idx);
-    const double cfR = fx_hlld_fast_speed(R, err, blk, idx);
-    const double SL = fx_min(L.vx - cfL, R.vx - cfR);
-    const double SR = fx_max(L.vx + cfL, R.vx + cfR);
-    if (!(SL < SR)) {
-        fx_fail(err, FX_ERR_HLLD_ORDER, blk, idx);
-    }
-    if (0.0 <= SL) {
-        for (int v = 0; v < 9; ++v) o.F[v] = fx_hlld_state_f(L, v);
-        fx_face_outputs(L.vx, L.vy, L.vz, L.bx, L.by, L.bz, o);
-        return;
-    }
-    if (SR <= 0.0) {
-        for (int v = 0; v < 9; ++v) o.F[v] = fx_hlld_state_f(R, v);
-        fx_face_outputs(R.vx, R.vy, R.vz, R.bx, R.by, R.bz, o);
-        return;
-    }
-    const double denom = R.rho * (SR - R.vx) - L.rho * (SL - L.vx);
-    if (fabs(denom) <= 1.0e-14 *
-        (fabs(R.rho * (SR - R.vx)) + fabs(L.rho * (SL - L.vx)) + 1.0)) {
-        fx_fail(err, FX_ERR_HLLD_DENOM, blk, idx);
-    }
-    const double SM = (R.rho * R.vx * (SR - R.vx) -
-        L.rho * L.vx * (SL - L.vx) + (L.pt - R.pt)) / denom;
-    const double pt_star_l = L.pt + L.rho * (SL - L.vx) * (SM - L.vx);
-    const double pt_star_r = R.pt + R.rho * (SR - R.vx) * (SM - R.vx);
-    const double pt_star = 0.5 * (pt_star_l + pt_star_r);
-    if (pt_star <= 0.0 || !isfinite(pt_star)) {
-        /* HLL fallback, src/prj_riemann.c:392-409 */
-        const double inv = 1.0 / (SR - SL);
-        double Uh[9];
-        for (int v = 0; v < 9; ++v) {
-            const double lf = fx_hlld_state_f(L, v);
-            const double rf = fx_hlld_state_f(R, v);
-            const double lu = fx_hlld_state_u(L, v);
-            const double ru = fx_hlld_state_u(R, v);
-            o.F[v] = (SR * lf - SL * rf + SL * SR * (ru - lu)) * inv;
-            Uh[v] = (SR * ru - SL * lu + lf - rf) * inv;
-        }
-        const double rho = Uh[0];
-        fx_face_outputs(Uh[1] / rho, Uh[2] / rho, Uh[3] / rho, Uh[6], Uh[7], Uh[8], o);
-        return;
-    }
-    const bool bn_small = (0.5 * bn * bn < FX_HLLD_SMALL * pt_star);
-    FxHlldStar Ls, Rs, ss;
-    if (0.0 <= SM) {
-        fx_hlld_outer_star(L, SL, SM, pt_star, Ls, err, blk, idx);
-        const double SLs = SM - fabs(bn) / sqrt(Ls.rho);
-        if (0.0 <= SLs || bn_small) {
-            for (int v = 0; v < 9; ++v) {
-                o.F[v] = fx_hlld_state_f(L, v) + SL * (fx_hlld_u(Ls, v) - fx_hlld_state_u(L, v));
-            }
-            fx_face_outputs(Ls.vx, Ls.vy, Ls.vz, Ls.bx, Ls.by, Ls.bz, o);
-        } else {
-            fx_hlld_outer_star(R, SR, SM, pt_star, Rs, err, blk, idx);
-            fx_hlld_double_star(Ls, Rs, bn, false, ss, err, blk, idx);
-            for (int v = 0; v < 9; ++v) {
-                const double us = fx_hlld_u(Ls, v);
-                o.F[v] = fx_hlld_state_f(L, v) + SL * (us - fx_hlld_state_u(L, v)) +
-                    SLs * (fx_hlld_u(ss, v) - us);
-            }
-            fx_face_outputs(ss.vx, ss.vy, ss.vz, ss.bx, ss.by, ss.bz, o);
-        }
-    } else {
-        fx_hlld_outer_star(R, SR, SM, pt_star, Rs, err, blk, idx);
-        const double SRs = SM + fabs(bn) / sqrt(Rs.rho);
-        if (SRs <= 0.0 || bn_small) {
-            for (int v = 0; v < 9; ++v) {
-                o.F[v] = fx_hlld_state_f(R, v) + SR * (fx_hlld_u(Rs, v) - fx_hlld_state_u(R, v));
-            }
-            fx_face_outputs(Rs.vx, Rs.vy, Rs.vz, Rs.bx, Rs.by, Rs.bz, o);
-        } else {
-            fx_hlld_outer_star(L, SL, SM, pt_star, Ls, err, blk, idx);
-            fx_hlld_double_star(Ls, Rs, bn, true, ss, err, blk, idx);
-            for (int v = 0; v < 9; ++v) {
-                const double us = fx_hlld_u(Rs, v);
-                o.F[v] = fx_hlld_state_f(R, v) + SR * (us - fx_hlld_state_u(R, v)) +
-                    SRs * (fx_hlld_u(ss, v) - us);
-            }
-            fx_face_outputs(ss.vx, ss.vy, ss.vz, ss.bx, ss.by, ss.bz, o);
-        }
-    }
-}
-
-/* Same solver with the left and right star branches folded into one code
- * path.  With `left` = (0 <= SM), the reference's two branches
- * (src/prj_riemann.c:413-438) are the same sequence of operations applied to
- * the near state N = left ? L : R and the far state F = left ? R : L:
+/* prj_riemann_hlld, src/prj_riemann.c:321-440, with its left and right star
+ * branches folded into one code path.  With `left` = (0 <= SM), the
+ * reference's two branches (src/prj_riemann.c:413-438) are the same sequence
+ * of operations applied to the near state N = left ? L : R and the far state
+ * F = left ? R : L:
  *   Ns = outer_star(N, S_N); a = |bn|/sqrt(Ns.rho); S_Ns = SM -/+ a;
  *   single star if (left ? 0 <= S_Ns : S_Ns <= 0) || bn_small;
  *   else Fs = outer_star(F, S_F) and the double star of (Ls, Rs), whose
  *   energy update e = Ns.e -/+ sqrt(Ns.rho) sign(bn) (vb_Ns - vb_ss) uses the
  *   near star in both branches (its normal velocity is SM on either side).
  * Selecting operands and choosing between x - t and x + t are exact, so the
- * result is bit-identical to fx_riemann_hlld; warps whose faces straddle
- * SM = 0 no longer execute both branches. */
+ * result is the reference's bit for bit; warps whose faces straddle SM = 0 do
+ * not execute both branches.  What L and R have computed before the selection
+ * (S - vx, rho (S - vx), the total pressure) is selected, not computed again.
+ * The single-star flux comes first and the double star adds its jump to it;
+ * rho, vx and ye do not jump across the Alfven wave, so three of those
+ * terms are S_Ns times +0.0. */
 template <class BR, class E = FxErr>
 FX_HD void fx_riemann_hlld_folded_br(const double *WL, const double *WR,
     double pL, double pR, double gL, double gR, double bn, FxFaceOut &o,
@@ -787,9 +783,7 @@ FX_HD void fx_riemann_hlld_folded_br(const double *WL, const double *WR,
     const double bL = L.vx + cfL, bR = R.vx + cfR;
     const double SL = br.bit(FX_BR_SL, aL < aR) ? aL : aR;   /* fx_min */
     const double SR = br.bit(FX_BR_SR, bL > bR) ? bL : bR;   /* fx_max */
-    if (!(SL < SR)) {
-        fx_fail(err, FX_ERR_HLLD_ORDER, blk, idx);
-    }
+    fx_check_order(err, SL, SR, blk, idx);
     const bool super_l = br.bit(FX_BR_SUPER_L, 0.0 <= SL);
     if (super_l || br.bit(FX_BR_SUPER_R, SR <= 0.0)) {
         const FxHlldState &X = super_l ? L : R;
@@ -798,17 +792,16 @@ FX_HD void fx_riemann_hlld_folded_br(const double *WL, const double *WR,
         fx_face_outputs(X.vx, X.vy, X.vz, X.bx, X.by, X.bz, o);
         return;
     }
-    const double denom = R.rho * (SR - R.vx) - L.rho * (SL - L.vx);
-    if (fabs(denom) <= 1.0e-14 *
-        (fabs(R.rho * (SR - R.vx)) + fabs(L.rho * (SL - L.vx)) + 1.0)) {
-        fx_fail(err, FX_ERR_HLLD_DENOM, blk, idx);
-    }
-    const double SM = fx_div(R.rho * R.vx * (SR - R.vx) -
-        L.rho * L.vx * (SL - L.vx) + (L.pt - R.pt), denom);
-    const double pt_star_l = L.pt + L.rho * (SL - L.vx) * (SM - L.vx);
-    const double pt_star_r = R.pt + R.rho * (SR - R.vx) * (SM - R.vx);
+    const double alL = SL - L.vx, alR = SR - R.vx;
+    const double raL = L.rho * alL, raR = R.rho * alR;
+    const double denom = raR - raL;
+    fx_check_cancel(err, FX_ERR_HLLD_DENOM, denom, raR, raL, blk, idx);
+    const double SM = fx_div(R.rho * R.vx * alR - L.rho * L.vx * alL + (L.pt - R.pt), denom);
+    const double pt_star_l = L.pt + raL * (SM - L.vx);
+    const double pt_star_r = R.pt + raR * (SM - R.vx);
     const double pt_star = 0.5 * (pt_star_l + pt_star_r);
-    if (br.bit(FX_BR_HLL, pt_star <= 0.0 || !isfinite(pt_star))) {
+    /* pt_star <= 0 or not finite; a positive normal value passes at once */
+    if (br.bit(FX_BR_HLL, !fx_pos_normal(pt_star) && (pt_star <= 0.0 || !isfinite(pt_star)))) {
         const double inv = fx_div(1.0, SR - SL);
         double Uh[9];
 #pragma unroll
@@ -829,23 +822,25 @@ FX_HD void fx_riemann_hlld_folded_br(const double *WL, const double *WR,
     const FxHlldState N = left ? L : R;
     const double SN = left ? SL : SR;
     FxHlldStar Ns;
-    fx_hlld_outer_star_br(N, SN, SM, pt_star, Ns, err, blk, idx, br, FX_BR_DEGEN_N);
+    fx_hlld_outer_star_br(N, left ? alL : alR, left ? raL : raR, SN, SM, pt_star, Ns, err, blk, idx, br,
+        FX_BR_DEGEN_N);
     const double sqN = sqrt(Ns.rho);
     const double a = fx_div(fabs(bn), sqN);
     const double SNs = left ? SM - a : SM + a;
     const bool single = br.bit(FX_BR_SINGLE, (left ? (0.0 <= SNs) : (SNs <= 0.0)) || bn_small);
-    if (single) {
 #pragma unroll
-        for (int v = 0; v < 9; ++v) {
-            o.F[v] = fx_hlld_state_f(N, v) + SN * (fx_hlld_u(Ns, v) - fx_hlld_state_u(N, v));
-        }
+    for (int v = 0; v < 9; ++v) {
+        o.F[v] = fx_hlld_state_f(N, v) + SN * (fx_hlld_u(Ns, v) - fx_hlld_state_u(N, v));
+    }
+    if (single) {
         fx_face_outputs(Ns.vx, Ns.vy, Ns.vz, Ns.bx, Ns.by, Ns.bz, o);
         return;
     }
     const FxHlldState Fr = left ? R : L;
     const double SF = left ? SR : SL;
     FxHlldStar Fs;
-    fx_hlld_outer_star_br(Fr, SF, SM, pt_star, Fs, err, blk, idx, br, FX_BR_DEGEN_F);
+    fx_hlld_outer_star_br(Fr, left ? alR : alL, left ? raR : raL, SF, SM, pt_star, Fs, err, blk, idx, br,
+        FX_BR_DEGEN_F);
     const FxHlldStar Ls = left ? Ns : Fs;
     const FxHlldStar Rs = left ? Fs : Ns;
     /* prj_hlld_double_star_one, src/prj_riemann.c:234-282 */
@@ -853,9 +848,7 @@ FX_HD void fx_riemann_hlld_folded_br(const double *WL, const double *WR,
     const double sqF = sqrt(Fs.rho);
     const double sqrt_l = left ? sqN : sqF;
     const double sqrt_r = left ? sqF : sqN;
-    if (sqrt_l + sqrt_r <= 0.0) {
-        fx_fail(err, FX_ERR_HLLD_DSTAR, blk, idx);
-    }
+    fx_check_weights(err, sqrt_l + sqrt_r, blk, idx);
     const double inv_sum = fx_div(1.0, sqrt_l + sqrt_r);
     const double sign_bx = br.bit(FX_BR_BNEG, bn < 0.0) ? -1.0 : 1.0;
     FxHlldStar ss = Ns;
@@ -865,13 +858,14 @@ FX_HD void fx_riemann_hlld_folded_br(const double *WL, const double *WR,
     ss.bz = (sqrt_l * Rs.bz + sqrt_r * Ls.bz + sqrt_l * sqrt_r * (Rs.vz - Ls.vz) * sign_bx) * inv_sum;
     const double vbdot_ss = Ns.vx * bn + ss.vy * ss.by + ss.vz * ss.bz;
     const double vbdot_n = Ns.vx * bn + Ns.vy * Ns.by + Ns.vz * Ns.bz;
-    const double t = (left ? sqrt_l : sqrt_r) * sign_bx * (vbdot_n - vbdot_ss);
+    const double t = sqN * sign_bx * (vbdot_n - vbdot_ss);
     ss.e = left ? Ns.e - t : Ns.e + t;
+    const double z = SNs * 0.0;
 #pragma unroll
     for (int v = 0; v < 9; ++v) {
-        const double us = fx_hlld_u(Ns, v);
-        o.F[v] = fx_hlld_state_f(N, v) + SN * (us - fx_hlld_state_u(N, v)) +
-            SNs * (fx_hlld_u(ss, v) - us);
+        const double jump = v == 0 || v == 1 || v == 5 || v == 6
+            ? z : SNs * (fx_hlld_u(ss, v) - fx_hlld_u(Ns, v));
+        o.F[v] = o.F[v] + jump;
     }
     fx_face_outputs(ss.vx, ss.vy, ss.vz, ss.bx, ss.by, ss.bz, o);
 }
@@ -895,93 +889,76 @@ FX_HD double fx_theta_limiter(double cfmax, double du, double dv, double dw)
     return fx_min(1.0, theta_r * theta_r);
 }
 
-/* prj_riemann_state, src/prj_riemann.c:1433-1492 (hydro: 6 components) */
-FX_HD void fx_hllc_state(const double *W, double p, double gamma,
-    double *U, double *F, double &cs)
+/* one side of the hydro solver: prj_riemann_state, src/prj_riemann.c:1433-1492 */
+struct FxHllcSide {
+    double rho, v1, v2, v3, eint, ye, p, mom; /* mom = rho * v1 */
+};
+
+FX_HD void fx_hllc_side(const double *W, double p, FxHllcSide &s)
 {
-    const double rho = W[FX_RHO];
-    const double v1 = W[FX_V1];
-    const double v2 = W[FX_V2];
-    const double v3 = W[FX_V3];
-    const double eint = W[FX_EINT];
-    const double etot = rho * eint + 0.5 * rho * (v1 * v1 + v2 * v2 + v3 * v3);
-    U[0] = rho;
-    U[1] = rho * v1;
-    U[2] = rho * v2;
-    U[3] = rho * v3;
-    U[4] = etot;
-    U[5] = rho * W[FX_YE];
-    cs = sqrt(gamma * p / rho);
-    F[0] = rho * v1;
-    F[1] = rho * v1 * v1 + p;
-    F[2] = rho * v1 * v2;
-    F[3] = rho * v1 * v3;
-    F[4] = (etot + p) * v1;
-    F[5] = rho * W[FX_YE] * v1;
+    s.rho = W[FX_RHO];
+    s.v1 = W[FX_V1];
+    s.v2 = W[FX_V2];
+    s.v3 = W[FX_V3];
+    s.eint = W[FX_EINT];
+    s.ye = W[FX_YE];
+    s.p = p;
+    s.mom = s.rho * s.v1;
 }
 
-/* prj_riemann_hllc, src/prj_riemann.c:1494-1599; F[6], vface[3] out */
-static __device__ __noinline__ void fx_riemann_hllc(const double *WL, const double *WR,
+/* prj_riemann_hllc, src/prj_riemann.c:1494-1599; F[6], vface[3] out.  The
+ * reference's four outcomes (left or right state, left or right star) are
+ * one flux of the side X that the fan selects, plus the star's jump where the
+ * fan is subsonic: the same operations on selected operands, so a warp whose
+ * faces differ runs one path and only the selected side's flux and total
+ * energy are evaluated. */
+FX_HD void fx_riemann_hllc(const double *WL, const double *WR,
     double pL, double pR, double gL, double gR, double du, double dv, double dw,
     double *flux, double *v_face)
 {
-    double UL[6], UR[6], FL[6], FR[6], Ustar[6];
-    double csL, csR;
-    fx_hllc_state(WL, pL, gL, UL, FL, csL);
-    fx_hllc_state(WR, pR, gR, UR, FR, csR);
-    const double SL = fx_min(WL[FX_V1] - csL, WR[FX_V1] - csR);
-    const double SR = fx_max(WL[FX_V1] + csL, WR[FX_V1] + csR);
+    FxHllcSide L, R;
+    fx_hllc_side(WL, pL, L);
+    fx_hllc_side(WR, pR, R);
+    const double csL = sqrt(gL * pL / L.rho);
+    const double csR = sqrt(gR * pR / R.rho);
+    const double SL = fx_min(L.v1 - csL, R.v1 - csR);
+    const double SR = fx_max(L.v1 + csL, R.v1 + csR);
     const double cfmax = fx_max(csL, csR);
     const double theta = fx_theta_limiter(cfmax, du, dv, dw);
-    const double SM = (theta * (pR - pL) +
-        UL[1] * (SL - WL[FX_V1]) -
-        UR[1] * (SR - WR[FX_V1])) /
-        (UL[0] * (SL - WL[FX_V1]) -
-            UR[0] * (SR - WR[FX_V1]));
-    if (0.0 <= SL) {
-        for (int v = 0; v < 6; ++v) flux[v] = FL[v];
-        v_face[0] = WL[FX_V1];
-        v_face[1] = WL[FX_V2];
-        v_face[2] = WL[FX_V3];
-        return;
-    }
-    if (SR <= 0.0) {
-        for (int v = 0; v < 6; ++v) flux[v] = FR[v];
-        v_face[0] = WR[FX_V1];
-        v_face[1] = WR[FX_V2];
-        v_face[2] = WR[FX_V3];
+    const double aL = SL - L.v1;
+    const double aR = SR - R.v1;
+    const double raL = L.rho * aL;
+    const double raR = R.rho * aR;
+    const double SM = (theta * (pR - pL) + L.mom * aL - R.mom * aR) / (raL - raR);
+    const bool super_l = 0.0 <= SL;
+    const bool super_r = SR <= 0.0;
+    const bool left = super_l || (!super_r && 0.0 <= SM);
+    const FxHllcSide X = left ? L : R;
+    const double S = left ? SL : SR;
+    const double ra = left ? raL : raR;
+    const double E = X.rho * X.eint + 0.5 * X.rho * (X.v1 * X.v1 + X.v2 * X.v2 + X.v3 * X.v3);
+    const double rye = X.rho * X.ye;
+    flux[0] = X.mom;
+    flux[1] = X.mom * X.v1 + X.p;
+    flux[2] = X.mom * X.v2;
+    flux[3] = X.mom * X.v3;
+    flux[4] = (E + X.p) * X.v1;
+    flux[5] = rye * X.v1;
+    v_face[0] = X.v1;
+    v_face[1] = X.v2;
+    v_face[2] = X.v3;
+    if (super_l || super_r) {
         return;
     }
     v_face[0] = SM;
-    if (0.0 <= SM) {
-        v_face[1] = WL[FX_V2];
-        v_face[2] = WL[FX_V3];
-        for (int v = 0; v < 6; ++v) Ustar[v] = UL[v];
-        const double rho_star = UL[0] * (SL - WL[FX_V1]) / (SL - SM);
-        Ustar[0] = rho_star;
-        Ustar[1] = rho_star * SM;
-        Ustar[2] = rho_star * WL[FX_V2];
-        Ustar[3] = rho_star * WL[FX_V3];
-        const double e_over_rho = UL[4] / UL[0] +
-            (SM - WL[FX_V1]) * (SM + pL / (UL[0] * (SL - WL[FX_V1])));
-        Ustar[4] = rho_star * e_over_rho;
-        Ustar[5] = rho_star * WL[FX_YE];
-        for (int v = 0; v < 6; ++v) flux[v] = FL[v] + SL * (Ustar[v] - UL[v]);
-    } else {
-        v_face[1] = WR[FX_V2];
-        v_face[2] = WR[FX_V3];
-        for (int v = 0; v < 6; ++v) Ustar[v] = UR[v];
-        const double rho_star = UR[0] * (SR - WR[FX_V1]) / (SR - SM);
-        Ustar[0] = rho_star;
-        Ustar[1] = rho_star * SM;
-        Ustar[2] = rho_star * WR[FX_V2];
-        Ustar[3] = rho_star * WR[FX_V3];
-        const double e_over_rho = UR[4] / UR[0] +
-            (SM - WR[FX_V1]) * (SM + pR / (UR[0] * (SR - WR[FX_V1])));
-        Ustar[4] = rho_star * e_over_rho;
-        Ustar[5] = rho_star * WR[FX_YE];
-        for (int v = 0; v < 6; ++v) flux[v] = FR[v] + SR * (Ustar[v] - UR[v]);
-    }
+    const double rho_star = ra / (S - SM);
+    const double e_over_rho = E / X.rho + (SM - X.v1) * (SM + X.p / ra);
+    flux[0] = flux[0] + S * (rho_star - X.rho);
+    flux[1] = flux[1] + S * (rho_star * SM - X.mom);
+    flux[2] = flux[2] + S * (rho_star * X.v2 - X.rho * X.v2);
+    flux[3] = flux[3] + S * (rho_star * X.v3 - X.rho * X.v3);
+    flux[4] = flux[4] + S * (rho_star * e_over_rho - E);
+    flux[5] = flux[5] + S * (rho_star * X.ye - rye);
 }
 
 /* ------------------------------------------------------------------------ */
