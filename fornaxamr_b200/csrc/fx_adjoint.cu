@@ -227,13 +227,13 @@ __global__ void __launch_bounds__(128) k_adj_emf(FxAdjDev A, const int *__restri
     const int cells[4] = {fx_lidx(e[0], e[1], e[2]), 0, 0, 0};
     const int c0 = cells[0];
     const int cc[4] = {c0, c0 - su, c0 - su - sr, c0 - sr};
-    const double *vrr = A.vr + (size_t)b * FX_VR_COUNT + (size_t)right * 3 * FX_NCELLS;
-    const double *vru = A.vr + (size_t)b * FX_VR_COUNT + (size_t)up * 3 * FX_NCELLS;
+    const double *vrr = A.vn + (size_t)b * FX_VN_COUNT + (size_t)right * FX_NCELLS;
+    const double *vru = A.vn + (size_t)b * FX_VN_COUNT + (size_t)up * FX_NCELLS;
     double vn[4];
-    vn[0] = vrr[fx_bidx_cell(3, right, cc[0])];
-    vn[1] = vru[fx_bidx_cell(3, up, cc[0])];
-    vn[2] = vrr[fx_bidx_cell(3, right, cc[1])];
-    vn[3] = vru[fx_bidx_cell(3, up, cc[3])];
+    vn[0] = vrr[cc[0]];
+    vn[1] = vru[cc[0]];
+    vn[2] = vrr[cc[1]];
+    vn[3] = vru[cc[3]];
     double fb[4] = {0, 0, 0, 0}, cb[4] = {0, 0, 0, 0};
     fxa_emf_upwind_vjp(vn, eb, fb, cb);
     double *b1r = A.bvb1 + (size_t)b * FX_BV_COUNT + (size_t)right * FX_NCELLS;

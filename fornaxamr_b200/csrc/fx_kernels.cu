@@ -295,11 +295,15 @@ __global__ void __launch_bounds__(TPB, MINB) k_flux(FxDev D, const int *__restri
         for (int lv = 0; lv < (FULL ? 9 : 6); ++lv) {
             D.flux[fbase + fx_bidx(9, fx_gmap(dir, lv), i, j, k)] = o.F[lv];
         }
-#pragma unroll
-        for (int m = 0; m < (FULL ? 3 : 1); ++m) {
-            D.vr[vbase + fx_bidx(3, (dir + m) % 3, i, j, k)] = o.v[m];
-        }
         const size_t bvi = (size_t)b * FX_BV_COUNT + (size_t)dir * FX_NCELLS + cR;
+        if constexpr (FULL) {
+#pragma unroll
+            for (int m = 0; m < 3; ++m) {
+                D.vr[vbase + fx_bidx(3, (dir + m) % 3, i, j, k)] = o.v[m];
+            }
+        } else {
+            D.vn[bvi] = o.v[0];
+        }
         D.bv1[bvi] = o.bv1;
         D.bv2[bvi] = o.bv2;
         if constexpr (BRM == 0) {
@@ -329,9 +333,13 @@ __global__ void __launch_bounds__(TPB, MINB) k_flux(FxDev D, const int *__restri
         for (int lv = 0; lv < 6; ++lv) {
             D.flux[fbase + fx_bidx(6, fx_gmap(dir, lv), i, j, k)] = F[lv];
         }
+        if constexpr (FULL) {
 #pragma unroll
-        for (int m = 0; m < (FULL ? 3 : 1); ++m) {
-            D.vr[vbase + fx_bidx(3, (dir + m) % 3, i, j, k)] = v[m];
+            for (int m = 0; m < 3; ++m) {
+                D.vr[vbase + fx_bidx(3, (dir + m) % 3, i, j, k)] = v[m];
+            }
+        } else {
+            D.vn[(size_t)b * FX_VN_COUNT + (size_t)dir * FX_NCELLS + cR] = v[0];
         }
     }
 }
@@ -353,6 +361,9 @@ __device__ __forceinline__ double fx_cell_emf(const double *Wb, int dir, int c)
     return bA * vB - bB * vA;
 }
 
+/* FULL: the plain form, normal velocities in vr; else the batched form
+ * on a short list, in vn */
+template <bool FULL>
 __global__ void __launch_bounds__(128) k_emf_edges(FxDev D, const int *__restrict__ blist, int wslot, int bfslot)
 {
     if (D.ctl->skip) {
@@ -385,8 +396,6 @@ __global__ void __launch_bounds__(128) k_emf_edges(FxDev D, const int *__restric
     const double *Wb = D.W + (size_t)b * FX_W_COUNT(9) + (size_t)wslot * FX_NCELLS;
     const double *bv1r = D.bv1 + (size_t)b * FX_BV_COUNT + (size_t)right * FX_NCELLS;
     const double *bv2u = D.bv2 + (size_t)b * FX_BV_COUNT + (size_t)up * FX_NCELLS;
-    const double *vrr = D.vr + (size_t)b * FX_VR_COUNT + (size_t)right * 3 * FX_NCELLS;
-    const double *vru = D.vr + (size_t)b * FX_VR_COUNT + (size_t)up * 3 * FX_NCELLS;
     double f[4], c[4], vn[4];
     /* face0 = e (right-normal), face1 = e (up-normal), face2 = e - up
      * (right-normal), face3 = e - right (up-normal) */
@@ -398,10 +407,21 @@ __global__ void __launch_bounds__(128) k_emf_edges(FxDev D, const int *__restric
     c[1] = fx_cell_emf(Wb, dir, c1);
     c[2] = fx_cell_emf(Wb, dir, c2);
     c[3] = fx_cell_emf(Wb, dir, c3);
-    vn[0] = vrr[fx_bidx_cell(3, right, c0)];
-    vn[1] = vru[fx_bidx_cell(3, up, c0)];
-    vn[2] = vrr[fx_bidx_cell(3, right, c1)];
-    vn[3] = vru[fx_bidx_cell(3, up, c3)];
+    if constexpr (FULL) {
+        const double *vrr = D.vr + (size_t)b * FX_VR_COUNT + (size_t)right * 3 * FX_NCELLS;
+        const double *vru = D.vr + (size_t)b * FX_VR_COUNT + (size_t)up * 3 * FX_NCELLS;
+        vn[0] = vrr[fx_bidx_cell(3, right, c0)];
+        vn[1] = vru[fx_bidx_cell(3, up, c0)];
+        vn[2] = vrr[fx_bidx_cell(3, right, c1)];
+        vn[3] = vru[fx_bidx_cell(3, up, c3)];
+    } else {
+        const double *vrr = D.vn + (size_t)b * FX_VN_COUNT + (size_t)right * FX_NCELLS;
+        const double *vru = D.vn + (size_t)b * FX_VN_COUNT + (size_t)up * FX_NCELLS;
+        vn[0] = vrr[c0];
+        vn[1] = vru[c0];
+        vn[2] = vrr[c1];
+        vn[3] = vru[c3];
+    }
     const int eidx = fx_edge_idx(dir, e[0], e[1], e[2]);
     for (int n = 0; n < 4; ++n) {
         if (!isfinite(f[n]) || !isfinite(c[n]) || !isfinite(vn[n])) {
@@ -471,181 +491,224 @@ __global__ void __launch_bounds__(128) k_emf_edges(FxDev D, const int *__restric
     D.emf[(size_t)b * FX_EMF_COUNT + (size_t)dir * FX_NEDGES + eidx] = emf;
 }
 
-/* One CTA per (block, chunk of edge layers along i).  For each layer i the
- * CTA first evaluates, once per cell of plane i (j, k in [-1, 16]), the
- * three cell-centred EMF components and the artificial eta (the reference
- * precomputes the same per-cell grids, src/prj_timeint.c:313-338 and
- * prj_timeint_mhd_fill_eta_mask), keeping planes i - 1 and i in shared
- * memory; then its threads sweep the layer's edges of all three directions
- * (an edge along x at layer i reads plane i only, edges along y and z read
- * planes i - 1 and i).  The face EMFs and normal velocities of an edge come
- * straight from global memory (each is read by two edges, coalesced along
- * k).  Arithmetic of prj_timeint_mhd_update_emf (src/prj_timeint.c:292-413). */
-/* edge layers per CTA: measured flat between 1 and 17 layers (0.178-0.189
- * ms for 512 blocks), 2 the fastest */
-constexpr int kEmfChunk = 2;
-constexpr int kEmfChunks = (FX_BS + 1 + kEmfChunk - 1) / kEmfChunk;
+/* One CTA per (block, chunk of edge layers along i), one thread per node
+ * (j, k) in [-1, 16]^2, marching along i.  A thread loads its cell (velocity,
+ * field, density) and its three faces (two EMF products and the normal
+ * velocity each) once per plane; values of the nodes j - 1 and k - 1 come through shared memory (two
+ * buffers, one barrier per plane), values of plane i - 1 from its own
+ * registers.  The cell EMFs are evaluated once per cell, as the reference's
+ * per-cell grids are (src/prj_timeint.c:313-338); arithmetic of
+ * prj_timeint_mhd_update_emf (src/prj_timeint.c:292-413).
+ * Bound by memory latency and DRAM: 512 blocks 123 us, 528 MB at 4.3 TB/s
+ * (compulsory about 475 MB), against 163 us and 729 MB for the kernel that
+ * staged the cells of two layers and had each edge gather its eight face
+ * values with the velocities in three-component tiles.  80 registers, 22
+ * warps per SM; three CTAs per SM spill (177 us); loading one plane ahead
+ * into registers spills, prefetching it into L2 or L1 measured 128-129 us.
+ * The resistive term, zero in nearly every run, is a second pass, so that the
+ * first carries nothing for it. */
+constexpr int kEmfNodes = (FX_BS + 2) * (FX_BS + 2);
+constexpr int kEmfThreads = (kEmfNodes + 31) / 32 * 32;
 
-__global__ void __launch_bounds__(256, 5) k_emf(FxDev D, const int *__restrict__ blist, int wslot, int bfslot)
+/* shared planes: cell EMFs, then what an edge reads from the node j - 1
+ * (bv1 z, vr z, bv2 x, vr x) or k - 1 (bv2 y, vr y, bv1 x, vr x) */
+enum { FX_EP_E1, FX_EP_E2, FX_EP_E3, FX_EP_BV1Z, FX_EP_VRZ, FX_EP_BV2X, FX_EP_VRX, FX_EP_BV2Y, FX_EP_VRY,
+    FX_EP_BV1X, FX_EP_COUNT };
+
+/* maximum artificial eta of an edge's four cells (src/prj_timeint.c:265-290) */
+__device__ __noinline__ double fx_edge_eta(FxErr *err, const double *Wb, int b, int eidx, int c0, int su, int sr)
+{
+    const int cells[4] = {c0, c0 - su, c0 - su - sr, c0 - sr};
+    double eta = 0.0;
+    for (int n = 0; n < 4; ++n) {
+        const double ce = fx_cell_eta(Wb[(size_t)FX_RHO * kPlane + cells[n]], Wb[(size_t)FX_YE * kPlane + cells[n]]);
+        if (!isfinite(ce) || ce < 0.0) {
+            fx_fail(err, FX_ERR_ETA, b, eidx);
+        }
+        if (ce > eta) {
+            eta = ce;
+        }
+    }
+    return eta;
+}
+
+/* curl B term of one edge, src/prj_mhd.c:682-709 */
+__device__ __noinline__ double fx_edge_curl_b(const double *bf, const FxBlockDev &B, int bfslot, int dir, int i, int j, int k)
+{
+    const double *b1 = bf + (size_t)(0 * FX_NSTAGES + bfslot) * FX_NFACES;
+    const double *b2 = bf + (size_t)(1 * FX_NSTAGES + bfslot) * FX_NFACES;
+    const double *b3 = bf + (size_t)(2 * FX_NSTAGES + bfslot) * FX_NFACES;
+    if (dir == 0) {
+        return (b3[fx_face_idx(2, i, j, k)] - b3[fx_face_idx(2, i, j - 1, k)]) / B.dx[1] -
+            (b2[fx_face_idx(1, i, j, k)] - b2[fx_face_idx(1, i, j, k - 1)]) / B.dx[2];
+    }
+    if (dir == 1) {
+        return (b1[fx_face_idx(0, i, j, k)] - b1[fx_face_idx(0, i, j, k - 1)]) / B.dx[2] -
+            (b3[fx_face_idx(2, i, j, k)] - b3[fx_face_idx(2, i - 1, j, k)]) / B.dx[0];
+    }
+    return (b2[fx_face_idx(1, i, j, k)] - b2[fx_face_idx(1, i - 1, j, k)]) / B.dx[0] -
+        (b1[fx_face_idx(0, i, j, k)] - b1[fx_face_idx(0, i, j - 1, k)]) / B.dx[1];
+}
+
+/* infinite or NaN: the high word's exponent is all ones */
+__device__ __forceinline__ bool fx_nonfinite(double x) { return (fx_hi(x) & 0x7ff00000) == 0x7ff00000; }
+
+/* one edge from its four face EMFs, cell EMFs and normal velocities.  A
+ * non-finite face EMF makes the sum of the four non-finite, so the result's
+ * check covers it. */
+template <int DIR>
+__device__ __forceinline__ void fx_edge_store(const FxDev &D, int b, int i, int j, int k, const double (&f)[4],
+    const double (&c)[4], const double (&vn)[4])
+{
+    const int eidx = fx_edge_idx(DIR, i, j, k);
+    const double emf = fx_emf_upwind(f, c, vn);
+    if (fx_nonfinite(emf) || fx_nonfinite(vn[0]) || fx_nonfinite(vn[1]) || fx_nonfinite(vn[2]) || fx_nonfinite(vn[3])) {
+        fx_fail(D.err, FX_ERR_EMF_NONFINITE, b, eidx);
+    }
+    D.emf[(size_t)b * FX_EMF_COUNT + (size_t)DIR * FX_NEDGES + eidx] = emf;
+}
+
+/* the resistive term of one edge, added to the EMF its thread has stored */
+__device__ __noinline__ void fx_edge_resist(const FxDev &D, int b, int wslot, int bfslot, int dir, int i, int j, int k)
+{
+    const int eidx = fx_edge_idx(dir, i, j, k);
+    const double *Wb = D.W + (size_t)b * FX_W_COUNT(9) + (size_t)wslot * FX_NCELLS;
+    const double eta = D.mhd_eta + fx_edge_eta(D.err, Wb, b, eidx, fx_lidx(i, j, k), fx_axis_stride((dir + 1) % 3),
+        fx_axis_stride((dir + 2) % 3));
+    if (eta == 0.0) {
+        return;
+    }
+    double *e = D.emf + (size_t)b * FX_EMF_COUNT + (size_t)dir * FX_NEDGES + eidx;
+    const double emf = *e + eta * fx_edge_curl_b(D.Bf + (size_t)b * FX_BF_COUNT, D.blk[b], bfslot, dir, i, j, k);
+    if (!isfinite(emf)) {
+        fx_fail(D.err, FX_ERR_EMF_NONFINITE, b, eidx);
+    }
+    *e = emf;
+}
+
+__global__ void __launch_bounds__(kEmfThreads, 2) k_emf(const __grid_constant__ FxDev D, const int *__restrict__ blist, int wslot,
+    int bfslot, int nchunk)
 {
     if (D.ctl->skip) {
         return;
     }
-    constexpr int P2 = FX_PBS * FX_PBS;          /* cells per plane */
-    /* [plane parity][E1, E2, E3, eta][in-plane cell] */
-    __shared__ double cq[2][4][P2];
+    extern __shared__ double emf_planes[]; /* [2][FX_EP_COUNT][kEmfNodes] */
+    constexpr int ROW = FX_BS + 2;
+    constexpr int N = kEmfNodes;
     const int b = blist[blockIdx.y];
-    const int l0 = blockIdx.x * kEmfChunk;
-    const int l1 = min(l0 + kEmfChunk, FX_BS + 1);
-    const double *Wb = D.W + (size_t)b * FX_W_COUNT(9) + (size_t)wslot * FX_NCELLS;
+    const int l0 = (FX_BS + 1) * (int)blockIdx.x / nchunk;
+    const int l1 = (FX_BS + 1) * ((int)blockIdx.x + 1) / nchunk;
+    const int t = threadIdx.x;
+    const bool node = t < N;
+    const int jj = t / ROW;
+    const int j = jj - 1;
+    const int k = t - jj * ROW - 1;
+    const bool inner = node && j >= 0 && k >= 0; /* the node's edges exist */
 
-    /* cell quantities of plane i into buffer (i + 2) & 1 */
-    auto cells = [&](int i) {
-        double (*q)[P2] = cq[(i + 2) & 1];
-        for (int t = threadIdx.x; t < (FX_BS + 2) * (FX_BS + 2); t += blockDim.x) {
-            const int jj = t / (FX_BS + 2);
-            const int kk = t - jj * (FX_BS + 2);
-            const int c = fx_lidx(i, jj - 1, kk - 1);
-            const double b1 = Wb[(size_t)FX_B1 * kPlane + c];
-            const double b2 = Wb[(size_t)FX_B2 * kPlane + c];
-            const double b3 = Wb[(size_t)FX_B3 * kPlane + c];
-            const double v1 = Wb[(size_t)FX_V1 * kPlane + c];
-            const double v2 = Wb[(size_t)FX_V2 * kPlane + c];
-            const double v3 = Wb[(size_t)FX_V3 * kPlane + c];
+    /* plane offset 0 is plane i = 0 */
+    const int c0 = fx_lidx(0, node ? j : 0, node ? k : 0);
+    constexpr int PL = FX_PBS * FX_PBS;
+    const double *w = D.W + (size_t)b * FX_W_COUNT(9) + (size_t)wslot * FX_NCELLS + c0;
+    const double *p1 = D.bv1 + (size_t)b * FX_BV_COUNT + c0;
+    const double *p2 = D.bv2 + (size_t)b * FX_BV_COUNT + c0;
+    const double *pv = D.vn + (size_t)b * FX_VN_COUNT + c0;
+
+    /* values of plane i - 1 */
+    double pE2 = 0.0, pE3 = 0.0, pE2k = 0.0, pE3j = 0.0, pbv1y = 0.0, pvry = 0.0, pbv2z = 0.0, pvrz = 0.0;
+    bool resist = D.mhd_eta != 0.0;
+    for (int i = l0 - 1; i < l1; ++i) {
+        double *sp = emf_planes + (i & 1) * (FX_EP_COUNT * N) + t;
+        double bv1y = 0.0, bv2z = 0.0;
+        bool heavy = false;
+        if (node) {
+            const double *q = w + i * PL;
+            const double rho = q[(size_t)FX_RHO * kPlane];
+            const double v1 = q[(size_t)FX_V1 * kPlane], v2 = q[(size_t)FX_V2 * kPlane], v3 = q[(size_t)FX_V3 * kPlane];
+            const double b1 = q[(size_t)FX_B1 * kPlane], b2 = q[(size_t)FX_B2 * kPlane], b3 = q[(size_t)FX_B3 * kPlane];
+            double bv1x = 0.0, bv2x = 0.0, vrx = 0.0, bv2y = 0.0, vry = 0.0, bv1z = 0.0, vrz = 0.0;
+            if (i >= 0) {
+                bv1x = p1[i * PL];
+                bv2x = p2[i * PL];
+                vrx = pv[i * PL];
+            }
+            if (j >= 0) {
+                bv1y = p1[FX_NCELLS + i * PL];
+                bv2y = p2[FX_NCELLS + i * PL];
+                vry = pv[FX_NCELLS + i * PL];
+            }
+            if (k >= 0) {
+                bv1z = p1[2 * FX_NCELLS + i * PL];
+                bv2z = p2[2 * FX_NCELLS + i * PL];
+                vrz = pv[2 * FX_NCELLS + i * PL];
+            }
             /* prj_timeint_mhd_cell_emf_all, src/prj_timeint.c:171-176 */
-            const double e1 = b2 * v3 - b3 * v2;
-            const double e2 = b3 * v1 - b1 * v3;
-            const double e3 = b1 * v2 - b2 * v1;
-            if (!isfinite(e1) || !isfinite(e2) || !isfinite(e3)) {
-                fx_fail(D.err, FX_ERR_EMF_NONFINITE, b, c);
+            const double E1 = b2 * v3 - b3 * v2;
+            const double E2 = b3 * v1 - b1 * v3;
+            const double E3 = b1 * v2 - b2 * v1;
+            if (fx_nonfinite(E1) || fx_nonfinite(E2) || fx_nonfinite(E3)) {
+                fx_fail(D.err, FX_ERR_EMF_NONFINITE, b, c0 + i * PL);
             }
-            const double eta = fx_cell_eta(Wb[(size_t)FX_RHO * kPlane + c], Wb[(size_t)FX_YE * kPlane + c]);
-            if (!isfinite(eta) || eta < 0.0) {
-                fx_fail(D.err, FX_ERR_ETA, b, c);
-            }
-            const int pc = (jj - 1 + FX_NG) * FX_PBS + (kk - 1 + FX_NG);
-            q[0][pc] = e1;
-            q[1][pc] = e2;
-            q[2][pc] = e3;
-            q[3][pc] = eta;
+            /* the artificial eta is zero up to this density (fx_cell_eta) */
+            heavy = rho > FX_ETA_RHO_FLOOR;
+            sp[FX_EP_E1 * N] = E1;
+            sp[FX_EP_E2 * N] = E2;
+            sp[FX_EP_E3 * N] = E3;
+            sp[FX_EP_BV1Z * N] = bv1z;
+            sp[FX_EP_VRZ * N] = vrz;
+            sp[FX_EP_BV2X * N] = bv2x;
+            sp[FX_EP_VRX * N] = vrx;
+            sp[FX_EP_BV2Y * N] = bv2y;
+            sp[FX_EP_VRY * N] = vry;
+            sp[FX_EP_BV1X * N] = bv1x;
         }
-    };
-
-    constexpr int N0 = (FX_BS + 1) * (FX_BS + 1);   /* x edges of a layer (i < 16) */
-    constexpr int N1 = FX_BS * (FX_BS + 1);         /* y edges */
-    constexpr int N2 = (FX_BS + 1) * FX_BS;         /* z edges */
-    cells(l0 - 1);
-    for (int i0 = l0; i0 < l1; ++i0) {
-        cells(i0);
-        __syncthreads();
-        const int cur = (i0 + 2) & 1;   /* buffer of plane i0; plane i0 - 1 in 1 - cur */
-        const int n0 = i0 < FX_BS ? N0 : 0;
-        const int ntot = n0 + N1 + N2;
-        for (int t = threadIdx.x; t < ntot; t += blockDim.x) {
-            int dir, u = t;
-            if (u < n0) {
-                dir = 0;
-            } else if ((u -= n0) < N1) {
-                dir = 1;
-            } else {
-                u -= N1;
-                dir = 2;
-            }
-            /* k runs over 17 edges for x and y edges, 16 for z edges:
-             * constant divisors */
-            int j, k;
-            if (dir == 2) {
-                j = u / FX_BS;
-                k = u - j * FX_BS;
-            } else {
-                j = u / (FX_BS + 1);
-                k = u - j * (FX_BS + 1);
-            }
-            const int up = (dir + 1) % 3;
-            const int right = (dir + 2) % 3;
-            /* the four cells: c0 = e, c1 = e - up, c2 = e - up - right,
-             * c3 = e - right; buffer and in-plane index */
-            const int pc = (j + FX_NG) * FX_PBS + (k + FX_NG);
-            int cb[4], ci[4];
-            if (dir == 0) {
-                cb[0] = cur; ci[0] = pc;
-                cb[1] = cur; ci[1] = pc - FX_PBS;
-                cb[2] = cur; ci[2] = pc - FX_PBS - 1;
-                cb[3] = cur; ci[3] = pc - 1;
-            } else if (dir == 1) {
-                cb[0] = cur; ci[0] = pc;
-                cb[1] = cur; ci[1] = pc - 1;
-                cb[2] = 1 - cur; ci[2] = pc - 1;
-                cb[3] = 1 - cur; ci[3] = pc;
-            } else {
-                cb[0] = cur; ci[0] = pc;
-                cb[1] = 1 - cur; ci[1] = pc;
-                cb[2] = 1 - cur; ci[2] = pc - FX_PBS;
-                cb[3] = cur; ci[3] = pc - FX_PBS;
-            }
-            double c[4];
-            /* edge resistivity: run-time eta plus the maximum artificial eta
-             * of the four incident cells (src/prj_timeint.c:265-290) */
-            double eta_cells = 0.0;
-#pragma unroll
-            for (int n = 0; n < 4; ++n) {
-                c[n] = cq[cb[n]][dir][ci[n]];
-                const double ce = cq[cb[n]][3][ci[n]];
-                if (ce > eta_cells) {
-                    eta_cells = ce;
-                }
-            }
-            const int c0 = fx_lidx(i0, j, k);
-            const int c1 = c0 - fx_axis_stride(up);
-            const int c3 = c0 - fx_axis_stride(right);
-            const double *bv1r = D.bv1 + (size_t)b * FX_BV_COUNT + (size_t)right * FX_NCELLS;
-            const double *bv2u = D.bv2 + (size_t)b * FX_BV_COUNT + (size_t)up * FX_NCELLS;
-            const double *vrr = D.vr + (size_t)b * FX_VR_COUNT + (size_t)right * 3 * FX_NCELLS;
-            const double *vru = D.vr + (size_t)b * FX_VR_COUNT + (size_t)up * 3 * FX_NCELLS;
-            double f[4], vn[4];
-            f[0] = bv1r[c0];
-            f[1] = bv2u[c0];
-            f[2] = bv1r[c1];
-            f[3] = bv2u[c3];
-            vn[0] = vrr[fx_bidx_cell(3, right, c0)];
-            vn[1] = vru[fx_bidx_cell(3, up, c0)];
-            vn[2] = vrr[fx_bidx_cell(3, right, c1)];
-            vn[3] = vru[fx_bidx_cell(3, up, c3)];
-            const int eidx = fx_edge_idx(dir, i0, j, k);
-            for (int n = 0; n < 4; ++n) {
-                if (!isfinite(f[n]) || !isfinite(vn[n])) {
-                    fx_fail(D.err, FX_ERR_EMF_NONFINITE, b, eidx);
-                }
-            }
-            const double eta = D.mhd_eta + eta_cells;
-            double emf = fx_emf_upwind(f, c, vn);
-            if (eta != 0.0) {
-                /* resistive term, src/prj_mhd.c:682-709 */
-                const double *bf = D.Bf + (size_t)b * FX_BF_COUNT;
-                const double *b1 = bf + (size_t)(0 * FX_NSTAGES + bfslot) * FX_NFACES;
-                const double *b2 = bf + (size_t)(1 * FX_NSTAGES + bfslot) * FX_NFACES;
-                const double *b3 = bf + (size_t)(2 * FX_NSTAGES + bfslot) * FX_NFACES;
-                const FxBlockDev &B = D.blk[b];
-                const int i = i0;
-                double curl_b;
-                if (dir == 0) {
-                    curl_b = (b3[fx_face_idx(2, i, j, k)] - b3[fx_face_idx(2, i, j - 1, k)]) / B.dx[1] -
-                        (b2[fx_face_idx(1, i, j, k)] - b2[fx_face_idx(1, i, j, k - 1)]) / B.dx[2];
-                } else if (dir == 1) {
-                    curl_b = (b1[fx_face_idx(0, i, j, k)] - b1[fx_face_idx(0, i, j, k - 1)]) / B.dx[2] -
-                        (b3[fx_face_idx(2, i, j, k)] - b3[fx_face_idx(2, i - 1, j, k)]) / B.dx[0];
-                } else {
-                    curl_b = (b2[fx_face_idx(1, i, j, k)] - b2[fx_face_idx(1, i - 1, j, k)]) / B.dx[0] -
-                        (b1[fx_face_idx(0, i, j, k)] - b1[fx_face_idx(0, i, j - 1, k)]) / B.dx[1];
-                }
-                emf += eta * curl_b;
-            }
-            if (!isfinite(emf)) {
-                fx_fail(D.err, FX_ERR_EMF_NONFINITE, b, eidx);
-            }
-            D.emf[(size_t)b * FX_EMF_COUNT + (size_t)dir * FX_NEDGES + eidx] = emf;
+        resist |= __syncthreads_or(heavy) != 0;
+        if (!inner) {
+            continue;
         }
-        __syncthreads(); /* plane i0 - 1's buffer takes plane i0 + 1 next */
+        const double E2 = sp[FX_EP_E2 * N], E3 = sp[FX_EP_E3 * N];
+        const double E2k = sp[FX_EP_E2 * N - 1], E3j = sp[FX_EP_E3 * N - ROW];
+        const double vry = sp[FX_EP_VRY * N], vrz = sp[FX_EP_VRZ * N];
+        if (i >= l0) {
+            /* face0 = e (right-normal), face1 = e (up-normal), face2 = e - up
+             * (right-normal), face3 = e - right (up-normal); cells e, e - up,
+             * e - up - right, e - right */
+            if (i < FX_BS) {
+                const double f[4] = {sp[FX_EP_BV1Z * N], sp[FX_EP_BV2Y * N], sp[FX_EP_BV1Z * N - ROW], sp[FX_EP_BV2Y * N - 1]};
+                const double c[4] = {sp[FX_EP_E1 * N], sp[FX_EP_E1 * N - ROW], sp[FX_EP_E1 * N - ROW - 1], sp[FX_EP_E1 * N - 1]};
+                const double vn[4] = {vrz, vry, sp[FX_EP_VRZ * N - ROW], sp[FX_EP_VRY * N - 1]};
+                fx_edge_store<0>(D, b, i, j, k, f, c, vn);
+            }
+            if (j < FX_BS) {
+                const double f[4] = {sp[FX_EP_BV1X * N], bv2z, sp[FX_EP_BV1X * N - 1], pbv2z};
+                const double c[4] = {E2, E2k, pE2k, pE2};
+                const double vn[4] = {sp[FX_EP_VRX * N], vrz, sp[FX_EP_VRX * N - 1], pvrz};
+                fx_edge_store<1>(D, b, i, j, k, f, c, vn);
+            }
+            if (k < FX_BS) {
+                const double f[4] = {bv1y, sp[FX_EP_BV2X * N], pbv1y, sp[FX_EP_BV2X * N - ROW]};
+                const double c[4] = {E3, pE3, pE3j, E3j};
+                const double vn[4] = {vry, sp[FX_EP_VRX * N], pvry, sp[FX_EP_VRX * N - ROW]};
+                fx_edge_store<2>(D, b, i, j, k, f, c, vn);
+            }
+        }
+        pE2 = E2;
+        pE3 = E3;
+        pE2k = E2k;
+        pE3j = E3j;
+        pbv1y = bv1y;
+        pvry = vry;
+        pbv2z = bv2z;
+        pvrz = vrz;
+    }
+    /* resistive edges (a run-time eta, or a cell above the density floor in
+     * these planes) in a second pass, so that the pass above carries nothing
+     * for them */
+    if (resist && inner) {
+        for (int i = l0; i < l1; ++i) {
+            if (i < FX_BS) fx_edge_resist(D, b, wslot, bfslot, 0, i, j, k);
+            if (j < FX_BS) fx_edge_resist(D, b, wslot, bfslot, 1, i, j, k);
+            if (k < FX_BS) fx_edge_resist(D, b, wslot, bfslot, 2, i, j, k);
+        }
     }
 }
 
@@ -717,9 +780,10 @@ __global__ void __launch_bounds__(128) k_bf_update(FxDev D, const int *__restric
 /* STAGE 1 / 2: the RK2 stages; STAGE 0: the stage-1 arithmetic written in
  * place to slot 0 with the field of Bf slot 0 (an eSSPRK substep,
  * prj_timeint_eSSPRK_step, src/prj_timeint.c:2484-2508) */
-template <bool MHD, int STAGE>
-__global__ void __launch_bounds__(128) k_cell_update(FxDev D, const int *__restrict__ blist,
-    int gravity, int store_rhs)
+/* FULL: the plain form (face velocities in vr, rhs stored), else the batched
+ * one */
+template <bool MHD, int STAGE, bool FULL>
+__global__ void __launch_bounds__(128) k_cell_update(FxDev D, const int *__restrict__ blist, int gravity)
 {
     if (D.ctl->skip) {
         return;
@@ -773,18 +837,31 @@ __global__ void __launch_bounds__(128) k_cell_update(FxDev D, const int *__restr
         const double g2 = g[FX_NCELLS + c];
         const double g3 = g[2 * FX_NCELLS + c];
         const double rho = Ws[(size_t)FX_RHO * kPlane + c];
-        const double *vr = D.vr + (size_t)b * FX_VR_COUNT;
         rhs[FX_V1] += rho * g1;
         rhs[FX_V2] += rho * g2;
         rhs[FX_V3] += rho * g3;
-        const double v_avg1 = (vr[fx_bidx(3, 0, i, j, k)] + vr[fx_bidx(3, 0, i + 1, j, k)]) * 0.5;
-        const double v_avg2 = (vr[3 * FX_NCELLS + fx_bidx(3, 1, i, j, k)] +
-            vr[3 * FX_NCELLS + fx_bidx(3, 1, i, j + 1, k)]) * 0.5;
-        const double v_avg3 = (vr[6 * FX_NCELLS + fx_bidx(3, 2, i, j, k)] +
-            vr[6 * FX_NCELLS + fx_bidx(3, 2, i, j, k + 1)]) * 0.5;
+        double vf[3][2];
+        if constexpr (FULL) {
+            const double *vr = D.vr + (size_t)b * FX_VR_COUNT;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                vf[d][0] = vr[d * 3 * FX_NCELLS + fx_bidx(3, d, i, j, k)];
+                vf[d][1] = vr[d * 3 * FX_NCELLS + fx_bidx(3, d, i + (d == 0), j + (d == 1), k + (d == 2))];
+            }
+        } else {
+            const double *vn = D.vn + (size_t)b * FX_VN_COUNT + c;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                vf[d][0] = vn[d * FX_NCELLS];
+                vf[d][1] = vn[d * FX_NCELLS + fx_axis_stride(d)];
+            }
+        }
+        const double v_avg1 = (vf[0][0] + vf[0][1]) * 0.5;
+        const double v_avg2 = (vf[1][0] + vf[1][1]) * 0.5;
+        const double v_avg3 = (vf[2][0] + vf[2][1]) * 0.5;
         rhs[FX_ETOT] += rho * (v_avg1 * g1 + v_avg2 * g2 + v_avg3 * g3);
     }
-    if (store_rhs) {
+    if constexpr (FULL) {
         double *r = D.rhs + (size_t)b * FX_RHS_COUNT(nv);
 #pragma unroll
         for (int v = 0; v < nv; ++v) {
@@ -1735,15 +1812,46 @@ void fx_launch_cell_field_active(const FxDev &D, const int *blist, int nlist, cu
     k_cell_field_active<<<dim3(fx_blocks(NC, 256), nlist), 256, 0, s>>>(D, blist);
 }
 
-void fx_launch_emf(const FxDev &D, const int *blist, int nlist, int wslot, int bfslot, cudaStream_t s)
+/* the batched form's face arrays written in the reference's layout, for a
+ * caller that goes on with the plain entry points or downloads them */
+__global__ void __launch_bounds__(256) k_expand_faces(FxDev D, const int *__restrict__ blist)
 {
-    if (nlist <= 0) return;
-    if (nlist < 16) {
-        const int ne = 3 * FX_BS * (FX_BS + 1) * (FX_BS + 1);
-        k_emf_edges<<<dim3(fx_blocks(ne, 128), nlist), 128, 0, s>>>(D, blist, wslot, bfslot);
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= FX_NCELLS) {
         return;
     }
-    k_emf<<<dim3(kEmfChunks, nlist), 256, 0, s>>>(D, blist, wslot, bfslot);
+    const int b = blist[blockIdx.y];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        D.vr[(size_t)b * FX_VR_COUNT + d * 3 * FX_NCELLS + fx_bidx_cell(3, d, t)] =
+            D.vn[(size_t)b * FX_VN_COUNT + d * FX_NCELLS + t];
+    }
+}
+
+void fx_launch_expand_faces(const FxDev &D, const int *blist, int nlist, cudaStream_t s)
+{
+    if (nlist <= 0) return;
+    k_expand_faces<<<dim3(fx_blocks(FX_NCELLS, 256), nlist), 256, 0, s>>>(D, blist);
+}
+
+void fx_launch_emf(const FxDev &D, const int *blist, int nlist, int wslot, int bfslot, int full, cudaStream_t s)
+{
+    if (nlist <= 0) return;
+    if (full || nlist < 16) {
+        const dim3 grid(fx_blocks(3 * FX_BS * (FX_BS + 1) * (FX_BS + 1), 128), nlist);
+        if (full) k_emf_edges<true><<<grid, 128, 0, s>>>(D, blist, wslot, bfslot);
+        else k_emf_edges<false><<<grid, 128, 0, s>>>(D, blist, wslot, bfslot);
+        return;
+    }
+    /* chunks of edge layers: two rounds of the 296 CTAs that fit (two per
+     * SM), at least two chunks, since each chunk reads one plane again: 64
+     * blocks 20.6 us with 10 chunks, 22.7 with 14 */
+    constexpr int fill = 592;
+    const int nchunk = nlist * 17 <= fill ? 17 : nlist * 2 >= fill ? 2 : (fill + nlist - 1) / nlist;
+    constexpr int smem = 2 * FX_EP_COUNT * kEmfNodes * (int)sizeof(double);
+    static const cudaError_t opted = cudaFuncSetAttribute(k_emf, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    (void)opted;
+    k_emf<<<dim3(nchunk, nlist), kEmfThreads, smem, s>>>(D, blist, wslot, bfslot, nchunk);
 }
 
 void fx_launch_bf_update(const FxDev &D, const int *blist, int nlist, int stage, cudaStream_t s)
@@ -1753,19 +1861,25 @@ void fx_launch_bf_update(const FxDev &D, const int *blist, int nlist, int stage,
     k_bf_update<<<dim3(fx_blocks(nf, 128), 3, nlist), 128, 0, s>>>(D, blist, stage);
 }
 
+template <bool MHD, bool FULL>
+static void launch_cell_update(const FxDev &D, const int *blist, int nlist, int stage, int gravity, cudaStream_t s)
+{
+    const dim3 grid(fx_blocks(FX_BS * FX_BS * FX_BS, 128), nlist);
+    if (stage == 1) k_cell_update<MHD, 1, FULL><<<grid, 128, 0, s>>>(D, blist, gravity);
+    else if (stage == 2) k_cell_update<MHD, 2, FULL><<<grid, 128, 0, s>>>(D, blist, gravity);
+    else k_cell_update<MHD, 0, FULL><<<grid, 128, 0, s>>>(D, blist, gravity);
+}
+
 void fx_launch_cell_update(const FxDev &D, const int *blist, int nlist, int stage,
-    int gravity, int store_rhs, cudaStream_t s)
+    int gravity, int full, cudaStream_t s)
 {
     if (nlist <= 0) return;
-    const dim3 grid(fx_blocks(FX_BS * FX_BS * FX_BS, 128), nlist);
     if (D.nv == 9) {
-        if (stage == 1) k_cell_update<true, 1><<<grid, 128, 0, s>>>(D, blist, gravity, store_rhs);
-        else if (stage == 2) k_cell_update<true, 2><<<grid, 128, 0, s>>>(D, blist, gravity, store_rhs);
-        else k_cell_update<true, 0><<<grid, 128, 0, s>>>(D, blist, gravity, store_rhs);
+        if (full) launch_cell_update<true, true>(D, blist, nlist, stage, gravity, s);
+        else launch_cell_update<true, false>(D, blist, nlist, stage, gravity, s);
     } else {
-        if (stage == 1) k_cell_update<false, 1><<<grid, 128, 0, s>>>(D, blist, gravity, store_rhs);
-        else if (stage == 2) k_cell_update<false, 2><<<grid, 128, 0, s>>>(D, blist, gravity, store_rhs);
-        else k_cell_update<false, 0><<<grid, 128, 0, s>>>(D, blist, gravity, store_rhs);
+        if (full) launch_cell_update<false, true>(D, blist, nlist, stage, gravity, s);
+        else launch_cell_update<false, false>(D, blist, nlist, stage, gravity, s);
     }
 }
 

@@ -48,6 +48,10 @@ struct FxDev {
     double *Bf;   /* [b][dir][stage][face]         (FACE_IDX) */
     double *flux; /* [b][dir][AoSoA nc=nv]         (VIDX) */
     double *vr;   /* [b][dir][AoSoA nc=3]          (VRIDX) */
+    /* the batched form's face velocities, normal component only: the
+     * reference's AoSoA tile holds three components of which later phases
+     * read one, and DRAM moves whole tiles */
+    double *vn;   /* [b][dir][cell]                (IDX) */
     double *bv1;  /* [b][dir][cell]                (IDX) */
     double *bv2;
     double *emf;  /* [b][dir][edge]                (EDGE_IDX) */
@@ -168,13 +172,17 @@ struct FxXent {
 /* launchers (fx_kernels.cu); all asynchronous on `s` */
 void fx_launch_flux(const FxDev &D, const int *blist, int nlist, int ndir, int wslot, int bfslot,
     int full, cudaStream_t s);
-void fx_launch_emf(const FxDev &D, const int *blist, int nlist, int wslot, int bfslot, cudaStream_t s);
+/* full: the plain form (velocities in vr), else the batched one (vn) */
+void fx_launch_emf(const FxDev &D, const int *blist, int nlist, int wslot, int bfslot, int full, cudaStream_t s);
+/* the batched form's face arrays of the listed blocks in the reference's
+ * layout (the entries the batched form has) */
+void fx_launch_expand_faces(const FxDev &D, const int *blist, int nlist, cudaStream_t s);
 /* stage 1, 2: the RK2 stages; stage 0: an eSSPRK forward-Euler substep in
  * place on slot 0 (prj_timeint_mhd_update_bf stage 0 and the stage-1 cell
  * update writing slot 0) */
 void fx_launch_bf_update(const FxDev &D, const int *blist, int nlist, int stage, cudaStream_t s);
 void fx_launch_cell_update(const FxDev &D, const int *blist, int nlist, int stage,
-    int gravity, int store_rhs, cudaStream_t s);
+    int gravity, int full, cudaStream_t s);
 /* dt_stage = dt / divisor in the control block */
 void fx_launch_stage_dt(const FxDev &D, double divisor, cudaStream_t s);
 /* prj_timeint_eSSPRK_save_state (src/prj_timeint.c:2311-2352): W of the
@@ -244,7 +252,7 @@ struct FxAdjDev {
     double *bvb1;
     double *bvb2;
     double *Eb;
-    const double *vr; /* face velocities recomputed from Wbef (normal component) */
+    const double *vn; /* normal face velocities recomputed from Wbef, [b][dir][cell] */
 };
 
 #define FX_ADJ_G_COUNT (9 * FX_NCELLS)

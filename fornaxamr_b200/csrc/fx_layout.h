@@ -99,6 +99,7 @@ FX_HD int fx_bidx_cell(int nc, int v, int cell)
 #define FX_BF_COUNT (3 * FX_NSTAGES * FX_NFACES)
 #define FX_FLUX_COUNT(nv) (3 * (nv) * FX_NCELLS)
 #define FX_VR_COUNT (3 * 3 * FX_NCELLS)
+#define FX_VN_COUNT (3 * FX_NCELLS)
 #define FX_BV_COUNT (3 * FX_NCELLS)
 #define FX_EMF_COUNT (3 * FX_NEDGES)
 #define FX_EOS_COUNT (3 * FX_NCELLS)

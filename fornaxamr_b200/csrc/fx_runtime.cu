@@ -58,7 +58,8 @@ struct fx_ctx {
     FxDev D{};
 
     FxBlockDev *d_blk = nullptr;
-    double *d_W = nullptr, *d_Bf = nullptr, *d_flux = nullptr, *d_vr = nullptr;
+    double *d_W = nullptr, *d_Bf = nullptr, *d_flux = nullptr, *d_vr = nullptr, *d_vn = nullptr;
+    bool compact_faces = false; /* the last face fluxes are the batched form's (vn) */
     double *d_bv1 = nullptr, *d_bv2 = nullptr, *d_emf = nullptr, *d_eos = nullptr;
     double *d_rhs = nullptr, *d_grav = nullptr;
     double *d_W2 = nullptr, *d_Bf2 = nullptr; /* eSSPRK10_4 stage slot 2 */
@@ -89,7 +90,7 @@ struct fx_ctx {
      * fx_adjoint_forward and the adjoint arrays */
     int adj_nsteps = 0;
     double adj_dt = 0.0;
-    double *d_ckW = nullptr, *d_ckBf = nullptr, *d_ckVr = nullptr;
+    double *d_ckW = nullptr, *d_ckBf = nullptr, *d_ckVn = nullptr;
     double *d_Wb = nullptr, *d_Bfb = nullptr, *d_G = nullptr;
     double *d_bvb1 = nullptr, *d_bvb2 = nullptr, *d_Eb = nullptr;
     double adj_ms = 0.0;              /* device time of the last reverse sweep */
@@ -233,6 +234,7 @@ void free_mesh(fx_ctx *c)
     cudaFree(c->d_Bf);
     cudaFree(c->d_flux);
     cudaFree(c->d_vr);
+    cudaFree(c->d_vn);
     cudaFree(c->d_bv1);
     cudaFree(c->d_bv2);
     cudaFree(c->d_emf);
@@ -254,15 +256,15 @@ void free_mesh(fx_ctx *c)
     cudaFree(c->d_ecorr);
     for (size_t &cap : c->tab_cap) cap = 0;
     c->d_blk = nullptr;
-    c->d_W = c->d_Bf = c->d_flux = c->d_vr = c->d_bv1 = c->d_bv2 = nullptr;
+    c->d_W = c->d_Bf = c->d_flux = c->d_vr = c->d_vn = c->d_bv1 = c->d_bv2 = nullptr;
     c->d_emf = c->d_eos = c->d_rhs = c->d_grav = nullptr;
     c->d_ids = c->d_active = nullptr;
     c->d_cops = c->d_fops = nullptr;
     c->d_fcorr = c->d_ecorr = nullptr;
     cudaFree(c->d_ckW);
     cudaFree(c->d_ckBf);
-    cudaFree(c->d_ckVr);
-    c->d_ckVr = nullptr;
+    cudaFree(c->d_ckVn);
+    c->d_ckVn = nullptr;
     cudaFree(c->d_adj_csrc);
     cudaFree(c->d_adj_fsrc);
     cudaFree(c->d_adj_ents);
@@ -278,6 +280,7 @@ void free_mesh(fx_ctx *c)
     c->d_ckW = c->d_ckBf = c->d_Wb = c->d_Bfb = c->d_G = nullptr;
     c->d_bvb1 = c->d_bvb2 = c->d_Eb = nullptr;
     c->adj_nsteps = 0;
+    c->compact_faces = false;
     c->nblocks = 0;
     c->nactive = 0;
     c->cap = 0;
@@ -337,6 +340,16 @@ void per_block(fx_ctx *c, int form, F &&fn)
     } else {
         fn(c->d_active, c->nactive);
     }
+}
+
+/* Face arrays: the batched form keeps its own (compact) ones.  A plain entry
+ * point, or a download, after batched stages first gets what they hold in
+ * the reference's layout. */
+void expand_faces(fx_ctx *c)
+{
+    if (!c->compact_faces) return;
+    fx_launch_expand_faces(c->D, c->d_active, c->nactive, c->stream);
+    c->compact_faces = false;
 }
 
 /* the whole ghost fill of prj_boundary_fill_ghosts_and_bf: one launch per
@@ -426,10 +439,11 @@ void stage_seq(fx_ctx *c, int form, int stage)
         }
     }
     per_block(c, form, [&](const int *l, int n) { fx_launch_flux(c->D, l, n, 3, src, src, full, s); });
+    c->compact_faces = !full;
     shard_exchange(c, FX_XF, src);
     flux_correct(c, full ? c->nv : 6, s);
     if (c->cfg.mhd) {
-        per_block(c, form, [&](const int *l, int n) { fx_launch_emf(c->D, l, n, src, src, s); });
+        per_block(c, form, [&](const int *l, int n) { fx_launch_emf(c->D, l, n, src, src, full, s); });
         shard_exchange(c, FX_XE, src);
         emf_correct(c, s);
         per_block(c, form, [&](const int *l, int n) { fx_launch_bf_update(c->D, l, n, stage, s); });
@@ -470,9 +484,10 @@ void essprk_substep(fx_ctx *c, int form)
     cudaStream_t s = c->stream;
     const int full = form == FX_FORM_PLAIN ? 1 : 0;
     per_block(c, form, [&](const int *l, int n) { fx_launch_flux(c->D, l, n, 3, 0, 0, full, s); });
+    c->compact_faces = !full;
     flux_correct(c, full ? c->nv : 6, s);
     if (c->cfg.mhd) {
-        per_block(c, form, [&](const int *l, int n) { fx_launch_emf(c->D, l, n, 0, 0, s); });
+        per_block(c, form, [&](const int *l, int n) { fx_launch_emf(c->D, l, n, 0, 0, full, s); });
         emf_correct(c, s);
         per_block(c, form, [&](const int *l, int n) { fx_launch_bf_update(c->D, l, n, 0, s); });
     }
@@ -695,6 +710,7 @@ int alloc_block_arrays(fx_ctx *c, int cap, int keep)
     if ((rc = regrow(c, &c->d_W, w_count(c), cap, keep))) return rc;
     if ((rc = regrow(c, &c->d_flux, (size_t)FX_FLUX_COUNT(c->nv), cap, keep))) return rc;
     if ((rc = regrow(c, &c->d_vr, (size_t)FX_VR_COUNT, cap, keep))) return rc;
+    if ((rc = regrow(c, &c->d_vn, (size_t)FX_VN_COUNT, cap, keep))) return rc;
     if ((rc = regrow(c, &c->d_eos, (size_t)FX_EOS_COUNT, cap, keep))) return rc;
     if ((rc = regrow(c, &c->d_rhs, (size_t)FX_RHS_COUNT(c->nv), cap, keep))) return rc;
     if (c->cfg.mhd) {
@@ -777,6 +793,7 @@ int install_tables(fx_ctx *c)
     c->D.Bf = c->d_Bf;
     c->D.flux = c->d_flux;
     c->D.vr = c->d_vr;
+    c->D.vn = c->d_vn;
     c->D.bv1 = c->d_bv1;
     c->D.bv2 = c->d_bv2;
     c->D.emf = c->d_emf;
@@ -916,7 +933,7 @@ void drop_adjoint(fx_ctx *c)
 {
     cudaFree(c->d_ckW);
     cudaFree(c->d_ckBf);
-    cudaFree(c->d_ckVr);
+    cudaFree(c->d_ckVn);
     cudaFree(c->d_adj_csrc);
     cudaFree(c->d_adj_fsrc);
     cudaFree(c->d_adj_ents);
@@ -926,7 +943,7 @@ void drop_adjoint(fx_ctx *c)
     cudaFree(c->d_bvb1);
     cudaFree(c->d_bvb2);
     cudaFree(c->d_Eb);
-    c->d_ckW = c->d_ckBf = c->d_ckVr = nullptr;
+    c->d_ckW = c->d_ckBf = c->d_ckVn = nullptr;
     c->d_adj_csrc = c->d_adj_fsrc = nullptr;
     c->d_adj_ents = nullptr;
     c->d_Wb = c->d_Bfb = c->d_G = c->d_bvb1 = c->d_bvb2 = c->d_Eb = nullptr;
@@ -1561,6 +1578,7 @@ int fx_download_array(fx_ctx *c, int b, int which, int dir, double *out)
     const double *src = nullptr;
     size_t count = 0;
     const size_t nv = (size_t)c->nv;
+    if (which == FX_ARR_VRIEMANN) expand_faces(c);
     switch (which) {
     case FX_ARR_W: {
         int rc = xfer_w(c, b, 1, out, cudaMemcpyDeviceToHost, false);
@@ -1613,6 +1631,7 @@ int fx_flux_update(fx_ctx *c, int b, int w_slot, int use_bf1)
     int rc = check_block(c, b);
     if (rc) return rc;
     if (w_slot < 0 || w_slot > 1 || use_bf1 < 0 || use_bf1 > 1) return set_err(c, FX_EINVAL, "bad slot");
+    expand_faces(c);
     fx_launch_set_dt(c->D, 0.0, c->stream);
     fx_launch_flux(c->D, c->d_ids + b, 1, 3, w_slot, use_bf1, 1, c->stream);
     return FX_SUCCESS;
@@ -1624,8 +1643,9 @@ int fx_mhd_update_emf(fx_ctx *c, int b, int stage)
     int rc = check_block(c, b);
     if (rc) return rc;
     if (!c->cfg.mhd || stage < 0 || stage > 1) return set_err(c, FX_EINVAL, "bad emf call");
+    expand_faces(c);
     fx_launch_set_dt(c->D, 0.0, c->stream);
-    fx_launch_emf(c->D, c->d_ids + b, 1, stage, stage, c->stream);
+    fx_launch_emf(c->D, c->d_ids + b, 1, stage, stage, 1, c->stream);
     return FX_SUCCESS;
 }
 
@@ -1646,6 +1666,7 @@ int fx_update_cells(fx_ctx *c, int b, int stage, double dt, double *dt_src)
     int rc = check_block(c, b);
     if (rc) return rc;
     if (stage != 1 && stage != 2) return set_err(c, FX_EINVAL, "bad stage");
+    expand_faces(c);
     fx_launch_set_dt(c->D, dt, c->stream);
     if (dt_src) fx_launch_reset_reductions(c->D, 2, c->stream);
     fx_launch_cell_update(c->D, c->d_ids + b, 1, stage, c->cfg.gravity, 1, c->stream);
@@ -1663,6 +1684,7 @@ int fx_riemann_flux_send(fx_ctx *c)
 {
     if (c && c->nranks > 1) return set_err(c, FX_EINVAL, "%s: not available on a sharded mesh", __func__);
     if (!has_mesh(c)) return c ? set_err(c, FX_ENOMESH, "no mesh") : FX_EINVAL;
+    expand_faces(c);
     fx_launch_set_dt(c->D, 0.0, c->stream);
     flux_correct(c, c->nv, c->stream);
     return FX_SUCCESS;
@@ -1771,6 +1793,7 @@ int fx_step(fx_ctx *c, int form, double dt, double *dt_src)
         int rc = build_step_graph(c);
         if (rc) return rc;
         FX_CUDA(c, cudaGraphLaunch(c->g_step, c->stream));
+        c->compact_faces = true;
         c->last_slot = 0;
     }
     shard_min(c, 1, 1);
@@ -1835,6 +1858,7 @@ int fx_run(fx_ctx *c, int form, int nsteps, double cfl, double dt_factor, double
         for (int n = 0; n < nsteps; ++n) {
             FX_CUDA(c, cudaGraphLaunch(c->g_run, c->stream));
         }
+        if (nsteps > 0) c->compact_faces = true;
     }
     c->last_slot = 0;
     FX_CUDA(c, cudaMemcpyAsync(c->h_ctl, c->d_ctl, sizeof(FxCtl), cudaMemcpyDeviceToHost, c->stream));
@@ -1862,7 +1886,7 @@ int fx_time_phase(fx_ctx *c, int phase, int reps, double dt, double *ms)
     auto launch = [&]() {
         switch (phase) {
         case FX_PHASE_FLUX: fx_launch_flux(c->D, c->d_active, c->nactive, 3, 0, 0, 0, s); break;
-        case FX_PHASE_EMF: fx_launch_emf(c->D, c->d_active, c->nactive, 0, 0, s); break;
+        case FX_PHASE_EMF: fx_launch_emf(c->D, c->d_active, c->nactive, 0, 0, 0, s); break;
         case FX_PHASE_CT: fx_launch_bf_update(c->D, c->d_active, c->nactive, 1, s); break;
         case FX_PHASE_CELLS: fx_launch_cell_update(c->D, c->d_active, c->nactive, 1, c->cfg.gravity, 0, s); break;
         case FX_PHASE_GHOST: ghost_fill(c, 1); break;
@@ -1870,6 +1894,7 @@ int fx_time_phase(fx_ctx *c, int phase, int reps, double dt, double *ms)
         }
     };
     fx_launch_set_dt(c->D, dt, s);
+    if (phase == FX_PHASE_FLUX || phase == FX_PHASE_STEP) c->compact_faces = true;
     launch();
     cudaEvent_t e0, e1;
     FX_CUDA(c, cudaEventCreate(&e0));
@@ -1897,6 +1922,7 @@ int fx_autotune(fx_ctx *c, double *times_ms, int n, int *choice)
     FX_CUDA(c, cudaEventCreate(&e0));
     FX_CUDA(c, cudaEventCreate(&e1));
     fx_launch_set_dt(c->D, 0.0, s);
+    c->compact_faces = true;
     int best = 0;
     double best_ms = 1.0e30;
     for (int v = 0; v < FX_FLUX_VARIANTS; ++v) {
@@ -2066,6 +2092,7 @@ int fx_amr_adapt(fx_ctx *c, int *changed)
         c->D.Bf = c->d_Bf;
         c->D.flux = c->d_flux;
         c->D.vr = c->d_vr;
+    c->D.vn = c->d_vn;
         c->D.bv1 = c->d_bv1;
         c->D.bv2 = c->d_bv2;
         c->D.emf = c->d_emf;
@@ -2459,7 +2486,7 @@ int adjoint_reverse(fx_ctx *c)
             A.Wbef = c->d_ckW + (k - 1) * wn;
             A.Bfbef = c->d_ckBf + (k - 1) * bn;
             A.Waft = c->d_ckW + k * wn;
-            A.vr = c->d_ckVr + (k - 1) * nb * FX_VR_COUNT;
+            A.vn = c->d_ckVn + (k - 1) * nb * FX_VN_COUNT;
             adj_ghost(c, A, dst);
             fx_launch_adj_cells(A, c->d_active, c->nactive, stage, s);
             FX_CUDA(c, cudaMemsetAsync(c->d_Eb, 0, nb * FX_EMF_COUNT * sizeof(double), s));
@@ -2497,7 +2524,7 @@ int fx_adjoint_forward(fx_ctx *c, int nsteps, double dt)
     if (c->adj_nsteps != nsteps || !c->d_ckW) {
         if ((rc = dev_alloc(c, &c->d_ckW, nck * wn))) return rc;
         if ((rc = dev_alloc(c, &c->d_ckBf, nck * bn))) return rc;
-        if ((rc = dev_alloc(c, &c->d_ckVr, (nck - 1) * nb * FX_VR_COUNT))) return rc;
+        if ((rc = dev_alloc(c, &c->d_ckVn, (nck - 1) * nb * FX_VN_COUNT))) return rc;
     }
     cudaStream_t s = c->stream;
     const cudaMemcpyKind d2d = cudaMemcpyDeviceToDevice;
@@ -2512,8 +2539,8 @@ int fx_adjoint_forward(fx_ctx *c, int nsteps, double dt)
             FX_CUDA(c, cudaMemcpyAsync(c->d_ckBf + k * bn, c->d_Bf, bn * sizeof(double), d2d, s));
             /* the stage's face velocities: their signs pick the upwind EMF
              * terms the reverse pass differentiates */
-            FX_CUDA(c, cudaMemcpyAsync(c->d_ckVr + (k - 1) * nb * FX_VR_COUNT, c->d_vr,
-                nb * FX_VR_COUNT * sizeof(double), d2d, s));
+            FX_CUDA(c, cudaMemcpyAsync(c->d_ckVn + (k - 1) * nb * FX_VN_COUNT, c->d_vn,
+                nb * FX_VN_COUNT * sizeof(double), d2d, s));
         }
     }
     c->adj_nsteps = nsteps;
