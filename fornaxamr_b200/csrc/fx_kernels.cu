@@ -1082,6 +1082,10 @@ __global__ void k_step_end(FxDev D)
 /* Ghost-fill programs                                                       */
 /* ------------------------------------------------------------------------ */
 
+/* the primitives the fill writes: all but the cell-centred field, which
+ * follows from the faces */
+constexpr int kGhostVars = 6;
+
 /* prj_reconstruct_cell_for_prolongate_minmod (src/prj_reconstruct.h:111-143):
  * per axis base + slope * target, combined as vx + vy + vz - 2 base; target
  * offsets are +-1/4 of a coarse cell.  use_BJ = 1 takes fx_bj_cell /
@@ -1110,7 +1114,7 @@ __device__ __forceinline__ double fx_prolong_face(const double *q, int f, int s0
  * other instance keeps the copy-dominated wave kernel at its small register
  * count */
 template <bool BJ>
-__device__ __forceinline__ void fx_ghost_cell_op(const FxDev &D, const FxGop op, int wslot, int nvg)
+__device__ __forceinline__ void fx_ghost_cell_op(const FxDev &D, const FxGop op, int wslot)
 {
     const int db = FX_CELL_BLOCK(op.dst);
     const int dc = FX_CELL_IDX(op.dst);
@@ -1124,7 +1128,7 @@ __device__ __forceinline__ void fx_ghost_cell_op(const FxDev &D, const FxGop op,
             const double ty = (op.aux & 2) ? 0.25 : -0.25;
             const double tz = (op.aux & 1) ? 0.25 : -0.25;
 #pragma unroll 1
-            for (int v = 0; v < nvg; ++v) {
+            for (int v = 0; v < kGhostVars; ++v) {
                 const double *q = Ws + (size_t)v * kPlane + sc;
                 Wd[(size_t)v * kPlane + dc] = fx_bj_cell(
                     [q](int di, int dj, int dk) { return q[(di * FX_PBS + dj) * FX_PBS + dk]; }, tx, ty, tz);
@@ -1135,18 +1139,18 @@ __device__ __forceinline__ void fx_ghost_cell_op(const FxDev &D, const FxGop op,
     /* every variable's value first, then the stores: the loads of all
      * variables are in flight together (the wave's operations are conflict
      * free, so no store of the wave feeds a load of it) */
-    double val[FX_MAXVAR];
+    double val[kGhostVars];
     switch (op.type) {
     case FX_GOP_COPY:
     case FX_GOP_COPY_NEG:
     case FX_GOP_COPY_USER:
 #pragma unroll
-        for (int v = 0; v < FX_MAXVAR; ++v) {
-            if (v < nvg) val[v] = Ws[(size_t)v * kPlane + sc];
+        for (int v = 0; v < kGhostVars; ++v) {
+            val[v] = Ws[(size_t)v * kPlane + sc];
         }
         if (op.type == FX_GOP_COPY_NEG) {
 #pragma unroll
-            for (int v = 0; v < FX_MAXVAR; ++v) {
+            for (int v = 0; v < kGhostVars; ++v) {
                 if (v == op.aux) val[v] = -val[v];
             }
         } else if (op.type == FX_GOP_COPY_USER && op.aux) {
@@ -1155,8 +1159,7 @@ __device__ __forceinline__ void fx_ghost_cell_op(const FxDev &D, const FxGop op,
         break;
     case FX_GOP_RESTRICT:
 #pragma unroll
-        for (int v = 0; v < FX_MAXVAR; ++v) {
-            if (v >= nvg) continue;
+        for (int v = 0; v < kGhostVars; ++v) {
             const double *q = Ws + (size_t)v * kPlane + sc;
             /* order of src/prj_boundary.c:238-261 */
             val[v] = 0.125 *
@@ -1171,8 +1174,8 @@ __device__ __forceinline__ void fx_ghost_cell_op(const FxDev &D, const FxGop op,
         const double ty = (op.aux & 2) ? 0.25 : -0.25;
         const double tz = (op.aux & 1) ? 0.25 : -0.25;
 #pragma unroll
-        for (int v = 0; v < FX_MAXVAR; ++v) {
-            if (v < nvg) val[v] = fx_prolong_cell(Ws + (size_t)v * kPlane, sc, tx, ty, tz);
+        for (int v = 0; v < kGhostVars; ++v) {
+            val[v] = fx_prolong_cell(Ws + (size_t)v * kPlane, sc, tx, ty, tz);
         }
         break;
     }
@@ -1180,8 +1183,8 @@ __device__ __forceinline__ void fx_ghost_cell_op(const FxDev &D, const FxGop op,
         return;
     }
 #pragma unroll
-    for (int v = 0; v < FX_MAXVAR; ++v) {
-        if (v < nvg) Wd[(size_t)v * kPlane + dc] = val[v];
+    for (int v = 0; v < kGhostVars; ++v) {
+        Wd[(size_t)v * kPlane + dc] = val[v];
     }
 }
 
@@ -1377,6 +1380,83 @@ __device__ __forceinline__ void fx_ghost_b_op(const FxDev &D, const FxBop op, in
     W[(size_t)FX_B3 * kPlane + c] = v[2];
 }
 
+/* two neighbouring doubles: one 16-byte access where the index is even (the
+ * block arrays and their planes start 16-byte aligned), else two */
+__device__ __forceinline__ double2 fx_load2(const double *p, int i)
+{
+    if ((i & 1) == 0) return *reinterpret_cast<const double2 *>(p + i);
+    return make_double2(p[i], p[i + 1]);
+}
+
+__device__ __forceinline__ void fx_store2(double *p, int i, double2 v)
+{
+    if ((i & 1) == 0) {
+        *reinterpret_cast<double2 *>(p + i) = v;
+    } else {
+        p[i] = v.x;
+        p[i + 1] = v.y;
+    }
+}
+
+/* one or two neighbouring cell copies, every load ahead of the stores */
+__device__ __forceinline__ void fx_ghost_cell_copy(const FxDev &D, const FxPair op, int slot)
+{
+    const int dst = op.dst & 0x7fffffff;
+    const int sc = FX_CELL_IDX(op.src), dc = FX_CELL_IDX(dst);
+    const double *Ws = D.W + (size_t)FX_CELL_BLOCK(op.src) * FX_W_COUNT(D.nv) + (size_t)slot * FX_NCELLS;
+    double *Wd = D.W + (size_t)FX_CELL_BLOCK(dst) * FX_W_COUNT(D.nv) + (size_t)slot * FX_NCELLS;
+    if (op.dst < 0) {
+        double val[kGhostVars];
+#pragma unroll
+        for (int v = 0; v < kGhostVars; ++v) val[v] = Ws[(size_t)v * kPlane + sc];
+#pragma unroll
+        for (int v = 0; v < kGhostVars; ++v) Wd[(size_t)v * kPlane + dc] = val[v];
+        return;
+    }
+    double2 val[kGhostVars];
+#pragma unroll
+    for (int v = 0; v < kGhostVars; ++v) val[v] = fx_load2(Ws + (size_t)v * kPlane, sc);
+#pragma unroll
+    for (int v = 0; v < kGhostVars; ++v) fx_store2(Wd + (size_t)v * kPlane, dc, val[v]);
+}
+
+/* direction array of a pair's face key, and the face in it */
+__device__ __forceinline__ double *fx_pair_faces(const FxDev &D, int key, int slot, int &f)
+{
+    const unsigned bd = ((unsigned)key & 0x7fffffffu) >> 14;
+    f = key & 16383;
+    /* block b, direction d: (2 (3 b + d) + slot) faces in */
+    return D.Bf + ((size_t)bd * FX_NSTAGES + slot) * FX_NFACES;
+}
+
+/* cell-centred field of two neighbouring cells (fx_ghost_b_op) */
+__device__ __forceinline__ void fx_ghost_b_pair(const FxDev &D, const FxBop op, int slot)
+{
+    double2 v[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        const int k0 = op.f[2 * d];
+        const int k1 = op.f[2 * d + 1];
+        const double2 a = fx_load2(D.Bf + (size_t)fx_face_key_block(k0) * FX_BF_COUNT +
+            ((size_t)d * FX_NSTAGES + slot) * FX_NFACES, fx_face_key_idx(k0));
+        const double2 b = fx_load2(D.Bf + (size_t)fx_face_key_block(k1) * FX_BF_COUNT +
+            ((size_t)d * FX_NSTAGES + slot) * FX_NFACES, fx_face_key_idx(k1));
+        v[d] = make_double2(0.5 * (a.x + b.x), 0.5 * (a.y + b.y));
+    }
+    const int b = FX_CELL_BLOCK(op.dst);
+    const int c = FX_CELL_IDX(op.dst);
+    if (fx_nonfinite(v[0].x) || fx_nonfinite(v[1].x) || fx_nonfinite(v[2].x)) {
+        fx_fail(D.err, FX_ERR_B_NONFINITE, b, c);
+    }
+    if (fx_nonfinite(v[0].y) || fx_nonfinite(v[1].y) || fx_nonfinite(v[2].y)) {
+        fx_fail(D.err, FX_ERR_B_NONFINITE, b, c + 1);
+    }
+    double *W = D.W + (size_t)b * FX_W_COUNT(9) + (size_t)slot * FX_NCELLS;
+    fx_store2(W + (size_t)FX_B1 * kPlane, c, v[0]);
+    fx_store2(W + (size_t)FX_B2 * kPlane, c, v[1]);
+    fx_store2(W + (size_t)FX_B3 * kPlane, c, v[2]);
+}
+
 /* face-prolongation groups of one wave (a separate kernel: the group
  * arithmetic would otherwise raise the register count, and so lower the
  * occupancy, of the copy-dominated wave kernel) */
@@ -1389,46 +1469,94 @@ __global__ void __launch_bounds__(128) k_ghost_groups(FxDev D, const FxPop *__re
     fx_ghost_prolong_group(D, pops[t], slot);
 }
 
-/* one conflict-free wave of the ghost fill: CTAs [0, nbc) run cell ops,
- * then face ops (FX_GW_FACE_OPS per thread) and cell-field ops.  At 6 CTAs
- * of 256 per SM the kernel keeps 40 registers without spills; on the 512-block
- * uniform fill this took 0.165 ms down to 0.148 ms. */
+/* face pairs per thread of the wave kernel */
+constexpr int FX_GW_FACE_PAIRS = 4;
+
+/* CTAs of each list of a wave */
+struct FxWaveGrid {
+    int cp, cg, fp, fg, b;
+};
+
+/* One conflict-free wave of the ghost fill: the lists of FxWave one after the
+ * other, a range of CTAs each.  Bound by DRAM and latency.
+ * 512 blocks 149 us (148 with one 16-byte entry per element),
+ * 105 blocks 24.7 (30.9), the 470-block blast's fill 288 (314; its groups run
+ * beside).  Pairs and single copies in lists of their own, each a pass over the
+ * mesh, measured 190 us: they share sectors. */
 template <bool BJ>
-__global__ void __launch_bounds__(256, 6) k_ghost_wave(FxDev D, const FxGop *__restrict__ cops, int nc,
-    const FxGop *__restrict__ fops, int nf, const FxBop *__restrict__ bops, int nb, int slot, int nvg)
+__global__ void __launch_bounds__(256, BJ ? 4 : 6) k_ghost_wave(FxDev D, FxWave w, FxWaveGrid g, int slot)
 {
     if (D.ctl->skip) {
         return;
     }
-    constexpr int UF = FX_GW_FACE_OPS;
-    const int nbc = (nc + 255) / 256;
-    const int nbf = (nf + 256 * UF - 1) / (256 * UF);
     int blk = blockIdx.x;
-    if (blk < nbc) {
+    if (blk < g.cp) {
         const int t = blk * 256 + threadIdx.x;
-        if (t < nc) fx_ghost_cell_op<BJ>(D, cops[t], slot, nvg);
+        if (t < w.ncp) fx_ghost_cell_copy(D, w.cp[t], slot);
         return;
     }
-    blk -= nbc;
-    if (blk < nbf) {
-        /* operations t0 + 256 u, u < UF: every load first, then the stores */
-        const int t0 = blk * 256 * UF + threadIdx.x;
-        double v[UF];
-        double *dst[UF];
+    blk -= g.cp;
+    if (blk < g.fp) {
+        /* pairs t0 + 256 u: every load first, then the stores */
+        constexpr int UP = FX_GW_FACE_PAIRS;
+        const int t0 = blk * 256 * UP + threadIdx.x;
+        double2 v[UP];
+        FxPair op[UP];
 #pragma unroll
-        for (int u = 0; u < UF; ++u) {
-            const int t = t0 + 256 * u;
-            dst[u] = t < nf ? fx_ghost_face_value(D, fops[t], slot, v[u]) : nullptr;
+        for (int u = 0; u < UP; ++u) {
+            if (t0 + 256 * u < w.nfp) op[u] = w.fp[t0 + 256 * u];
         }
 #pragma unroll
-        for (int u = 0; u < UF; ++u) {
-            if (dst[u]) *dst[u] = v[u];
+        for (int u = 0; u < UP; ++u) {
+            if (t0 + 256 * u < w.nfp) {
+                int f;
+                const double *p = fx_pair_faces(D, op[u].src, slot, f);
+                if (op[u].dst < 0) v[u].x = p[f];
+                else v[u] = fx_load2(p, f);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < UP; ++u) {
+            if (t0 + 256 * u < w.nfp) {
+                int f;
+                double *p = fx_pair_faces(D, op[u].dst, slot, f);
+                if (op[u].dst < 0) p[f] = v[u].x;
+                else fx_store2(p, f, v[u]);
+            }
         }
         return;
     }
-    blk -= nbf;
-    const int t = blk * 256 + threadIdx.x;
-    if (t < nb) fx_ghost_b_op(D, bops[t], slot);
+    blk -= g.fp;
+    if (blk < g.b) {
+        const int t = blk * 256 + threadIdx.x;
+        if (t < w.nb) {
+            const FxBop op = w.b[t];
+            if (op.pad == 2) fx_ghost_b_pair(D, op, slot);
+            else fx_ghost_b_op(D, op, slot);
+        }
+        return;
+    }
+    blk -= g.b;
+    if (blk < g.cg) {
+        const int t = blk * 256 + threadIdx.x;
+        if (t < w.ncg) fx_ghost_cell_op<BJ>(D, w.cg[t], slot);
+        return;
+    }
+    blk -= g.cg;
+    /* operations t0 + 256 u, u < UF: every load first, then the stores */
+    constexpr int UF = FX_GW_FACE_OPS;
+    const int t0 = blk * 256 * UF + threadIdx.x;
+    double v[UF];
+    double *dst[UF];
+#pragma unroll
+    for (int u = 0; u < UF; ++u) {
+        const int t = t0 + 256 * u;
+        dst[u] = t < w.nfg ? fx_ghost_face_value(D, w.fg[t], slot, v[u]) : nullptr;
+    }
+#pragma unroll
+    for (int u = 0; u < UF; ++u) {
+        if (dst[u]) *dst[u] = v[u];
+    }
 }
 
 /* exchanges of a sharded mesh: one thread per listed element */
@@ -1898,21 +2026,15 @@ void fx_launch_calc_dt(const FxDev &D, const int *blist, int nlist, int wslot, d
     k_calc_dt<<<dim3(fx_blocks(FX_BS * FX_BS * FX_BS, 256), nlist), 256, 0, s>>>(D, blist, wslot, cfl);
 }
 
-void fx_launch_ghost_wave(const FxDev &D, const FxGop *cops, int nc, const FxGop *fops, int nf,
-    const FxPop *pops, int np, const FxBop *bops, int nb, int slot, int nvg, cudaStream_t s)
+void fx_launch_ghost_wave(const FxDev &D, const FxWave &w, int slot, cudaStream_t s)
 {
-    /* the operations of a wave are conflict free: the two launches may run
-     * in either order */
-    const unsigned grid = fx_blocks(nc, 256) + fx_blocks(nf, 256 * FX_GW_FACE_OPS) + fx_blocks(nb, 256);
+    const FxWaveGrid g = {(int)fx_blocks(w.ncp, 256), (int)fx_blocks(w.ncg, 256),
+        (int)fx_blocks(w.nfp, 256 * FX_GW_FACE_PAIRS), (int)fx_blocks(w.nfg, 256 * FX_GW_FACE_OPS),
+        (int)fx_blocks(w.nb, 256)};
+    const unsigned grid = (unsigned)(g.cp + g.cg + g.fp + g.fg + g.b);
     if (grid > 0) {
-        if (D.use_bj) {
-            k_ghost_wave<true><<<grid, 256, 0, s>>>(D, cops, nc, fops, nf, bops, nb, slot, nvg);
-        } else {
-            k_ghost_wave<false><<<grid, 256, 0, s>>>(D, cops, nc, fops, nf, bops, nb, slot, nvg);
-        }
-    }
-    if (np > 0) {
-        k_ghost_groups<<<fx_blocks(np, 128), 128, 0, s>>>(D, pops, np, slot);
+        if (D.use_bj) k_ghost_wave<true><<<grid, 256, 0, s>>>(D, w, g, slot);
+        else k_ghost_wave<false><<<grid, 256, 0, s>>>(D, w, g, slot);
     }
 }
 

@@ -114,6 +114,35 @@ struct FxBop {
     int32_t pad;
 };
 
+/* Copies of one or two neighbouring elements, dst <- src (and dst + 1 <- src +
+ * 1): cell keys, or face keys FX_PFACE(block, dir, face).  Nine of ten copies
+ * of a fill have such a neighbour (ghost rows run along k, at least two
+ * deep). */
+struct FxPair {
+    int32_t dst; /* with FX_PAIR_ONE set: one element */
+    int32_t src;
+};
+#define FX_PAIR_ONE 0x80000000u
+
+/* face key of a pair: 14 bits of face (8400, or 14400 with four ghost
+ * layers), 17 of 3 block + direction (blocks below FX_PFACE_BLOCKS) */
+#define FX_PFACE_BLOCKS 43690
+#define FX_PFACE(b, dir, f) ((int32_t)((((uint32_t)(b) * 3u + (uint32_t)(dir)) << 14) | (uint32_t)(f)))
+
+/* One wave of the ghost fill as the device runs it: cell copies, the other
+ * cell operations, face copies, the other face operations, cell-field
+ * operations (pad 2: of the cells dst, dst + 1 from the faces f[n], f[n] + 1;
+ * pad 1: of dst).  Every list keeps the program's order, so that what lies
+ * together in memory is touched together. */
+struct FxWave {
+    int ncp, ncg, nfp, nfg, nb;
+    const FxPair *cp;
+    const FxGop *cg;
+    const FxPair *fp;
+    const FxGop *fg;
+    const FxBop *b;
+};
+
 /* Divergence-preserving prolongation of the face field onto one 2x2x2 group
  * of fine cells (prj_mhd_prolong_bf_from_buffer, src/prj_mhd.c:374-512).
  * pos packs the fine corner (fi, fj, fk) and the coarse cell (ci, cj, ck),
@@ -197,10 +226,9 @@ void fx_launch_eos_fill(const FxDev &D, const int *blist, int nlist, int wslot, 
     cudaStream_t s);
 void fx_launch_calc_dt(const FxDev &D, const int *blist, int nlist, int wslot, double cfl,
     cudaStream_t s);
-/* one wave of the ghost fill (cell ops, face ops, face-prolongation groups
- * and cell-field ops) */
-void fx_launch_ghost_wave(const FxDev &D, const FxGop *cops, int nc, const FxGop *fops, int nf,
-    const FxPop *pops, int np, const FxBop *bops, int nb, int slot, int nvg, cudaStream_t s);
+/* one wave of the ghost fill without its face-prolongation groups
+ * (fx_launch_prolong_groups) */
+void fx_launch_ghost_wave(const FxDev &D, const FxWave &w, int slot, cudaStream_t s);
 /* gather the listed elements into buf / scatter buf into them */
 void fx_launch_xpack(const FxDev &D, const FxXent *ents, int n, double *buf, int slot, cudaStream_t s);
 void fx_launch_xunpack(const FxDev &D, const FxXent *ents, int n, const double *buf, int slot, cudaStream_t s);

@@ -2007,6 +2007,87 @@ void fx_plan_workspace_recycle(FxPlanWorkspace *ws, FxPlan &&old)
     ws->spare.b_ops.swap(old.ghost.b_ops);
 }
 
+namespace {
+
+/* ops [b0, b1) in order: every one that make() accepts, joined with the
+ * next where joins() says so, to `packed`, the others to `rest`; in parts by
+ * thread (a pair across a part's end stays apart) */
+template <class Op, class Packed, class Joins, class Make>
+void pack_range(const std::vector<Op> &ops, int b0, int b1, std::vector<Packed> &packed, std::vector<Op> &rest,
+    Joins joins, Make make)
+{
+    const int n = b1 - b0;
+    const int nt = n < 50000 ? 1 : std::max(1, compile_threads());
+    std::vector<std::vector<Packed>> ps(nt);
+    std::vector<std::vector<Op>> rs(nt);
+    parallel_for(nt, [&](int t) {
+        const int lo = b0 + (int)((int64_t)n * t / nt), hi = b0 + (int)((int64_t)n * (t + 1) / nt);
+        ps[t].reserve((hi - lo) / 2 + 1);
+        for (int q = lo; q < hi; ++q) {
+            const bool two = q + 1 < hi && joins(ops[q], ops[q + 1]);
+            Packed x;
+            if (make(ops[q], two, x)) {
+                ps[t].push_back(x);
+                q += two ? 1 : 0;
+            } else {
+                rs[t].push_back(ops[q]);
+            }
+        }
+    });
+    for (int t = 0; t < nt; ++t) {
+        packed.insert(packed.end(), ps[t].begin(), ps[t].end());
+        rest.insert(rest.end(), rs[t].begin(), rs[t].end());
+    }
+}
+
+int32_t pair_dst(int32_t key, bool two) { return two ? key : (int32_t)((uint32_t)key | FX_PAIR_ONE); }
+
+} // namespace
+
+void fx_pack_program(const FxProgram &g, FxPacked &out)
+{
+    out = FxPacked();
+    std::vector<FxBop> none;
+    for (auto &b : out.begin) b.assign(1, 0);
+    for (int w = 0; w < g.nwaves(); ++w) {
+        pack_range(g.cell_ops, g.cell_begin[w], g.cell_begin[w + 1], out.cp, out.cg,
+            [](const FxGop &a, const FxGop &b) {
+                return a.type == FX_GOP_COPY && b.type == FX_GOP_COPY && b.dst == a.dst + 1 && b.src == a.src + 1;
+            },
+            [](const FxGop &a, bool two, FxPair &x) {
+                x = FxPair{pair_dst(a.dst, two), a.src};
+                return a.type == FX_GOP_COPY;
+            });
+        pack_range(g.face_ops, g.face_begin[w], g.face_begin[w + 1], out.fp, out.fg,
+            [](const FxGop &a, const FxGop &b) {
+                return a.type == FX_FOP_COPY && b.type == FX_FOP_COPY && (a.aux & 3) == (b.aux & 3) &&
+                    b.dst == a.dst + 1 && b.src == a.src + 1;
+            },
+            [](const FxGop &a, bool two, FxPair &x) {
+                const int db = a.dst >> 15, sb = a.src >> 15;
+                x = FxPair{pair_dst(FX_PFACE(db, a.aux & 3, a.dst & 32767), two),
+                    FX_PFACE(sb, a.aux & 3, a.src & 32767)};
+                return a.type == FX_FOP_COPY && db < FX_PFACE_BLOCKS && sb < FX_PFACE_BLOCKS;
+            });
+        pack_range(g.b_ops, g.b_begin[w], g.b_begin[w + 1], out.b, none,
+            [](const FxBop &a, const FxBop &b) {
+                bool ok = b.dst == a.dst + 1;
+                for (int n = 0; n < 6; ++n) ok = ok && b.f[n] == a.f[n] + 1;
+                return ok;
+            },
+            [](const FxBop &a, bool two, FxBop &x) {
+                x = a;
+                x.pad = two ? 2 : 1;
+                return true;
+            });
+        out.begin[0].push_back((int)out.cp.size());
+        out.begin[1].push_back((int)out.cg.size());
+        out.begin[2].push_back((int)out.fp.size());
+        out.begin[3].push_back((int)out.fg.size());
+        out.begin[4].push_back((int)out.b.size());
+    }
+}
+
 bool fx_build_plan(const fx_config &cfg, int nblocks, const fx_block_desc *blocks,
     FxPlan &plan, std::string *err, FxPlanWorkspace *ws)
 {

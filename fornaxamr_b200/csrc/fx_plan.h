@@ -27,6 +27,18 @@ struct FxProgram {
     int nwaves() const { return cell_begin.empty() ? 0 : (int)cell_begin.size() - 1; }
 };
 
+/* The cell, face and cell-field operations of a program's waves sorted for
+ * the device (FxWave): neighbouring copies joined to pairs.  The operations
+ * of a wave are conflict free, so their order is free. */
+struct FxPacked {
+    std::vector<FxPair> cp, fp;
+    std::vector<FxGop> cg, fg;
+    std::vector<FxBop> b;
+    std::vector<int> begin[5]; /* per list (in FxWave's order): wave offsets, one more than waves */
+};
+
+void fx_pack_program(const FxProgram &g, FxPacked &out);
+
 struct FxPlanStats {
     long long emitted_cell_ops = 0; /* writes that land in the reference sequence */
     long long emitted_face_ops = 0;

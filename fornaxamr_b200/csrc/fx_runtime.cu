@@ -66,14 +66,19 @@ struct fx_ctx {
     int *d_ids = nullptr;
     int *d_active = nullptr;
     int nactive = 0;
-    FxGop *d_cops = nullptr, *d_fops = nullptr;
+    /* the ghost-fill program as the device runs it (FxWave) */
+    FxPair *d_cp = nullptr, *d_fp = nullptr;
+    FxGop *d_cg = nullptr, *d_fg = nullptr;
     FxPop *d_pops = nullptr;
     FxBop *d_bops = nullptr;
+    std::vector<FxWave> waves;
     FxCorr *d_fcorr = nullptr, *d_ecorr = nullptr;
-    /* element capacities of the seven program tables above (active list,
-     * cell / face / group / cell-field ops, flux / EMF records): an adapt
-     * reuses them when the new programs fit */
-    size_t tab_cap[7] = {0, 0, 0, 0, 0, 0, 0};
+    /* element capacities of the program tables (active list, cell and face
+     * copies, other cell / face ops, groups, cell-field ops, flux / EMF
+     * records): an adapt reuses them when the new programs fit */
+    size_t tab_cap[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    cudaStream_t side = nullptr;      /* a wave's face-prolongation groups, beside its copies */
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
 
     FxErr *d_err = nullptr;
     unsigned long long *d_red = nullptr;
@@ -99,6 +104,8 @@ struct fx_ctx {
     std::vector<int> adj_cbeg, adj_fbeg;
     FxAdjSrc *d_adj_csrc = nullptr, *d_adj_fsrc = nullptr;
     FxAdjEnt *d_adj_ents = nullptr;
+    FxGop *d_adj_cops = nullptr, *d_adj_fops = nullptr; /* the program's operations one by one */
+    FxBop *d_adj_bops = nullptr;
 
     /* decision record / replay of the plain form (fx_branch_trace) */
     unsigned long long *d_br_words = nullptr, *d_br_edges = nullptr;
@@ -246,12 +253,17 @@ void free_mesh(fx_ctx *c)
     c->d_W2 = c->d_Bf2 = nullptr;
     cudaFree(c->d_ids);
     cudaFree(c->d_active);
-    cudaFree(c->d_cops);
-    cudaFree(c->d_fops);
+    cudaFree(c->d_cp);
+    cudaFree(c->d_fp);
+    cudaFree(c->d_cg);
+    cudaFree(c->d_fg);
     cudaFree(c->d_pops);
     cudaFree(c->d_bops);
+    c->d_cp = c->d_fp = nullptr;
     c->d_pops = nullptr;
     c->d_bops = nullptr;
+    c->waves.clear();
+    c->compact_faces = false;
     cudaFree(c->d_fcorr);
     cudaFree(c->d_ecorr);
     for (size_t &cap : c->tab_cap) cap = 0;
@@ -259,7 +271,7 @@ void free_mesh(fx_ctx *c)
     c->d_W = c->d_Bf = c->d_flux = c->d_vr = c->d_vn = c->d_bv1 = c->d_bv2 = nullptr;
     c->d_emf = c->d_eos = c->d_rhs = c->d_grav = nullptr;
     c->d_ids = c->d_active = nullptr;
-    c->d_cops = c->d_fops = nullptr;
+    c->d_cg = c->d_fg = nullptr;
     c->d_fcorr = c->d_ecorr = nullptr;
     cudaFree(c->d_ckW);
     cudaFree(c->d_ckBf);
@@ -268,6 +280,11 @@ void free_mesh(fx_ctx *c)
     cudaFree(c->d_adj_csrc);
     cudaFree(c->d_adj_fsrc);
     cudaFree(c->d_adj_ents);
+    cudaFree(c->d_adj_cops);
+    cudaFree(c->d_adj_fops);
+    cudaFree(c->d_adj_bops);
+    c->d_adj_cops = c->d_adj_fops = nullptr;
+    c->d_adj_bops = nullptr;
     c->d_adj_csrc = c->d_adj_fsrc = nullptr;
     c->d_adj_ents = nullptr;
     c->adj_ghost_ready = false;
@@ -280,7 +297,6 @@ void free_mesh(fx_ctx *c)
     c->d_ckW = c->d_ckBf = c->d_Wb = c->d_Bfb = c->d_G = nullptr;
     c->d_bvb1 = c->d_bvb2 = c->d_Eb = nullptr;
     c->adj_nsteps = 0;
-    c->compact_faces = false;
     c->nblocks = 0;
     c->nactive = 0;
     c->cap = 0;
@@ -328,6 +344,18 @@ int local_block(fx_ctx *c, int *b)
     return FX_SUCCESS;
 }
 
+/* streams and events beside the context's own are made when first needed
+ * (each costs a context's set-up about a millisecond) */
+bool make_event(cudaEvent_t *e)
+{
+    return *e || cudaEventCreateWithFlags(e, cudaEventDisableTiming) == cudaSuccess;
+}
+
+bool make_stream(cudaStream_t *s)
+{
+    return *s || cudaStreamCreateWithFlags(s, cudaStreamNonBlocking) == cudaSuccess;
+}
+
 /* ---- phase sequencing ------------------------------------------------------ */
 
 template <typename F>
@@ -359,11 +387,17 @@ void ghost_fill(fx_ctx *c, int slot)
 {
     const FxProgram &g = c->plan.ghost;
     for (int w = 0; w < g.nwaves(); ++w) {
-        fx_launch_ghost_wave(c->D,
-            c->d_cops + g.cell_begin[w], g.cell_begin[w + 1] - g.cell_begin[w],
-            c->d_fops + g.face_begin[w], g.face_begin[w + 1] - g.face_begin[w],
-            c->d_pops + g.p_begin[w], g.p_begin[w + 1] - g.p_begin[w],
-            c->d_bops + g.b_begin[w], g.b_begin[w + 1] - g.b_begin[w], slot, 6, c->stream);
+        const int np = g.p_begin[w + 1] - g.p_begin[w];
+        /* the operations of a wave are conflict free: its groups (few, long
+         * threads that leave most SMs idle) run beside its copies */
+        if (np > 0) {
+            cudaEventRecord(c->ev_fork, c->stream);
+            cudaStreamWaitEvent(c->side, c->ev_fork, 0);
+            fx_launch_prolong_groups(c->D, c->d_pops + g.p_begin[w], np, slot, c->side);
+            cudaEventRecord(c->ev_join, c->side);
+        }
+        fx_launch_ghost_wave(c->D, c->waves[w], slot, c->stream);
+        if (np > 0) cudaStreamWaitEvent(c->stream, c->ev_join, 0);
     }
 }
 
@@ -751,12 +785,16 @@ int install_tables(fx_ctx *c)
     int rc;
     size_t *cap = c->tab_cap;
     if ((rc = dev_reserve(c, &c->d_active, &cap[0], (size_t)c->nactive))) return rc;
-    if ((rc = dev_reserve(c, &c->d_cops, &cap[1], c->plan.ghost.cell_ops.size()))) return rc;
-    if ((rc = dev_reserve(c, &c->d_fops, &cap[2], c->plan.ghost.face_ops.size()))) return rc;
-    if ((rc = dev_reserve(c, &c->d_pops, &cap[3], c->plan.ghost.p_ops.size()))) return rc;
-    if ((rc = dev_reserve(c, &c->d_bops, &cap[4], c->plan.ghost.b_ops.size()))) return rc;
-    if ((rc = dev_reserve(c, &c->d_fcorr, &cap[5], c->plan.flux_corr.size()))) return rc;
-    if ((rc = dev_reserve(c, &c->d_ecorr, &cap[6], c->plan.emf_corr.size()))) return rc;
+    FxPacked pk;
+    fx_pack_program(c->plan.ghost, pk);
+    if ((rc = dev_reserve(c, &c->d_cp, &cap[1], pk.cp.size()))) return rc;
+    if ((rc = dev_reserve(c, &c->d_fp, &cap[2], pk.fp.size()))) return rc;
+    if ((rc = dev_reserve(c, &c->d_cg, &cap[3], pk.cg.size()))) return rc;
+    if ((rc = dev_reserve(c, &c->d_fg, &cap[4], pk.fg.size()))) return rc;
+    if ((rc = dev_reserve(c, &c->d_pops, &cap[5], c->plan.ghost.p_ops.size()))) return rc;
+    if ((rc = dev_reserve(c, &c->d_bops, &cap[6], pk.b.size()))) return rc;
+    if ((rc = dev_reserve(c, &c->d_fcorr, &cap[7], c->plan.flux_corr.size()))) return rc;
+    if ((rc = dev_reserve(c, &c->d_ecorr, &cap[8], c->plan.emf_corr.size()))) return rc;
     cudaStream_t s = c->stream;
     const cudaMemcpyKind h2d = cudaMemcpyHostToDevice;
     FX_CUDA(c, cudaMemcpyAsync(c->d_blk, hb.data(), (size_t)nblocks * sizeof(FxBlockDev), h2d, s));
@@ -765,17 +803,33 @@ int install_tables(fx_ctx *c)
         FX_CUDA(c, cudaMemcpyAsync(c->d_active, c->plan.active.data(), (size_t)c->nactive * sizeof(int), h2d, s));
     }
     const FxProgram &g = c->plan.ghost;
-    if (!g.cell_ops.empty()) {
-        FX_CUDA(c, cudaMemcpyAsync(c->d_cops, g.cell_ops.data(), g.cell_ops.size() * sizeof(FxGop), h2d, s));
+    auto put = [&](void *dst, const void *src, size_t bytes) {
+        return bytes ? cudaMemcpyAsync(dst, src, bytes, h2d, s) : cudaSuccess;
+    };
+    FX_CUDA(c, put(c->d_cp, pk.cp.data(), pk.cp.size() * sizeof(FxPair)));
+    FX_CUDA(c, put(c->d_fp, pk.fp.data(), pk.fp.size() * sizeof(FxPair)));
+    FX_CUDA(c, put(c->d_cg, pk.cg.data(), pk.cg.size() * sizeof(FxGop)));
+    FX_CUDA(c, put(c->d_fg, pk.fg.data(), pk.fg.size() * sizeof(FxGop)));
+    FX_CUDA(c, put(c->d_pops, g.p_ops.data(), g.p_ops.size() * sizeof(FxPop)));
+    FX_CUDA(c, put(c->d_bops, pk.b.data(), pk.b.size() * sizeof(FxBop)));
+    if (!g.p_ops.empty() && !(make_stream(&c->side) && make_event(&c->ev_fork) && make_event(&c->ev_join))) {
+        return set_err(c, FX_ECUDA, "cannot make the ghost fill's second stream");
     }
-    if (!g.face_ops.empty()) {
-        FX_CUDA(c, cudaMemcpyAsync(c->d_fops, g.face_ops.data(), g.face_ops.size() * sizeof(FxGop), h2d, s));
-    }
-    if (!g.p_ops.empty()) {
-        FX_CUDA(c, cudaMemcpyAsync(c->d_pops, g.p_ops.data(), g.p_ops.size() * sizeof(FxPop), h2d, s));
-    }
-    if (!g.b_ops.empty()) {
-        FX_CUDA(c, cudaMemcpyAsync(c->d_bops, g.b_ops.data(), g.b_ops.size() * sizeof(FxBop), h2d, s));
+    c->waves.clear();
+    for (int w = 0; w < g.nwaves(); ++w) {
+        auto n = [&](int l) { return pk.begin[l][w + 1] - pk.begin[l][w]; };
+        FxWave v{};
+        v.ncp = n(0);
+        v.ncg = n(1);
+        v.nfp = n(2);
+        v.nfg = n(3);
+        v.nb = n(4);
+        v.cp = c->d_cp + pk.begin[0][w];
+        v.cg = c->d_cg + pk.begin[1][w];
+        v.fp = c->d_fp + pk.begin[2][w];
+        v.fg = c->d_fg + pk.begin[3][w];
+        v.b = c->d_bops + pk.begin[4][w];
+        c->waves.push_back(v);
     }
     if (!c->plan.flux_corr.empty()) {
         FX_CUDA(c, cudaMemcpyAsync(c->d_fcorr, c->plan.flux_corr.data(),
@@ -937,6 +991,11 @@ void drop_adjoint(fx_ctx *c)
     cudaFree(c->d_adj_csrc);
     cudaFree(c->d_adj_fsrc);
     cudaFree(c->d_adj_ents);
+    cudaFree(c->d_adj_cops);
+    cudaFree(c->d_adj_fops);
+    cudaFree(c->d_adj_bops);
+    c->d_adj_cops = c->d_adj_fops = nullptr;
+    c->d_adj_bops = nullptr;
     cudaFree(c->d_Wb);
     cudaFree(c->d_Bfb);
     cudaFree(c->d_G);
@@ -1046,6 +1105,9 @@ void fx_destroy(fx_ctx *c)
     cudaFreeHost(c->h_err);
     cudaFreeHost(c->h_red);
     cudaFreeHost(c->h_ctl);
+    if (c->ev_fork) cudaEventDestroy(c->ev_fork);
+    if (c->ev_join) cudaEventDestroy(c->ev_join);
+    if (c->side) cudaStreamDestroy(c->side);
     if (c->stream) {
         cudaStreamDestroy(c->stream);
     }
@@ -2433,7 +2495,13 @@ int build_adj_ghost(fx_ctx *c)
     if ((rc = dev_alloc(c, &c->d_adj_csrc, cs.size()))) return rc;
     if ((rc = dev_alloc(c, &c->d_adj_fsrc, fs.size()))) return rc;
     if ((rc = dev_alloc(c, &c->d_adj_ents, ents.size()))) return rc;
+    if ((rc = dev_alloc(c, &c->d_adj_cops, g.cell_ops.size()))) return rc;
+    if ((rc = dev_alloc(c, &c->d_adj_fops, g.face_ops.size()))) return rc;
+    if ((rc = dev_alloc(c, &c->d_adj_bops, g.b_ops.size()))) return rc;
     const cudaMemcpyKind h2d = cudaMemcpyHostToDevice;
+    if (!g.cell_ops.empty()) FX_CUDA(c, cudaMemcpyAsync(c->d_adj_cops, g.cell_ops.data(), g.cell_ops.size() * sizeof(FxGop), h2d, c->stream));
+    if (!g.face_ops.empty()) FX_CUDA(c, cudaMemcpyAsync(c->d_adj_fops, g.face_ops.data(), g.face_ops.size() * sizeof(FxGop), h2d, c->stream));
+    if (!g.b_ops.empty()) FX_CUDA(c, cudaMemcpyAsync(c->d_adj_bops, g.b_ops.data(), g.b_ops.size() * sizeof(FxBop), h2d, c->stream));
     if (!cs.empty()) FX_CUDA(c, cudaMemcpyAsync(c->d_adj_csrc, cs.data(), cs.size() * sizeof(FxAdjSrc), h2d, c->stream));
     if (!fs.empty()) FX_CUDA(c, cudaMemcpyAsync(c->d_adj_fsrc, fs.data(), fs.size() * sizeof(FxAdjSrc), h2d, c->stream));
     if (!ents.empty()) FX_CUDA(c, cudaMemcpyAsync(c->d_adj_ents, ents.data(), ents.size() * sizeof(FxAdjEnt), h2d, c->stream));
@@ -2450,9 +2518,9 @@ void adj_ghost(fx_ctx *c, const FxAdjDev &A, int slot)
     for (int w = g.nwaves() - 1; w >= 0; --w) {
         fx_launch_adj_gather(A, c->d_adj_csrc + c->adj_cbeg[w], c->adj_cbeg[w + 1] - c->adj_cbeg[w],
             c->d_adj_fsrc + c->adj_fbeg[w], c->adj_fbeg[w + 1] - c->adj_fbeg[w], c->d_adj_ents, slot, c->stream);
-        fx_launch_adj_zero(A, c->d_cops + g.cell_begin[w], g.cell_begin[w + 1] - g.cell_begin[w],
-            c->d_fops + g.face_begin[w], g.face_begin[w + 1] - g.face_begin[w],
-            c->d_bops + g.b_begin[w], g.b_begin[w + 1] - g.b_begin[w], slot, c->stream);
+        fx_launch_adj_zero(A, c->d_adj_cops + g.cell_begin[w], g.cell_begin[w + 1] - g.cell_begin[w],
+            c->d_adj_fops + g.face_begin[w], g.face_begin[w + 1] - g.face_begin[w],
+            c->d_adj_bops + g.b_begin[w], g.b_begin[w + 1] - g.b_begin[w], slot, c->stream);
     }
 }
 

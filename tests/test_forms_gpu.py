@@ -84,3 +84,64 @@ def test_plain_entry_points_after_a_batched_step():
         for q in (0, 1):
             a, b = (g[1][3 * q + d].reshape(20, 20, 20) for g in got)
             assert np.array_equal(a[m], b[m])
+
+
+def _run_both(blocks, coord, W, Bf, steps=2, **kw):
+    out = []
+    ns = 3 if kw.get("integrator") == fx.INT_ESSPRK10_4 else 2
+    for form in (fx.FORM_PLAIN, fx.FORM_BATCHED):
+        ctx = fx.Context(Bf is not None, 5.0 / 3.0, coord, **kw)
+        ctx.set_mesh(mesh.to_desc(blocks))
+        for b in range(len(blocks)):
+            w = np.zeros((W.shape[1], ns, W.shape[3]))
+            w[:, :2] = W[b]
+            f = None
+            if Bf is not None:
+                f = np.zeros((3, ns, Bf.shape[3]))
+                f[:, :2] = Bf[b]
+                f = [x.ravel() for x in f]
+            ctx.upload_block(b, w.ravel(), f)
+        ctx.boundary_fill(1, 0)
+        clock = ctx.run(form, steps, 0.4, 1.2, 1.0e30, (0.0, 0.0, 0))
+        act = [b for b in range(len(blocks)) if blocks[b].active == 1]
+        flux = [ctx.download_array(b, fx.ARR_FLUX, d) for b in (act[0], act[-1]) for d in range(3)]
+        out.append((clock, [ctx.download_block(b) for b in act], flux))
+        ctx.close()
+    assert out[0][0] == out[1][0]
+    for (Wa, ea, Ba), (Wb, eb, Bb) in zip(out[0][1], out[1][1]):
+        assert np.array_equal(Wa, Wb) and np.array_equal(ea, eb)
+        for d in range(3 if Bf is not None else 0):
+            assert np.array_equal(Ba[d], Bb[d])
+    nv = W.shape[1]
+    for n, (a, b) in enumerate(zip(out[0][2], out[1][2])):
+        d = n % 3
+        core = tuple(slice(2, 19 if q == d else 18) for q in range(3))
+        for v in range(6):
+            x, y = (f.reshape(20, 20, 5, nv, 4)[:, :, :, v].reshape(20, 20, 20)[core] for f in (a, b))
+            assert np.array_equal(x, y)
+
+
+AMR_COORD = (-0.7, 0.7, -0.7, 0.7, -0.7, 0.7)
+
+
+@pytest.mark.parametrize("mhd", [True, False])
+@pytest.mark.parametrize("use_bj", [False, True])
+def test_amr_steps_of_both_forms_are_the_same(mhd, use_bj):
+    """Three levels: corrections on the compact fluxes, waves with pairs,
+    single operations and face-prolongation groups."""
+    blocks = mesh.static_amr_mesh((3,) * 3, AMR_COORD, 2, mesh.ball_refiner((0.1, 0.05, 0.0), (0.4, 0.2)))
+    recs = fx.plan_export(fx.make_config(mhd, 5.0 / 3.0, AMR_COORD), mesh.to_desc(blocks), 3) if mhd else None
+    W, Bf = problems.amr_blast(blocks, recs, mhd=mhd)
+    _run_both(blocks, AMR_COORD, W, Bf, use_bj=use_bj)
+
+
+@pytest.mark.parametrize("root", [(1, 1, 1), (2, 3, 3)])
+@pytest.mark.parametrize("recon,integ", [(fx.RECON_MC, fx.INT_RK2), (fx.RECON_WENO3, fx.INT_RK2),
+                                         (fx.RECON_MC, fx.INT_ESSPRK10_4)])
+@pytest.mark.parametrize("mhd", [True, False])
+def test_uniform_steps_of_both_forms_are_the_same(root, recon, integ, mhd):
+    blocks = mesh.uniform_mesh(root, COORD)
+    W, Bf = problems.fourier_mhd(blocks, nmodes=4, kmax=3)
+    if not mhd:
+        W, Bf = np.ascontiguousarray(W[:, :6]), None
+    _run_both(blocks, COORD, W, Bf, recon=recon, integrator=integ)
