@@ -41,6 +41,11 @@ struct FxXdev {
 };
 enum { FX_XG = 0, FX_XF = 1, FX_XE = 2 }; /* ghost fill (cells + faces), flux, EMF */
 
+/* streams of the plain form: one block's launch fills a fraction of the
+ * device for a few microseconds, so one after the other they cost their
+ * latency each */
+constexpr int FX_LANES = 8;
+
 struct fx_ctx {
     int device = 0;
     fx_config cfg{};
@@ -77,6 +82,11 @@ struct fx_ctx {
      * copies, other cell / face ops, groups, cell-field ops, flux / EMF
      * records): an adapt reuses them when the new programs fit */
     size_t tab_cap[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    /* the plain form's per-block launches take turns on these streams (a
+     * block always on the same one) between lanes_open and lanes_close */
+    cudaStream_t lane[FX_LANES] = {};
+    cudaEvent_t ev_lane[FX_LANES] = {};
+    bool lanes = false;
     cudaStream_t side = nullptr;      /* a wave's face-prolongation groups, beside its copies */
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
 
@@ -356,17 +366,49 @@ bool make_stream(cudaStream_t *s)
     return *s || cudaStreamCreateWithFlags(s, cudaStreamNonBlocking) == cudaSuccess;
 }
 
+bool make_lanes(fx_ctx *c)
+{
+    bool ok = make_event(&c->ev_fork);
+    for (int l = 0; ok && l < FX_LANES; ++l) ok = make_stream(&c->lane[l]) && make_event(&c->ev_lane[l]);
+    return ok;
+}
+
 /* ---- phase sequencing ------------------------------------------------------ */
 
+/* The plain form's per-block launches of consecutive phases are independent
+ * from block to block (each reads and writes its own block), so between
+ * lanes_open and lanes_close they run on FX_LANES streams, each block's in
+ * order on one of them.  What couples blocks (corrections, the ghost fill,
+ * reductions read by the host) runs on the context's stream after
+ * lanes_close. */
+void lanes_open(fx_ctx *c, int form)
+{
+    if (form != FX_FORM_PLAIN || c->lanes || c->plan.active.size() < 2 || !make_lanes(c)) return;
+    cudaEventRecord(c->ev_fork, c->stream);
+    for (cudaStream_t l : c->lane) cudaStreamWaitEvent(l, c->ev_fork, 0);
+    c->lanes = true;
+}
+
+void lanes_close(fx_ctx *c)
+{
+    if (!c->lanes) return;
+    for (int l = 0; l < FX_LANES; ++l) {
+        cudaEventRecord(c->ev_lane[l], c->lane[l]);
+        cudaStreamWaitEvent(c->stream, c->ev_lane[l], 0);
+    }
+    c->lanes = false;
+}
+
+/* fn(block list, its length, stream) */
 template <typename F>
 void per_block(fx_ctx *c, int form, F &&fn)
 {
     if (form == FX_FORM_PLAIN) {
-        for (int b : c->plan.active) {
-            fn(c->d_ids + b, 1);
+        for (size_t q = 0; q < c->plan.active.size(); ++q) {
+            fn(c->d_ids + c->plan.active[q], 1, c->lanes ? c->lane[q % FX_LANES] : c->stream);
         }
     } else {
-        fn(c->d_active, c->nactive);
+        fn(c->d_active, c->nactive, c->stream);
     }
 }
 
@@ -449,13 +491,59 @@ void shard_min(fx_ctx *c, int first, int count)
     if (c->transport->min_u64(c->d_red + first, count, c->stream)) c->xerr = c->transport->err;
 }
 
+/* the fill of W slot `slot` between stages: eos (active) -> ghost fill ->
+ * eos (mesh), the eosvar arrays in the plain form only */
+void refill(fx_ctx *c, int form, int slot)
+{
+    if (form == FX_FORM_PLAIN) {
+        lanes_open(c, form);
+        per_block(c, form, [&](const int *l, int n, cudaStream_t s) { fx_launch_eos_fill(c->D, l, n, slot, 1, s); });
+        lanes_close(c);
+    }
+    shard_exchange(c, FX_XG, slot);
+    ghost_fill(c, slot);
+    if (form == FX_FORM_PLAIN) {
+        lanes_open(c, form);
+        per_block(c, form, [&](const int *l, int n, cudaStream_t s) { fx_launch_eos_fill(c->D, l, n, slot, 0, s); });
+        lanes_close(c);
+    }
+}
+
+/* the phases of a stage: fluxes and EMFs of W slot wslot and field slot
+ * bfslot, the CT and cell updates of `stage`, the fill of slot dst */
+void stage_phases(fx_ctx *c, int form, int wslot, int bfslot, int stage, int dst)
+{
+    const int full = form == FX_FORM_PLAIN ? 1 : 0;
+    lanes_open(c, form);
+    per_block(c, form, [&](const int *l, int n, cudaStream_t s) { fx_launch_flux(c->D, l, n, 3, wslot, bfslot, full, s); });
+    c->compact_faces = !full;
+    shard_exchange(c, FX_XF, wslot);
+    if (!c->plan.flux_corr.empty()) {
+        lanes_close(c);
+        flux_correct(c, full ? c->nv : 6, c->stream);
+        lanes_open(c, form);
+    }
+    if (c->cfg.mhd) {
+        per_block(c, form, [&](const int *l, int n, cudaStream_t s) { fx_launch_emf(c->D, l, n, wslot, bfslot, full, s); });
+        shard_exchange(c, FX_XE, wslot);
+        if (!c->plan.emf_corr.empty()) {
+            lanes_close(c);
+            emf_correct(c, c->stream);
+            lanes_open(c, form);
+        }
+        per_block(c, form, [&](const int *l, int n, cudaStream_t s) { fx_launch_bf_update(c->D, l, n, stage, s); });
+    }
+    per_block(c, form, [&](const int *l, int n, cudaStream_t s) {
+        fx_launch_cell_update(c->D, l, n, stage, c->cfg.gravity, full, s);
+    });
+    refill(c, form, dst);
+}
+
 /* one RK2 stage; dt is read from the control block */
 void stage_seq(fx_ctx *c, int form, int stage)
 {
     const int src = stage == 1 ? 0 : 1; /* W / Bf slot the fluxes read */
     const int dst = stage == 1 ? 1 : 0; /* W slot the update writes */
-    cudaStream_t s = c->stream;
-    const int full = form == FX_FORM_PLAIN ? 1 : 0;
     /* decisions are recorded / replayed by the plain form only, one slot
      * of the buffers per stage */
     const int br_mode = c->D.br_mode;
@@ -472,74 +560,30 @@ void stage_seq(fx_ctx *c, int form, int stage)
             if (br_mode == FX_BRANCH_RECORD) c->br_recorded = c->br_stage;
         }
     }
-    per_block(c, form, [&](const int *l, int n) { fx_launch_flux(c->D, l, n, 3, src, src, full, s); });
-    c->compact_faces = !full;
-    shard_exchange(c, FX_XF, src);
-    flux_correct(c, full ? c->nv : 6, s);
-    if (c->cfg.mhd) {
-        per_block(c, form, [&](const int *l, int n) { fx_launch_emf(c->D, l, n, src, src, full, s); });
-        shard_exchange(c, FX_XE, src);
-        emf_correct(c, s);
-        per_block(c, form, [&](const int *l, int n) { fx_launch_bf_update(c->D, l, n, stage, s); });
-    }
-    per_block(c, form, [&](const int *l, int n) {
-        fx_launch_cell_update(c->D, l, n, stage, c->cfg.gravity, full, s);
-    });
-    if (form == FX_FORM_PLAIN) {
-        per_block(c, form, [&](const int *l, int n) { fx_launch_eos_fill(c->D, l, n, dst, 1, s); });
-    }
-    shard_exchange(c, FX_XG, dst);
-    ghost_fill(c, dst);
-    if (form == FX_FORM_PLAIN) {
-        per_block(c, form, [&](const int *l, int n) { fx_launch_eos_fill(c->D, l, n, dst, 0, s); });
-    }
+    stage_phases(c, form, src, src, stage, dst);
     c->last_slot = dst;
     if (!c->br_overflow) c->D.br_mode = br_mode;
-}
-
-/* the refill after a substep or a blend: eos (active) -> ghost fill -> eos
- * (mesh) on slot 0 */
-void refill0(fx_ctx *c, int form)
-{
-    cudaStream_t s = c->stream;
-    if (form == FX_FORM_PLAIN) {
-        per_block(c, form, [&](const int *l, int n) { fx_launch_eos_fill(c->D, l, n, 0, 1, s); });
-    }
-    ghost_fill(c, 0);
-    if (form == FX_FORM_PLAIN) {
-        per_block(c, form, [&](const int *l, int n) { fx_launch_eos_fill(c->D, l, n, 0, 0, s); });
-    }
 }
 
 /* one forward-Euler substep in place on slot 0, prj_timeint_eSSPRK_step
  * (src/prj_timeint.c:2452-2550); dt_stage holds dt / 6 */
 void essprk_substep(fx_ctx *c, int form)
 {
-    cudaStream_t s = c->stream;
-    const int full = form == FX_FORM_PLAIN ? 1 : 0;
-    per_block(c, form, [&](const int *l, int n) { fx_launch_flux(c->D, l, n, 3, 0, 0, full, s); });
-    c->compact_faces = !full;
-    flux_correct(c, full ? c->nv : 6, s);
-    if (c->cfg.mhd) {
-        per_block(c, form, [&](const int *l, int n) { fx_launch_emf(c->D, l, n, 0, 0, full, s); });
-        emf_correct(c, s);
-        per_block(c, form, [&](const int *l, int n) { fx_launch_bf_update(c->D, l, n, 0, s); });
-    }
-    per_block(c, form, [&](const int *l, int n) {
-        fx_launch_cell_update(c->D, l, n, 0, c->cfg.gravity, full, s);
-    });
-    refill0(c, form);
+    stage_phases(c, form, 0, 0, 0, 0);
 }
 
 void essprk_blend(fx_ctx *c, int form, int which, double w)
 {
-    per_block(c, form, [&](const int *l, int n) { fx_launch_essprk_blend(c->D, l, n, which, w, c->stream); });
-    refill0(c, form);
+    lanes_open(c, form);
+    per_block(c, form, [&](const int *l, int n, cudaStream_t s) { fx_launch_essprk_blend(c->D, l, n, which, w, s); });
+    refill(c, form, 0);
 }
 
 void essprk_save(fx_ctx *c, int form, int which)
 {
-    per_block(c, form, [&](const int *l, int n) { fx_launch_essprk_save(c->D, l, n, which, c->stream); });
+    lanes_open(c, form);
+    per_block(c, form, [&](const int *l, int n, cudaStream_t s) { fx_launch_essprk_save(c->D, l, n, which, s); });
+    lanes_close(c);
 }
 
 /* prj_timeint_eSSPRK10_4_advance (src/prj_timeint.c:2671-2729): Ketcheson's
@@ -1105,6 +1149,12 @@ void fx_destroy(fx_ctx *c)
     cudaFreeHost(c->h_err);
     cudaFreeHost(c->h_red);
     cudaFreeHost(c->h_ctl);
+    for (cudaStream_t l : c->lane) {
+        if (l) cudaStreamDestroy(l);
+    }
+    for (cudaEvent_t e : c->ev_lane) {
+        if (e) cudaEventDestroy(e);
+    }
     if (c->ev_fork) cudaEventDestroy(c->ev_fork);
     if (c->ev_join) cudaEventDestroy(c->ev_join);
     if (c->side) cudaStreamDestroy(c->side);
