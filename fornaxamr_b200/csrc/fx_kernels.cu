@@ -291,9 +291,20 @@ __global__ void __launch_bounds__(TPB, MINB) k_flux(FxDev D, const int *__restri
                 atomicAdd(D.br_flips, (unsigned long long)br.flips);
             }
         }
+        if constexpr (FULL) {
 #pragma unroll
-        for (int lv = 0; lv < (FULL ? 9 : 6); ++lv) {
-            D.flux[fbase + fx_bidx(9, fx_gmap(dir, lv), i, j, k)] = o.F[lv];
+            for (int lv = 0; lv < 9; ++lv) {
+                D.flux[fbase + fx_bidx(9, fx_gmap(dir, lv), i, j, k)] = o.F[lv];
+            }
+        } else if ((unsigned)i < (dir == 0 ? FX_BS + 1u : FX_BS) && (unsigned)j < (dir == 1 ? FX_BS + 1u : FX_BS) &&
+            (unsigned)k < (dir == 2 ? FX_BS + 1u : FX_BS)) {
+            /* the transverse ghost ring serves the EMFs only */
+            double *cf = D.cf + (size_t)b * FX_CF_COUNT + fx_cf_idx(dir, i, j, k);
+            const int plane = fx_cf_plane(dir);
+#pragma unroll
+            for (int lv = 0; lv < 6; ++lv) {
+                cf[fx_gmap(dir, lv) * plane] = o.F[lv];
+            }
         }
         const size_t bvi = (size_t)b * FX_BV_COUNT + (size_t)dir * FX_NCELLS + cR;
         if constexpr (FULL) {
@@ -329,9 +340,15 @@ __global__ void __launch_bounds__(TPB, MINB) k_flux(FxDev D, const int *__restri
         double F[6];
         double v[3];
         fx_riemann_hllc(WL, WR, pL, pR, gL, gR, du, dv, dw, F, v);
+        double *cf = D.cf + (size_t)b * FX_CF_COUNT + fx_cf_idx(dir, i, j, k);
+        const int plane = fx_cf_plane(dir);
 #pragma unroll
         for (int lv = 0; lv < 6; ++lv) {
-            D.flux[fbase + fx_bidx(6, fx_gmap(dir, lv), i, j, k)] = F[lv];
+            if constexpr (FULL) {
+                D.flux[fbase + fx_bidx(6, fx_gmap(dir, lv), i, j, k)] = F[lv];
+            } else {
+                cf[fx_gmap(dir, lv) * plane] = F[lv];
+            }
         }
         if constexpr (FULL) {
 #pragma unroll
@@ -801,18 +818,31 @@ __global__ void __launch_bounds__(128) k_cell_update(FxDev D, const int *__restr
     const int c = fx_lidx(i, j, k);
     const FxBlockDev &B = D.blk[b];
     const double *W = D.W + (size_t)b * FX_W_COUNT(nv);
-    const double *fx = D.flux + (size_t)b * FX_FLUX_COUNT(nv);
-    const double *fy = fx + (size_t)nv * FX_NCELLS;
-    const double *fz = fy + (size_t)nv * FX_NCELLS;
 
     /* prj_flux_div, src/prj_flux.c:2523-2533 (hydro components; the B
      * components are replaced by the face average below) */
     double fluxdiv[6];
 #pragma unroll
     for (int v = 0; v < 6; ++v) {
-        fluxdiv[v] = -(B.area[0] * (fx[fx_bidx(nv, v, i + 1, j, k)] - fx[fx_bidx(nv, v, i, j, k)]) +
-            B.area[1] * (fy[fx_bidx(nv, v, i, j + 1, k)] - fy[fx_bidx(nv, v, i, j, k)]) +
-            B.area[2] * (fz[fx_bidx(nv, v, i, j, k + 1)] - fz[fx_bidx(nv, v, i, j, k)])) / B.vol;
+        double f[3][2];
+        if constexpr (FULL) {
+            const double *fl = D.flux + (size_t)b * FX_FLUX_COUNT(nv);
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                f[d][0] = fl[(size_t)d * nv * FX_NCELLS + fx_bidx(nv, v, i, j, k)];
+                f[d][1] = fl[(size_t)d * nv * FX_NCELLS + fx_bidx(nv, v, i + (d == 0), j + (d == 1), k + (d == 2))];
+            }
+        } else {
+            const double *cf = D.cf + (size_t)b * FX_CF_COUNT;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                const double *q = cf + v * fx_cf_plane(d) + fx_cf_idx(d, i, j, k);
+                f[d][0] = q[0];
+                f[d][1] = q[d == 0 ? FX_BS * FX_BS : d == 1 ? FX_BS : 1];
+            }
+        }
+        fluxdiv[v] = -(B.area[0] * (f[0][1] - f[0][0]) + B.area[1] * (f[1][1] - f[1][0]) +
+            B.area[2] * (f[2][1] - f[2][0])) / B.vol;
     }
 
     double w[9];
@@ -1559,6 +1589,20 @@ __global__ void __launch_bounds__(256, BJ ? 4 : 6) k_ghost_wave(FxDev D, FxWave 
     }
 }
 
+/* compact position (variable 0, and the stride between variables) of a flux
+ * entry given as direction * nv * cells + AoSoA index of component 0 */
+__device__ __forceinline__ int fx_cf_of_entry(int nv, int entry, int &plane)
+{
+    const int dir = entry / (nv * FX_NCELLS);
+    const int r = entry - dir * nv * FX_NCELLS;
+    const int u = r / (FX_AOSOA_W * nv);
+    const int row = u / FX_AOSOA_KT;
+    const int k = (u - row * FX_AOSOA_KT) * FX_AOSOA_W + r % FX_AOSOA_W - FX_NG;
+    const int i = row / FX_PBS;
+    plane = fx_cf_plane(dir);
+    return fx_cf_idx(dir, i - FX_NG, row - i * FX_PBS - FX_NG, k);
+}
+
 /* exchanges of a sharded mesh: one thread per listed element */
 __device__ __forceinline__ double *fx_xelem(const FxDev &D, const FxXent &x, int slot, int q)
 {
@@ -1570,8 +1614,11 @@ __device__ __forceinline__ double *fx_xelem(const FxDev &D, const FxXent &x, int
         return D.Bf + (size_t)x.block * FX_BF_COUNT + ((size_t)dir * FX_NSTAGES + slot) * FX_NFACES +
             (x.idx - dir * FX_NFACES);
     }
-    case 2:
-        return D.flux + (size_t)x.block * FX_FLUX_COUNT(D.nv) + x.idx + (size_t)q * FX_AOSOA_W;
+    case 2: {
+        int plane;
+        const int e = fx_cf_of_entry(D.nv, x.idx, plane);
+        return D.cf + (size_t)x.block * FX_CF_COUNT + e + q * plane;
+    }
     default:
         return D.emf + (size_t)x.block * FX_EMF_COUNT + x.idx;
     }
@@ -1595,7 +1642,9 @@ __global__ void k_xunpack(FxDev D, const FxXent *__restrict__ ents, int n, const
     for (int q = 0; q < fx_xwidth(x.kind); ++q) *fx_xelem(D, x, slot, q) = buf[x.off + q];
 }
 
-/* coarse/fine corrections */
+/* coarse/fine corrections; FULL: in the plain form's flux arrays, else the
+ * batched form's */
+template <bool FULL>
 __global__ void k_flux_correct(FxDev D, const FxCorr *__restrict__ recs, int n, int ncomp)
 {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1605,12 +1654,25 @@ __global__ void k_flux_correct(FxDev D, const FxCorr *__restrict__ recs, int n, 
     const int r = t / ncomp;
     const int v = t - r * ncomp;
     const FxCorr rec = recs[r];
-    /* entries index component 0 of a block's stacked flux array; component
-     * v sits FX_AOSOA_W * v further in the AoSoA tile.  Sum order of
-     * src/prj_riemann.c:1756-1761. */
-    const double *s = D.flux + (size_t)rec.src_block * FX_FLUX_COUNT(D.nv) + (size_t)v * FX_AOSOA_W;
-    double *d = D.flux + (size_t)rec.dst_block * FX_FLUX_COUNT(D.nv) + (size_t)v * FX_AOSOA_W;
-    d[rec.dst] = 0.25 * (s[rec.src[0]] + s[rec.src[1]] + s[rec.src[2]] + s[rec.src[3]]);
+    /* sum order of src/prj_riemann.c:1756-1761 */
+    if constexpr (FULL) {
+        /* component v sits FX_AOSOA_W * v further in the AoSoA tile */
+        const double *s = D.flux + (size_t)rec.src_block * FX_FLUX_COUNT(D.nv) + (size_t)v * FX_AOSOA_W;
+        double *d = D.flux + (size_t)rec.dst_block * FX_FLUX_COUNT(D.nv) + (size_t)v * FX_AOSOA_W;
+        d[rec.dst] = 0.25 * (s[rec.src[0]] + s[rec.src[1]] + s[rec.src[2]] + s[rec.src[3]]);
+    } else {
+        const double *s = D.cf + (size_t)rec.src_block * FX_CF_COUNT;
+        double f[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            int plane;
+            const int e = fx_cf_of_entry(D.nv, rec.src[q], plane);
+            f[q] = s[e + v * plane];
+        }
+        int plane;
+        const int e = fx_cf_of_entry(D.nv, rec.dst, plane);
+        D.cf[(size_t)rec.dst_block * FX_CF_COUNT + e + v * plane] = 0.25 * (f[0] + f[1] + f[2] + f[3]);
+    }
 }
 
 __global__ void k_emf_correct(FxDev D, const FxCorr *__restrict__ recs, int n)
@@ -1949,8 +2011,15 @@ __global__ void __launch_bounds__(256) k_expand_faces(FxDev D, const int *__rest
         return;
     }
     const int b = blist[blockIdx.y];
+    const int i = t / (FX_PBS * FX_PBS) - FX_NG, j = (t / FX_PBS) % FX_PBS - FX_NG, k = t % FX_PBS - FX_NG;
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
+        if (i >= 0 && j >= 0 && k >= 0 && i < FX_BS + (d == 0) && j < FX_BS + (d == 1) && k < FX_BS + (d == 2)) {
+            for (int v = 0; v < 6; ++v) {
+                D.flux[(size_t)b * FX_FLUX_COUNT(D.nv) + (size_t)d * D.nv * FX_NCELLS + fx_bidx(D.nv, v, i, j, k)] =
+                    D.cf[(size_t)b * FX_CF_COUNT + v * fx_cf_plane(d) + fx_cf_idx(d, i, j, k)];
+            }
+        }
         D.vr[(size_t)b * FX_VR_COUNT + d * 3 * FX_NCELLS + fx_bidx_cell(3, d, t)] =
             D.vn[(size_t)b * FX_VN_COUNT + d * FX_NCELLS + t];
     }
@@ -2055,10 +2124,12 @@ void fx_launch_prolong_groups(const FxDev &D, const FxPop *pops, int np, int slo
     }
 }
 
-void fx_launch_flux_correct(const FxDev &D, const FxCorr *recs, int n, int ncomp, cudaStream_t s)
+void fx_launch_flux_correct(const FxDev &D, const FxCorr *recs, int n, int ncomp, int full, cudaStream_t s)
 {
     if (n <= 0) return;
-    k_flux_correct<<<fx_blocks(n * ncomp, 256), 256, 0, s>>>(D, recs, n, ncomp);
+    const unsigned grid = fx_blocks(n * ncomp, 256);
+    if (full) k_flux_correct<true><<<grid, 256, 0, s>>>(D, recs, n, ncomp);
+    else k_flux_correct<false><<<grid, 256, 0, s>>>(D, recs, n, ncomp);
 }
 
 void fx_launch_emf_correct(const FxDev &D, const FxCorr *recs, int n, cudaStream_t s)

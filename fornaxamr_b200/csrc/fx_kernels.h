@@ -48,6 +48,7 @@ struct FxDev {
     double *Bf;   /* [b][dir][stage][face]         (FACE_IDX) */
     double *flux; /* [b][dir][AoSoA nc=nv]         (VIDX) */
     double *vr;   /* [b][dir][AoSoA nc=3]          (VRIDX) */
+    double *cf;   /* the batched form's face fluxes [b][...] (fx_cf_idx) */
     /* the batched form's face velocities, normal component only: the
      * reference's AoSoA tile holds three components of which later phases
      * read one, and DRAM moves whole tiles */
@@ -238,7 +239,8 @@ void fx_launch_xunpack(const FxDev &D, const FxXent *ents, int n, const double *
 void fx_launch_dump_pack(const FxDev &D, const int *blist, int nlist, int faces, double *out, cudaStream_t s);
 /* cell-centred field of the listed blocks' active cells from the faces (slot 0) */
 void fx_launch_cell_field_active(const FxDev &D, const int *blist, int nlist, cudaStream_t s);
-void fx_launch_flux_correct(const FxDev &D, const FxCorr *recs, int n, int ncomp, cudaStream_t s);
+/* full: in the plain form's flux arrays, else the batched form's */
+void fx_launch_flux_correct(const FxDev &D, const FxCorr *recs, int n, int ncomp, int full, cudaStream_t s);
 void fx_launch_emf_correct(const FxDev &D, const FxCorr *recs, int n, cudaStream_t s);
 void fx_launch_reset_reductions(const FxDev &D, int which, cudaStream_t s);
 /* device-resident driver: dt selection before a step, dt_src clamp and time

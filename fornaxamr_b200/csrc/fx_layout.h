@@ -94,6 +94,25 @@ FX_HD int fx_bidx_cell(int nc, int v, int cell)
     return ((row * FX_AOSOA_KT + kk / FX_AOSOA_W) * nc + v) * FX_AOSOA_W + kk % FX_AOSOA_W;
 }
 
+/* Face fluxes of the batched form, [dir][variable 0-5][i][j][k]: the faces of
+ * the block itself only, in rows of 16 (20 along the sweep direction 2, 17 of
+ * them used), so rows start on 32-byte sectors and a variable's plane is
+ * read end to end. */
+#define FX_CF_PLANE ((FX_BS + 1) * FX_BS * FX_BS)       /* directions 0 and 1 */
+#define FX_CF_ROW2 (FX_BS + 4)
+#define FX_CF_PLANE2 (FX_BS * FX_BS * FX_CF_ROW2)
+#define FX_CF_COUNT (12 * FX_CF_PLANE + 6 * FX_CF_PLANE2)
+
+FX_HD int fx_cf_plane(int dir) { return dir == 2 ? FX_CF_PLANE2 : FX_CF_PLANE; }
+
+/* variable 0 of a face; variable v sits v planes further */
+FX_HD int fx_cf_idx(int dir, int i, int j, int k)
+{
+    return dir * 6 * FX_CF_PLANE + (dir == 0 ? (i * FX_BS + j) * FX_BS + k
+                                  : dir == 1 ? (i * (FX_BS + 1) + j) * FX_BS + k
+                                             : (i * FX_BS + j) * FX_CF_ROW2 + k);
+}
+
 /* per-block element counts of the stacked device arrays */
 #define FX_W_COUNT(nv) ((nv) * FX_NSTAGES * FX_NCELLS)
 #define FX_BF_COUNT (3 * FX_NSTAGES * FX_NFACES)

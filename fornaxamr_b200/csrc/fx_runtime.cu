@@ -63,8 +63,8 @@ struct fx_ctx {
     FxDev D{};
 
     FxBlockDev *d_blk = nullptr;
-    double *d_W = nullptr, *d_Bf = nullptr, *d_flux = nullptr, *d_vr = nullptr, *d_vn = nullptr;
-    bool compact_faces = false; /* the last face fluxes are the batched form's (vn) */
+    double *d_W = nullptr, *d_Bf = nullptr, *d_flux = nullptr, *d_vr = nullptr, *d_vn = nullptr, *d_cf = nullptr;
+    bool compact_faces = false; /* the last face fluxes are the batched form's (cf, vn) */
     double *d_bv1 = nullptr, *d_bv2 = nullptr, *d_emf = nullptr, *d_eos = nullptr;
     double *d_rhs = nullptr, *d_grav = nullptr;
     double *d_W2 = nullptr, *d_Bf2 = nullptr; /* eSSPRK10_4 stage slot 2 */
@@ -252,6 +252,7 @@ void free_mesh(fx_ctx *c)
     cudaFree(c->d_flux);
     cudaFree(c->d_vr);
     cudaFree(c->d_vn);
+    cudaFree(c->d_cf);
     cudaFree(c->d_bv1);
     cudaFree(c->d_bv2);
     cudaFree(c->d_emf);
@@ -278,7 +279,7 @@ void free_mesh(fx_ctx *c)
     cudaFree(c->d_ecorr);
     for (size_t &cap : c->tab_cap) cap = 0;
     c->d_blk = nullptr;
-    c->d_W = c->d_Bf = c->d_flux = c->d_vr = c->d_vn = c->d_bv1 = c->d_bv2 = nullptr;
+    c->d_W = c->d_Bf = c->d_flux = c->d_vr = c->d_vn = c->d_cf = c->d_bv1 = c->d_bv2 = nullptr;
     c->d_emf = c->d_eos = c->d_rhs = c->d_grav = nullptr;
     c->d_ids = c->d_active = nullptr;
     c->d_cg = c->d_fg = nullptr;
@@ -444,12 +445,14 @@ void ghost_fill(fx_ctx *c, int slot)
 }
 
 /* coarse/fine flux corrections (prj_riemann_flux_send), wave by wave;
- * ncomp: flux components the face kernel stored */
-void flux_correct(fx_ctx *c, int ncomp, cudaStream_t s)
+ * full: the plain form's arrays, every component, else the six the batched
+ * form keeps */
+void flux_correct(fx_ctx *c, int full, cudaStream_t s)
 {
+    const int ncomp = full ? c->nv : 6;
     const std::vector<int> &wb = c->plan.flux_corr_begin;
     for (size_t w = 0; w + 1 < wb.size(); ++w) {
-        fx_launch_flux_correct(c->D, c->d_fcorr + wb[w], wb[w + 1] - wb[w], ncomp, s);
+        fx_launch_flux_correct(c->D, c->d_fcorr + wb[w], wb[w + 1] - wb[w], ncomp, full, s);
     }
 }
 
@@ -520,7 +523,7 @@ void stage_phases(fx_ctx *c, int form, int wslot, int bfslot, int stage, int dst
     shard_exchange(c, FX_XF, wslot);
     if (!c->plan.flux_corr.empty()) {
         lanes_close(c);
-        flux_correct(c, full ? c->nv : 6, c->stream);
+        flux_correct(c, full, c->stream);
         lanes_open(c, form);
     }
     if (c->cfg.mhd) {
@@ -789,6 +792,7 @@ int alloc_block_arrays(fx_ctx *c, int cap, int keep)
     if ((rc = regrow(c, &c->d_flux, (size_t)FX_FLUX_COUNT(c->nv), cap, keep))) return rc;
     if ((rc = regrow(c, &c->d_vr, (size_t)FX_VR_COUNT, cap, keep))) return rc;
     if ((rc = regrow(c, &c->d_vn, (size_t)FX_VN_COUNT, cap, keep))) return rc;
+    if ((rc = regrow(c, &c->d_cf, (size_t)FX_CF_COUNT, cap, keep))) return rc;
     if ((rc = regrow(c, &c->d_eos, (size_t)FX_EOS_COUNT, cap, keep))) return rc;
     if ((rc = regrow(c, &c->d_rhs, (size_t)FX_RHS_COUNT(c->nv), cap, keep))) return rc;
     if (c->cfg.mhd) {
@@ -892,6 +896,7 @@ int install_tables(fx_ctx *c)
     c->D.flux = c->d_flux;
     c->D.vr = c->d_vr;
     c->D.vn = c->d_vn;
+    c->D.cf = c->d_cf;
     c->D.bv1 = c->d_bv1;
     c->D.bv2 = c->d_bv2;
     c->D.emf = c->d_emf;
@@ -1690,7 +1695,7 @@ int fx_download_array(fx_ctx *c, int b, int which, int dir, double *out)
     const double *src = nullptr;
     size_t count = 0;
     const size_t nv = (size_t)c->nv;
-    if (which == FX_ARR_VRIEMANN) expand_faces(c);
+    if (which == FX_ARR_FLUX || which == FX_ARR_VRIEMANN) expand_faces(c);
     switch (which) {
     case FX_ARR_W: {
         int rc = xfer_w(c, b, 1, out, cudaMemcpyDeviceToHost, false);
@@ -1798,7 +1803,7 @@ int fx_riemann_flux_send(fx_ctx *c)
     if (!has_mesh(c)) return c ? set_err(c, FX_ENOMESH, "no mesh") : FX_EINVAL;
     expand_faces(c);
     fx_launch_set_dt(c->D, 0.0, c->stream);
-    flux_correct(c, c->nv, c->stream);
+    flux_correct(c, 1, c->stream);
     return FX_SUCCESS;
 }
 
@@ -2205,6 +2210,7 @@ int fx_amr_adapt(fx_ctx *c, int *changed)
         c->D.flux = c->d_flux;
         c->D.vr = c->d_vr;
     c->D.vn = c->d_vn;
+    c->D.cf = c->d_cf;
         c->D.bv1 = c->d_bv1;
         c->D.bv2 = c->d_bv2;
         c->D.emf = c->d_emf;
