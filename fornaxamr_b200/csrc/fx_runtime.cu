@@ -14,6 +14,9 @@
  */
 #include <cuda_runtime.h>
 
+#include <atomic>
+#include <thread>
+#include <exception>
 #include <algorithm>
 #include <chrono>
 #include <cstdarg>
@@ -45,6 +48,8 @@ enum { FX_XG = 0, FX_XF = 1, FX_XE = 2 }; /* ghost fill (cells + faces), flux, E
  * device for a few microseconds, so one after the other they cost their
  * latency each */
 constexpr int FX_LANES = 8;
+
+constexpr size_t FX_STAGE_BYTES = 1 << 20;
 
 struct fx_ctx {
     int device = 0;
@@ -86,6 +91,10 @@ struct fx_ctx {
      * block always on the same one) between lanes_open and lanes_close */
     cudaStream_t lane[FX_LANES] = {};
     cudaEvent_t ev_lane[FX_LANES] = {};
+    /* page-locked staging of large copies from and to pageable memory, two
+     * buffers per lane (allocated by the first one) */
+    char *h_stage = nullptr;
+    cudaEvent_t ev_stage[FX_LANES][2] = {};
     bool lanes = false;
     cudaStream_t side = nullptr;      /* a wave's face-prolongation groups, beside its copies */
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
@@ -1032,6 +1041,90 @@ void child_groups(const FxAmrRefine &r, bool use_bj, std::vector<FxPop> &out)
     }
 }
 
+/* Copies `bytes` between host and device in the order of the context's
+ * stream; the host side is done when the call returns.  A large copy from
+ * or to pageable memory goes through page-locked buffers, a share of the
+ * array per host thread and lane (the driver's own staging copies with one
+ * thread, 5 to 8 GB/s, and faults a fresh array's pages in one by one).
+ * The 64-block adjoint's 74 MB in and 100 MB out: 33 -> 18 ms
+ * for the whole gradient. */
+int copy_pageable(fx_ctx *c, void *host, void *dev, size_t bytes, bool to_host)
+{
+    const cudaMemcpyKind kind = to_host ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice;
+    cudaPointerAttributes at{};
+    const bool pageable = cudaPointerGetAttributes(&at, host) != cudaSuccess || at.type == cudaMemoryTypeUnregistered;
+    cudaGetLastError();
+    const int lanes = (int)std::min<size_t>(FX_LANES, std::max(1u, std::thread::hardware_concurrency()));
+    bool staged = pageable && bytes >= 8 * FX_STAGE_BYTES && lanes > 1 && make_lanes(c);
+    for (auto &pair : c->ev_stage) {
+        for (cudaEvent_t &e : pair) staged = staged && make_event(&e);
+    }
+    if (staged && !c->h_stage &&
+        cudaMallocHost((void **)&c->h_stage, 2 * FX_LANES * FX_STAGE_BYTES) != cudaSuccess) {
+        cudaGetLastError();
+        c->h_stage = nullptr;
+        staged = false;
+    }
+    if (!staged) {
+        FX_CUDA(c, cudaMemcpyAsync(to_host ? host : dev, to_host ? dev : host, bytes, kind, c->stream));
+        FX_CUDA(c, cudaStreamSynchronize(c->stream));
+        return FX_SUCCESS;
+    }
+    FX_CUDA(c, cudaEventRecord(c->ev_fork, c->stream));
+    std::atomic<int> failed{0};
+    auto share = [&](int l) {
+        cudaSetDevice(c->device);
+        const size_t lo = bytes / lanes * l;
+        const size_t hi = l + 1 == lanes ? bytes : bytes / lanes * (l + 1);
+        const size_t n = (hi - lo + FX_STAGE_BYTES - 1) / FX_STAGE_BYTES;
+        cudaStream_t s = c->lane[l];
+        cudaError_t e = cudaStreamWaitEvent(s, c->ev_fork, 0);
+        auto part = [&](size_t q, size_t &off) {
+            off = lo + q * FX_STAGE_BYTES;
+            return std::min(FX_STAGE_BYTES, hi - off);
+        };
+        auto buf = [&](size_t q) { return c->h_stage + (2 * l + (q & 1)) * FX_STAGE_BYTES; };
+        auto put = [&](size_t q) { /* one DMA of part q, its event behind it */
+            size_t off;
+            const size_t m = part(q, off);
+            if (e == cudaSuccess) {
+                e = to_host ? cudaMemcpyAsync(buf(q), (char *)dev + off, m, kind, s)
+                            : cudaMemcpyAsync((char *)dev + off, buf(q), m, kind, s);
+            }
+            if (e == cudaSuccess) e = cudaEventRecord(c->ev_stage[l][q & 1], s);
+        };
+        for (size_t q = 0; to_host && q < std::min<size_t>(2, n); ++q) put(q);
+        for (size_t q = 0; q < n && e == cudaSuccess; ++q) {
+            size_t off;
+            const size_t m = part(q, off);
+            /* to the host: part q has arrived; from it: the buffer's last DMA has left */
+            e = cudaEventSynchronize(c->ev_stage[l][q & 1]);
+            if (e != cudaSuccess) break;
+            if (to_host) {
+                std::memcpy((char *)host + off, buf(q), m);
+                if (q + 2 < n) put(q + 2);
+            } else {
+                std::memcpy(buf(q), (const char *)host + off, m);
+                put(q);
+            }
+        }
+        if (e == cudaSuccess) e = cudaEventRecord(c->ev_lane[l], s);
+        if (e != cudaSuccess) failed = (int)e;
+    };
+    std::vector<std::thread> pool;
+    int started = 1;
+    try {
+        for (; started < lanes; ++started) pool.emplace_back(share, started);
+    } catch (const std::exception &) { /* no more threads: the shares left are done here */
+    }
+    share(0);
+    for (int l = started; l < lanes; ++l) share(l);
+    for (std::thread &t : pool) t.join();
+    if (failed) return set_err(c, FX_ECUDA, "staged copy: %s", cudaGetErrorString((cudaError_t)failed.load()));
+    for (int l = 0; l < lanes; ++l) FX_CUDA(c, cudaStreamWaitEvent(c->stream, c->ev_lane[l], 0));
+    return FX_SUCCESS;
+}
+
 void drop_adjoint(fx_ctx *c)
 {
     cudaFree(c->d_ckW);
@@ -1154,6 +1247,12 @@ void fx_destroy(fx_ctx *c)
     cudaFreeHost(c->h_err);
     cudaFreeHost(c->h_red);
     cudaFreeHost(c->h_ctl);
+    cudaFreeHost(c->h_stage);
+    for (auto &pair : c->ev_stage) {
+        for (cudaEvent_t e : pair) {
+            if (e) cudaEventDestroy(e);
+        }
+    }
     for (cudaStream_t l : c->lane) {
         if (l) cudaStreamDestroy(l);
     }
@@ -2692,9 +2791,9 @@ int fx_adjoint_backward(fx_ctx *c, const double *W_bar, const double *Bf_bar, do
         if ((rc = dev_alloc(c, &c->d_Eb, nb * FX_EMF_COUNT))) return rc;
     }
     cudaStream_t s = c->stream;
-    FX_CUDA(c, cudaMemcpyAsync(c->d_Wb, W_bar, wn * sizeof(double), cudaMemcpyHostToDevice, s));
+    if ((rc = copy_pageable(c, const_cast<double *>(W_bar), c->d_Wb, wn * sizeof(double), false))) return rc;
     if (Bf_bar) {
-        FX_CUDA(c, cudaMemcpyAsync(c->d_Bfb, Bf_bar, bn * sizeof(double), cudaMemcpyHostToDevice, s));
+        if ((rc = copy_pageable(c, const_cast<double *>(Bf_bar), c->d_Bfb, bn * sizeof(double), false))) return rc;
     } else {
         FX_CUDA(c, cudaMemsetAsync(c->d_Bfb, 0, bn * sizeof(double), s));
     }
@@ -2708,8 +2807,8 @@ int fx_adjoint_backward(fx_ctx *c, const double *W_bar, const double *Bf_bar, do
     if (initial_fill) {
         adj_ghost(c, A, 0);
     }
-    FX_CUDA(c, cudaMemcpyAsync(W_bar_out, c->d_Wb, wn * sizeof(double), cudaMemcpyDeviceToHost, s));
-    FX_CUDA(c, cudaMemcpyAsync(Bf_bar_out, c->d_Bfb, bn * sizeof(double), cudaMemcpyDeviceToHost, s));
+    if ((rc = copy_pageable(c, W_bar_out, c->d_Wb, wn * sizeof(double), true))) return rc;
+    if ((rc = copy_pageable(c, Bf_bar_out, c->d_Bfb, bn * sizeof(double), true))) return rc;
     return sync_and_check(c);
 }
 
