@@ -90,6 +90,27 @@ __device__ __forceinline__ void fx_recon_pair(const double (&q)[FxStencil<RECON>
     }
 }
 
+/* the value on one side of a face: the left state's (left) or the right's,
+ * read from the stencil's cells at q (first cell) with stride s */
+template <int RECON>
+__device__ __forceinline__ double fx_recon_one(const double *q, int s, bool left)
+{
+    if constexpr (RECON == FX_RECON_WENO7) {
+        const double *p = left ? q : q + 7 * s;
+        const int d = left ? s : -s;
+        return fx_weno7_plus(p[0], p[d], p[2 * d], p[3 * d], p[4 * d], p[5 * d], p[6 * d]);
+    } else {
+        const double *p = left ? q : q + s;
+        const double a = __ldg(p), b = __ldg(p + s), c = __ldg(p + 2 * s);
+        if constexpr (RECON == FX_RECON_WENO3) {
+            return fx_weno3_face(a, b, c, left ? 0.5 : -0.5);
+        } else {
+            const double h = fx_mc_half(b - a, c - b);
+            return left ? b + h : b - h;
+        }
+    }
+}
+
 /* MC face values of a 4-cell stencil with the limiter's selections through
  * a branch policy: bits 4 q + 0 and 4 q + 2 of the face's word */
 template <class BR>
@@ -209,6 +230,11 @@ __global__ void __launch_bounds__(TPB, MINB) k_flux(FxDev D, const int *__restri
 
     double WL[9];
     double WR[9];
+    /* the MHD solver takes the internal energy and composition of one side
+     * only and asks for them when it knows which: worth its late loads for
+     * the WENO values (WENO-Z3, 216 blocks: 490 -> 470 us), not for two MC
+     * slopes (512 blocks: 503 -> 551 us) */
+    constexpr bool kLazy = MHD && BRM == 0 && RECON != FX_RECON_MC;
     /* density and internal energy at the stencil cells also give the
      * reconstructed pressure (eosvar p = (g-1) rho e of each cell).  The
      * MC and WENO-Z3 stencils come through the read-only data path
@@ -231,14 +257,16 @@ __global__ void __launch_bounds__(TPB, MINB) k_flux(FxDev D, const int *__restri
     }
     if constexpr (BRM == 0) {
         fx_recon_pair<RECON>(rhoS, WL[FX_RHO], WR[FX_RHO]);
-        fx_recon_pair<RECON>(eintS, WL[FX_EINT], WR[FX_EINT]);
+        if constexpr (!kLazy) {
+            fx_recon_pair<RECON>(eintS, WL[FX_EINT], WR[FX_EINT]);
+        }
     } else {
         fx_recon_pair_br(rhoS, WL[FX_RHO], WR[FX_RHO], br, 4 * FX_RHO);
         fx_recon_pair_br(eintS, WL[FX_EINT], WR[FX_EINT], br, 4 * FX_EINT);
     }
 #pragma unroll
     for (int lv = 1; lv < nv; ++lv) {
-        if (lv == FX_EINT || (MHD && lv == FX_B1)) {
+        if (lv == FX_EINT || (MHD && lv == FX_B1) || (kLazy && lv == FX_YE)) {
             continue;
         }
         const double *q = Wb + (size_t)fx_gmap(dir, lv) * kPlane + c0;
@@ -282,7 +310,15 @@ __global__ void __launch_bounds__(TPB, MINB) k_flux(FxDev D, const int *__restri
         FxFaceOut o;
         if constexpr (BRM == 0) {
             FxBrFree bf;
-            fx_riemann_hlld_folded_br(WL, WR, pL, pR, gL, gR, bn, o, &suspect, b, cR, bf);
+            if constexpr (kLazy) {
+                fx_riemann_hlld_folded_br(WL, WR, pL, pR, gL, gR, bn, o, &suspect, b, cR, bf,
+                    [q0 = Wb + c0, s](bool left, double &eint, double &ye) {
+                        eint = fx_recon_one<RECON>(q0 + (size_t)FX_EINT * kPlane, s, left);
+                        ye = fx_recon_one<RECON>(q0 + (size_t)FX_YE * kPlane, s, left);
+                    });
+            } else {
+                fx_riemann_hlld_folded_br(WL, WR, pL, pR, gL, gR, bn, o, &suspect, b, cR, bf);
+            }
         } else {
             fx_riemann_hlld_folded_br(WL, WR, pL, pR, gL, gR, bn, o, D.err, b, cR, br);
             if constexpr (BRM == 1) {

@@ -580,7 +580,7 @@ FX_HD void fx_cons2prim(const double *u, double *w)
 #define FX_HLLD_SMALL 1.0e-8
 
 struct FxHlldState {
-    double rho, vx, vy, vz, bx, by, bz, p, gamma, ye, e, pt;
+    double rho, vx, vy, vz, bx, by, bz, p, gamma, ye, e, pt, mag;
 };
 
 struct FxHlldStar {
@@ -639,7 +639,9 @@ FX_HD double fx_hlld_state_f(const FxHlldState &s, int v)
 }
 
 /* prj_hlld_state_from_prim, src/prj_riemann.c:142-178; w is the local
- * (direction-rotated) primitive vector, the normal field is bn. */
+ * (direction-rotated) primitive vector, the normal field is bn.  The total
+ * energy and the composition come apart (fx_hlld_energy): the solver needs
+ * them on one side of the face only. */
 template <class E>
 FX_HD void fx_hlld_state_e(const double *w, double p, double gamma, double bn,
     FxHlldState &s, E *err, int blk, int idx)
@@ -653,18 +655,23 @@ FX_HD void fx_hlld_state_e(const double *w, double p, double gamma, double bn,
     s.bz = w[FX_B3];
     s.p = p;
     s.gamma = gamma;
-    s.ye = w[FX_YE];
     fx_check_state(err, s.rho, s.p, s.gamma, blk, idx);
+    s.mag = 0.5 * (s.bx * s.bx + s.by * s.by + s.bz * s.bz);
+    s.pt = s.p + s.mag;
+}
+
+FX_HD void fx_hlld_energy(FxHlldState &s, double eint, double ye)
+{
     const double kinetic = 0.5 * s.rho * (s.vx * s.vx + s.vy * s.vy + s.vz * s.vz);
-    const double magnetic = 0.5 * (s.bx * s.bx + s.by * s.by + s.bz * s.bz);
-    s.e = s.rho * w[FX_EINT] + kinetic + magnetic;
-    s.pt = s.p + magnetic;
+    s.e = s.rho * eint + kinetic + s.mag;
+    s.ye = ye;
 }
 
 FX_HD void fx_hlld_state(const double *w, double p, double gamma, double bn,
     FxHlldState &s, FxErr *err, int blk, int idx)
 {
     fx_hlld_state_e(w, p, gamma, bn, s, err, blk, idx);
+    fx_hlld_energy(s, w[FX_EINT], w[FX_YE]);
 }
 
 /* prj_hlld_fast_speed, src/prj_riemann.c:117-140; the clamp of a negative
@@ -768,11 +775,14 @@ FX_HD void fx_face_outputs(double vx, double vy, double vz,
  * (S - vx, rho (S - vx), the total pressure) is selected, not computed again.
  * The single-star flux comes first and the double star adds its jump to it;
  * rho, vx and ye do not jump across the Alfven wave, so three of those
- * terms are S_Ns times +0.0. */
-template <class BR, class E = FxErr>
+ * terms are S_Ns times +0.0.
+ * thermal(left, eint, ye) gives the internal energy and composition of the
+ * left or right state: only the near side's enter (but for the HLL
+ * fallback), so a caller can leave the other side's reconstruction out. */
+template <class BR, class E, class Thermal>
 FX_HD void fx_riemann_hlld_folded_br(const double *WL, const double *WR,
     double pL, double pR, double gL, double gR, double bn, FxFaceOut &o,
-    E *err, int blk, int idx, BR &br)
+    E *err, int blk, int idx, BR &br, const Thermal &thermal)
 {
     FxHlldState L, R;
     fx_hlld_state_e(WL, pL, gL, bn, L, err, blk, idx);
@@ -785,8 +795,12 @@ FX_HD void fx_riemann_hlld_folded_br(const double *WL, const double *WR,
     const double SR = br.bit(FX_BR_SR, bL > bR) ? bL : bR;   /* fx_max */
     fx_check_order(err, SL, SR, blk, idx);
     const bool super_l = br.bit(FX_BR_SUPER_L, 0.0 <= SL);
-    if (super_l || br.bit(FX_BR_SUPER_R, SR <= 0.0)) {
-        const FxHlldState &X = super_l ? L : R;
+    const bool super = super_l || br.bit(FX_BR_SUPER_R, SR <= 0.0);
+    if (super) {
+        FxHlldState X = super_l ? L : R;
+        double eint, ye;
+        thermal(super_l, eint, ye);
+        fx_hlld_energy(X, eint, ye);
 #pragma unroll
         for (int v = 0; v < 9; ++v) o.F[v] = fx_hlld_state_f(X, v);
         fx_face_outputs(X.vx, X.vy, X.vz, X.bx, X.by, X.bz, o);
@@ -804,6 +818,11 @@ FX_HD void fx_riemann_hlld_folded_br(const double *WL, const double *WR,
     if (br.bit(FX_BR_HLL, !fx_pos_normal(pt_star) && (pt_star <= 0.0 || !isfinite(pt_star)))) {
         const double inv = fx_div(1.0, SR - SL);
         double Uh[9];
+        double eint, ye;
+        thermal(true, eint, ye);
+        fx_hlld_energy(L, eint, ye);
+        thermal(false, eint, ye);
+        fx_hlld_energy(R, eint, ye);
 #pragma unroll
         for (int v = 0; v < 9; ++v) {
             const double lf = fx_hlld_state_f(L, v);
@@ -819,7 +838,12 @@ FX_HD void fx_riemann_hlld_folded_br(const double *WL, const double *WR,
     }
     const bool bn_small = br.bit(FX_BR_BNSMALL, 0.5 * bn * bn < FX_HLLD_SMALL * pt_star);
     const bool left = br.bit(FX_BR_LEFT, 0.0 <= SM);
-    const FxHlldState N = left ? L : R;
+    FxHlldState N = left ? L : R;
+    {
+        double eint, ye;
+        thermal(left, eint, ye);
+        fx_hlld_energy(N, eint, ye);
+    }
     const double SN = left ? SL : SR;
     FxHlldStar Ns;
     fx_hlld_outer_star_br(N, left ? alL : alR, left ? raL : raR, SN, SM, pt_star, Ns, err, blk, idx, br,
@@ -868,6 +892,19 @@ FX_HD void fx_riemann_hlld_folded_br(const double *WL, const double *WR,
         o.F[v] = o.F[v] + jump;
     }
     fx_face_outputs(ss.vx, ss.vy, ss.vz, ss.bx, ss.by, ss.bz, o);
+}
+
+/* with the internal energy and composition of WL and WR */
+template <class BR, class E = FxErr>
+FX_HD void fx_riemann_hlld_folded_br(const double *WL, const double *WR,
+    double pL, double pR, double gL, double gR, double bn, FxFaceOut &o,
+    E *err, int blk, int idx, BR &br)
+{
+    fx_riemann_hlld_folded_br(WL, WR, pL, pR, gL, gR, bn, o, err, blk, idx, br,
+        [WL, WR](bool left, double &eint, double &ye) {
+            eint = left ? WL[FX_EINT] : WR[FX_EINT];
+            ye = left ? WL[FX_YE] : WR[FX_YE];
+        });
 }
 
 FX_HD void fx_riemann_hlld_folded(const double *WL, const double *WR,

@@ -145,3 +145,57 @@ def test_uniform_steps_of_both_forms_are_the_same(root, recon, integ, mhd):
     if not mhd:
         W, Bf = np.ascontiguousarray(W[:, :6]), None
     _run_both(blocks, COORD, W, Bf, recon=recon, integrator=integ)
+
+
+@pytest.mark.parametrize("mhd", [True, False])
+def test_sharded_steps_match_one_device(mhd):
+    """Three ranks emulated in one process (flux and EMF records across
+    ranks read the compact face arrays) against one context."""
+    import threading
+    blocks = mesh.static_amr_mesh((3,) * 3, AMR_COORD, 2, mesh.ball_refiner((0.1, 0.05, 0.0), (0.25, 0.1)))
+    desc = mesh.to_desc(blocks)
+    recs = fx.plan_export(fx.make_config(mhd, 5.0 / 3.0, AMR_COORD), desc, 3) if mhd else None
+    W, Bf = problems.amr_blast(blocks, recs, mhd=mhd)
+
+    def field(b):
+        return None if Bf is None else [Bf[b, d].ravel() for d in range(3)]
+
+    one = fx.Context(mhd, 5.0 / 3.0, AMR_COORD)
+    one.set_mesh(desc)
+    for b in range(len(blocks)):
+        one.upload_block(b, W[b].ravel(), field(b))
+    one.boundary_fill(1, 0)
+    clock = one.run(fx.FORM_BATCHED, 2, 0.4, 1.2, 1.0e30, (0.0, 0.0, 0))
+    owner = fx.morton_owner(desc, 3)
+    group = fx.ShardGroup(3)
+    ctxs, got, err = [], [None] * 3, []
+    for r in range(3):
+        c = fx.Context(mhd, 5.0 / 3.0, AMR_COORD)
+        c.shard_set_mesh(desc, owner, 3, r)
+        c.attach_group(group)
+        for b in np.nonzero(owner == r)[0]:
+            c.upload_block(int(b), W[b].ravel(), field(b))
+        ctxs.append(c)
+
+    def work(r):
+        try:
+            ctxs[r].boundary_fill(1, 0)
+            got[r] = ctxs[r].run(fx.FORM_BATCHED, 2, 0.4, 1.2, 1.0e30, (0.0, 0.0, 0))
+        except Exception as e:  # re-raised below
+            err.append(e)
+    threads = [threading.Thread(target=work, args=(r,)) for r in range(3)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join(timeout=300)
+    assert not err, err
+    assert got == [clock] * 3
+    for r in range(3):
+        for b in np.nonzero(owner == r)[0]:
+            a, c = one.download_block(int(b)), ctxs[r].download_block(int(b))
+            assert np.array_equal(a[0], c[0])
+            for d in range(3 if mhd else 0):
+                assert np.array_equal(a[2][d], c[2][d])
+    for c in ctxs + [one]:
+        c.close()
+    group.close()
