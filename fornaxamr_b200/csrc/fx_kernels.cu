@@ -1298,15 +1298,25 @@ __device__ __forceinline__ int fx_face_stride(int d, int a)
 /* One Toth-Roe group: prj_mhd_prolong_bf_from_buffer (src/prj_mhd.c:374-512)
  * with prj_mhd_compute_buffer_inner_fluxes (src/prj_mhd.c:309-372), in the
  * reference's operation order.  Outer faces are area-weighted fluxes; kept
- * faces contribute their current fine value. */
-__device__ __forceinline__ void fx_ghost_prolong_group(const FxDev &D, const FxPop &op, int slot)
+ * faces contribute their current fine value.
+ * Four neighbouring lanes share a group, lane 2 a + b taking the sub-faces
+ * (a, b): six outer and three inner faces each, where one thread had 24 and
+ * 12 one after the other, and of the six sums over the outer fluxes (eight
+ * divisions in three of them) the lanes 0 to 2 one pair each.  The fluxes and
+ * sums go from lane to lane by shuffles, so every lane of the warp comes here;
+ * `live` lanes store.  Latency bound: a fill's later waves have few groups.
+ * 470-block blast: a fill of seven waves 288 -> 234 us. */
+__device__ __forceinline__ void fx_ghost_prolong_group(const FxDev &D, const FxPop &op, int slot, bool live)
 {
+    const int lane = threadIdx.x & 3;
+    const int a = lane >> 1, b = lane & 1;
+    const double sa = a ? 1.0 : -1.0, sb = b ? 1.0 : -1.0;
     const int f0[3] = {(op.pos & 31) - FX_NG, ((op.pos >> 5) & 31) - FX_NG, ((op.pos >> 10) & 31) - FX_NG};
     const int c0[3] = {((op.pos >> 15) & 31) - FX_NG, ((op.pos >> 20) & 31) - FX_NG, ((op.pos >> 25) & 31) - FX_NG};
     const FxBlockDev &fb = D.blk[op.fine];
     const double area[3] = {fb.dx[1] * fb.dx[2], fb.dx[0] * fb.dx[2], fb.dx[0] * fb.dx[1]};
-    /* outer fluxes o[d][side][a][b] */
-    double o[3][2][2][2];
+    /* this lane's outer fluxes [d][side] */
+    double of[3][2];
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
         const int t0 = d == 0 ? 1 : 0;
@@ -1320,42 +1330,42 @@ __device__ __forceinline__ void fx_ghost_prolong_group(const FxDev &D, const FxP
             int y[3] = {c0[0], c0[1], c0[2]};
             y[d] += side;
             const int cf = fx_face_idx(d, y[0], y[1], y[2]);
-#pragma unroll
-            for (int a = 0; a < 2; ++a) {
-#pragma unroll
-                for (int b = 0; b < 2; ++b) {
-                    const int q = 8 * d + 4 * side + 2 * a + b;
-                    int x[3] = {f0[0], f0[1], f0[2]};
-                    x[d] += 2 * side;
-                    x[t0] += a;
-                    x[t1] += b;
-                    const int xf = fx_face_idx(d, x[0], x[1], x[2]);
-                    double flux;
-                    if ((op.keep >> q) & 1) {
-                        flux = Bfine[xf] * area[d];
-                    } else {
-                        const double ta = a ? 0.25 : -0.25;
-                        const double tb = b ? 0.25 : -0.25;
-                        const double *qc = Bc + cf;
-                        const double value = (op.flags & 1)
-                            ? fx_bj_face([qc, s0, s1](int d0, int d1) { return qc[d0 * s0 + d1 * s1]; }, ta, tb)
-                            : fx_prolong_face(Bc, cf, s0, s1, ta, tb);
-                        flux = value * area[d];
-                        if ((op.owrite >> q) & 1) {
-                            Bfine[xf] = flux / area[d];
-                        }
-                    }
-                    o[d][side][a][b] = flux;
+            const int q = 8 * d + 4 * side + lane;
+            int x[3] = {f0[0], f0[1], f0[2]};
+            x[d] += 2 * side;
+            x[t0] += a;
+            x[t1] += b;
+            const int xf = fx_face_idx(d, x[0], x[1], x[2]);
+            if ((op.keep >> q) & 1) {
+                of[d][side] = Bfine[xf] * area[d];
+            } else {
+                const double ta = a ? 0.25 : -0.25;
+                const double tb = b ? 0.25 : -0.25;
+                const double *qc = Bc + cf;
+                const double value = (op.flags & 1)
+                    ? fx_bj_face([qc, s0, s1](int d0, int d1) { return qc[d0 * s0 + d1 * s1]; }, ta, tb)
+                    : fx_prolong_face(Bc, cf, s0, s1, ta, tb);
+                const double flux = value * area[d];
+                of[d][side] = flux;
+                if (live && ((op.owrite >> q) & 1)) {
+                    Bfine[xf] = flux / area[d];
                 }
             }
         }
     }
-    /* u[i][j][k] of the reference: u[0|2][j][k] = o[0][0|1][j][k],
-     * v[i][0|2][k] = o[1][0|1][i][k], w[i][j][0|2] = o[2][0|1][i][j] */
+    /* u[i][j][k] of the reference: u[0|2][j][k] is the outer flux of direction
+     * 0 on side 0|1 at sub-face (j, k), v[i][0|2][k] of direction 1 at (i, k),
+     * w[i][j][0|2] of direction 2 at (i, j).  Lane n sums, over i, j, k in
+     * this order, for n = 0, 1, 2:
+     *   Uxx += si sj v + si sk w, Vyy += sj sk w + sj si u, Wzz += sk si u + sk sj v
+     *   Uxyz += si sj sk u / (dx2s + dx3s), and cyclically
+     * (products of signs are exact) */
     const double dx1s = fb.dx[0] * fb.dx[0];
     const double dx2s = fb.dx[1] * fb.dx[1];
     const double dx3s = fb.dx[2] * fb.dx[2];
-    double Uxx = 0.0, Vyy = 0.0, Wzz = 0.0, Uxyz = 0.0, Vxyz = 0.0, Wxyz = 0.0;
+    const int n = lane < 3 ? lane : 0;
+    const double den = n == 0 ? dx2s + dx3s : n == 1 ? dx1s + dx3s : dx1s + dx2s;
+    double S = 0.0, T = 0.0;
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
         const double si = i ? 1.0 : -1.0;
@@ -1365,57 +1375,52 @@ __device__ __forceinline__ void fx_ghost_prolong_group(const FxDev &D, const FxP
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
                 const double sk = k ? 1.0 : -1.0;
-                const double u = o[0][i][j][k];
-                const double v = o[1][j][i][k];
-                const double w = o[2][k][i][j];
-                Uxx += si * sj * v + si * sk * w;
-                Vyy += sj * sk * w + sj * si * u;
-                Wzz += sk * si * u + sk * sj * v;
-                Uxyz += si * sj * sk * u / (dx2s + dx3s);
-                Vxyz += si * sj * sk * v / (dx1s + dx3s);
-                Wxyz += si * sj * sk * w / (dx1s + dx2s);
+                const int quad = threadIdx.x & 28;
+                const double u = __shfl_sync(0xffffffffu, of[0][i], quad | (2 * j + k));
+                const double v = __shfl_sync(0xffffffffu, of[1][j], quad | (2 * i + k));
+                const double w = __shfl_sync(0xffffffffu, of[2][k], quad | (2 * i + j));
+                const double X = n == 0 ? si * sj * v : n == 1 ? sj * sk * w : sk * si * u;
+                const double Y = n == 0 ? si * sk * w : n == 1 ? sj * si * u : sk * sj * v;
+                S += X + Y;
+                T += si * sj * sk * (n == 0 ? u : n == 1 ? v : w) / den;
             }
         }
     }
-    Uxx *= 0.125;
-    Vyy *= 0.125;
-    Wzz *= 0.125;
-    Uxyz *= 0.125;
-    Vxyz *= 0.125;
-    Wxyz *= 0.125;
+    S *= 0.125;
+    T *= 0.125;
+    const int quad = threadIdx.x & 28;
+    const double Uxx = __shfl_sync(0xffffffffu, S, quad);
+    const double Vyy = __shfl_sync(0xffffffffu, S, quad | 1);
+    const double Wzz = __shfl_sync(0xffffffffu, S, quad | 2);
+    const double Uxyz = __shfl_sync(0xffffffffu, T, quad);
+    const double Vxyz = __shfl_sync(0xffffffffu, T, quad | 1);
+    const double Wxyz = __shfl_sync(0xffffffffu, T, quad | 2);
+    if (!live) {
+        return;
+    }
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
         const int t0 = d == 0 ? 1 : 0;
         const int t1 = d == 2 ? 1 : 2;
-        double *Bfine = D.Bf + (size_t)op.fine * FX_BF_COUNT + ((size_t)d * FX_NSTAGES + slot) * FX_NFACES;
-#pragma unroll
-        for (int a = 0; a < 2; ++a) {
-#pragma unroll
-            for (int b = 0; b < 2; ++b) {
-                const int q = 4 * d + 2 * a + b;
-                if (!((op.iwrite >> q) & 1)) continue;
-                const double sa = a ? 1.0 : -1.0;
-                const double sb = b ? 1.0 : -1.0;
-                double flux;
-                if (d == 0) {        /* u[1][j][k], (a, b) = (j, k) */
-                    flux = 0.5 * (o[0][1][a][b] + o[0][0][a][b]) + Uxx + sb * dx3s * Vxyz + sa * dx2s * Wxyz;
-                } else if (d == 1) { /* v[i][1][k], (a, b) = (i, k) */
-                    flux = 0.5 * (o[1][1][a][b] + o[1][0][a][b]) + Vyy + sa * dx1s * Wxyz + sb * dx3s * Uxyz;
-                } else {             /* w[i][j][1], (a, b) = (i, j) */
-                    flux = 0.5 * (o[2][1][a][b] + o[2][0][a][b]) + Wzz + sb * dx2s * Uxyz + sa * dx1s * Vxyz;
-                }
-                const double value = flux / area[d];
-                int x[3] = {f0[0], f0[1], f0[2]};
-                x[d] += 1;
-                x[t0] += a;
-                x[t1] += b;
-                const int xf = fx_face_idx(d, x[0], x[1], x[2]);
-                if (!isfinite(value)) {
-                    fx_fail(D.err, FX_ERR_BF_NONFINITE, op.fine, xf);
-                }
-                Bfine[xf] = value;
-            }
+        if (!((op.iwrite >> (4 * d + lane)) & 1)) continue;
+        double flux;
+        if (d == 0) {        /* u[1][j][k], (a, b) = (j, k) */
+            flux = 0.5 * (of[0][1] + of[0][0]) + Uxx + sb * dx3s * Vxyz + sa * dx2s * Wxyz;
+        } else if (d == 1) { /* v[i][1][k], (a, b) = (i, k) */
+            flux = 0.5 * (of[1][1] + of[1][0]) + Vyy + sa * dx1s * Wxyz + sb * dx3s * Uxyz;
+        } else {             /* w[i][j][1], (a, b) = (i, j) */
+            flux = 0.5 * (of[2][1] + of[2][0]) + Wzz + sb * dx2s * Uxyz + sa * dx1s * Vxyz;
         }
+        const double value = flux / area[d];
+        int x[3] = {f0[0], f0[1], f0[2]};
+        x[d] += 1;
+        x[t0] += a;
+        x[t1] += b;
+        const int xf = fx_face_idx(d, x[0], x[1], x[2]);
+        if (!isfinite(value)) {
+            fx_fail(D.err, FX_ERR_BF_NONFINITE, op.fine, xf);
+        }
+        D.Bf[(size_t)op.fine * FX_BF_COUNT + ((size_t)d * FX_NSTAGES + slot) * FX_NFACES + xf] = value;
     }
 }
 
@@ -1528,11 +1533,11 @@ __device__ __forceinline__ void fx_ghost_b_pair(const FxDev &D, const FxBop op, 
  * occupancy, of the copy-dominated wave kernel) */
 __global__ void __launch_bounds__(128) k_ghost_groups(FxDev D, const FxPop *__restrict__ pops, int np, int slot)
 {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= np || D.ctl->skip) {
+    if (D.ctl->skip) {
         return;
     }
-    fx_ghost_prolong_group(D, pops[t], slot);
+    const int g = (blockIdx.x * blockDim.x + threadIdx.x) >> 2;
+    fx_ghost_prolong_group(D, pops[min(g, np - 1)], slot, g < np);
 }
 
 /* face pairs per thread of the wave kernel */
@@ -2156,7 +2161,7 @@ void fx_launch_xunpack(const FxDev &D, const FxXent *ents, int n, const double *
 void fx_launch_prolong_groups(const FxDev &D, const FxPop *pops, int np, int slot, cudaStream_t s)
 {
     if (np > 0) {
-        k_ghost_groups<<<fx_blocks(np, 128), 128, 0, s>>>(D, pops, np, slot);
+        k_ghost_groups<<<fx_blocks(4 * np, 128), 128, 0, s>>>(D, pops, np, slot);
     }
 }
 
