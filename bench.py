@@ -416,7 +416,7 @@ def run_amr(args, dev, kind):
         "plain": {"ms_per_step": ms_plain, "value": zones / (ms_plain * 1e-3)},
         "batched_over_plain": ms_plain / ms_batched,
         "phases_ms": phases,
-        "ghost_waves": ctx.info(4), "launches_per_batched_step": ctx.info(0) + 4,
+        "ghost_waves": ctx.info(4), "launches_per_batched_step": ctx.info(0) + 1,
         "setup_s": {"mesh": round(t_mesh, 1), "initial_state": round(t_init, 1), "ghost_compiler": round(t_plan, 1)},
         "steps": args.amr_steps,
     }
@@ -814,7 +814,7 @@ def run_fx(args, rank, world, local_rank):
     kernel_bytes = nb * 3 * 20 * 18 * 18 * 8 * 8 + faces * 8 + faces * 9 * 8
     prof = flux_profile_figures()
     traffic = prof["dram_bytes_per_launch"]
-    launches_per_step = ctx.info(0) + 4
+    launches_per_step = ctx.info(0) + 1
     line = {
         "metric": METRIC,
         "value": value,

@@ -211,8 +211,9 @@ void fx_launch_expand_faces(const FxDev &D, const int *blist, int nlist, cudaStr
  * place on slot 0 (prj_timeint_mhd_update_bf stage 0 and the stage-1 cell
  * update writing slot 0) */
 void fx_launch_bf_update(const FxDev &D, const int *blist, int nlist, int stage, cudaStream_t s);
+/* next_dt (stage 2, batched form): the timestep minimum of the new state too */
 void fx_launch_cell_update(const FxDev &D, const int *blist, int nlist, int stage,
-    int gravity, int full, cudaStream_t s);
+    int gravity, int full, int next_dt, cudaStream_t s);
 /* dt_stage = dt / divisor in the control block */
 void fx_launch_stage_dt(const FxDev &D, double divisor, cudaStream_t s);
 /* prj_timeint_eSSPRK_save_state (src/prj_timeint.c:2311-2352): W of the

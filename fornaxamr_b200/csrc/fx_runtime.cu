@@ -109,6 +109,7 @@ struct fx_ctx {
     cudaGraphExec_t g_step = nullptr; /* batched RK2 step, dt from the control block */
     cudaGraphExec_t g_run = nullptr;  /* batched driver step (calc_dt + step + dt update) */
     int last_slot = 0;                /* W slot written by the last stage */
+    bool next_dt = false;             /* stage 2 being issued takes the next step's timestep too */
 
     /* discrete adjoint: states after every stage of the last
      * fx_adjoint_forward and the adjoint arrays */
@@ -546,7 +547,7 @@ void stage_phases(fx_ctx *c, int form, int wslot, int bfslot, int stage, int dst
         per_block(c, form, [&](const int *l, int n, cudaStream_t s) { fx_launch_bf_update(c->D, l, n, stage, s); });
     }
     per_block(c, form, [&](const int *l, int n, cudaStream_t s) {
-        fx_launch_cell_update(c->D, l, n, stage, c->cfg.gravity, full, s);
+        fx_launch_cell_update(c->D, l, n, stage, c->cfg.gravity, full, c->next_dt ? 1 : 0, s);
     });
     refill(c, form, dst);
 }
@@ -640,10 +641,24 @@ int build_step_graph(fx_ctx *c)
     return FX_SUCCESS;
 }
 
+/* The RK2 driver loop on one rank takes each step's timestep minimum from the
+ * cell update that made its state; a run's first step gets it from k_calc_dt.
+ * eSSPRK ends in blends, and a sharded step minimises over the ranks first:
+ * they pass over the state. */
+bool steps_carry_dt(const fx_ctx *c) { return c->nranks == 1 && c->cfg.integrator == FX_INT_RK2; }
+
 /* one batched driver step: calc_dt, dt selection, the step, dt_src clamp;
  * sharded, the dt and dt_src keys are minimised over the ranks */
 void run_seq(fx_ctx *c, double cfl)
 {
+    if (steps_carry_dt(c)) {
+        fx_launch_step_begin(c->D, c->stream);
+        c->next_dt = true;
+        step_seq(c, FX_FORM_BATCHED);
+        c->next_dt = false;
+        fx_launch_step_end(c->D, c->stream);
+        return;
+    }
     fx_launch_reset_reductions(c->D, 1, c->stream);
     fx_launch_calc_dt(c->D, c->d_active, c->nactive, 0, cfl, c->stream);
     shard_min(c, 0, 1);
@@ -1885,7 +1900,7 @@ int fx_update_cells(fx_ctx *c, int b, int stage, double dt, double *dt_src)
     expand_faces(c);
     fx_launch_set_dt(c->D, dt, c->stream);
     if (dt_src) fx_launch_reset_reductions(c->D, 2, c->stream);
-    fx_launch_cell_update(c->D, c->d_ids + b, 1, stage, c->cfg.gravity, 1, c->stream);
+    fx_launch_cell_update(c->D, c->d_ids + b, 1, stage, c->cfg.gravity, 1, 0, c->stream);
     c->last_slot = stage == 1 ? 1 : 0;
     if (dt_src) {
         double v;
@@ -2066,6 +2081,10 @@ int fx_run(fx_ctx *c, int form, int nsteps, double cfl, double dt_factor, double
     v.dt_mult = dt_mult(c);
     *c->h_ctl = v;
     fx_launch_set_ctl(c->D, v, c->stream);
+    if (steps_carry_dt(c)) {
+        fx_launch_reset_reductions(c->D, 1, c->stream);
+        fx_launch_calc_dt(c->D, c->d_active, c->nactive, 0, cfl, c->stream);
+    }
     int rc;
     if (eager(c)) {
         for (int n = 0; n < nsteps; ++n) run_seq(c, cfl);
@@ -2104,7 +2123,7 @@ int fx_time_phase(fx_ctx *c, int phase, int reps, double dt, double *ms)
         case FX_PHASE_FLUX: fx_launch_flux(c->D, c->d_active, c->nactive, 3, 0, 0, 0, s); break;
         case FX_PHASE_EMF: fx_launch_emf(c->D, c->d_active, c->nactive, 0, 0, 0, s); break;
         case FX_PHASE_CT: fx_launch_bf_update(c->D, c->d_active, c->nactive, 1, s); break;
-        case FX_PHASE_CELLS: fx_launch_cell_update(c->D, c->d_active, c->nactive, 1, c->cfg.gravity, 0, s); break;
+        case FX_PHASE_CELLS: fx_launch_cell_update(c->D, c->d_active, c->nactive, 1, c->cfg.gravity, 0, 0, s); break;
         case FX_PHASE_GHOST: ghost_fill(c, 1); break;
         default: cudaGraphLaunch(c->g_step, s); break;
         }

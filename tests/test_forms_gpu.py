@@ -128,11 +128,12 @@ AMR_COORD = (-0.7, 0.7, -0.7, 0.7, -0.7, 0.7)
 @pytest.mark.parametrize("use_bj", [False, True])
 def test_amr_steps_of_both_forms_are_the_same(mhd, use_bj):
     """Three levels: corrections on the compact fluxes, waves with pairs,
-    single operations and face-prolongation groups."""
+    single operations and face-prolongation groups; steps enough for the
+    plain form's graph."""
     blocks = mesh.static_amr_mesh((3,) * 3, AMR_COORD, 2, mesh.ball_refiner((0.1, 0.05, 0.0), (0.4, 0.2)))
     recs = fx.plan_export(fx.make_config(mhd, 5.0 / 3.0, AMR_COORD), mesh.to_desc(blocks), 3) if mhd else None
     W, Bf = problems.amr_blast(blocks, recs, mhd=mhd)
-    _run_both(blocks, AMR_COORD, W, Bf, use_bj=use_bj)
+    _run_both(blocks, AMR_COORD, W, Bf, steps=6, use_bj=use_bj)
 
 
 @pytest.mark.parametrize("root", [(1, 1, 1), (2, 3, 3)])
@@ -144,7 +145,7 @@ def test_uniform_steps_of_both_forms_are_the_same(root, recon, integ, mhd):
     W, Bf = problems.fourier_mhd(blocks, nmodes=4, kmax=3)
     if not mhd:
         W, Bf = np.ascontiguousarray(W[:, :6]), None
-    _run_both(blocks, COORD, W, Bf, recon=recon, integrator=integ)
+    _run_both(blocks, COORD, W, Bf, steps=5, recon=recon, integrator=integ)
 
 
 @pytest.mark.parametrize("mhd", [True, False])
@@ -199,3 +200,23 @@ def test_sharded_steps_match_one_device(mhd):
     for c in ctxs + [one]:
         c.close()
     group.close()
+
+
+def test_driver_loop_stops_and_goes_on_as_the_plain_form():
+    """dt carried from step to step (batched RK2) against dt computed per step
+    (plain): a run cut short at t_end, a run that starts at t_end, another
+    CFL number, and state changed between runs."""
+    got = []
+    for form in (fx.FORM_PLAIN, fx.FORM_BATCHED):
+        ctx, n = _context((2, 2, 4))
+        clocks = [ctx.run(form, 3, 0.4, 1.2, 1.0e30, (0.0, 0.0, 0))]
+        clocks.append(ctx.run(form, 9, 0.4, 1.2, 1.4 * clocks[0][0], clocks[0]))
+        clocks.append(ctx.run(form, 2, 0.4, 1.2, clocks[1][0], clocks[1]))
+        clocks.append(ctx.run(form, 2, 0.2, 1.2, 1.0e30, clocks[2]))
+        ctx.step(form, 0.5 * clocks[3][1])
+        clocks.append(ctx.run(form, 2, 0.2, 2.0, 1.0e30, clocks[3]))
+        got.append((clocks, _state(ctx, n)))
+        ctx.close()
+    assert got[0][0] == got[1][0]
+    assert got[0][0][2] == got[0][0][1]
+    _same(got[0][1], got[1][1])
