@@ -2009,34 +2009,74 @@ void fx_plan_workspace_recycle(FxPlanWorkspace *ws, FxPlan &&old)
 
 namespace {
 
-/* ops [b0, b1) in order: every one that make() accepts, joined with the
- * next where joins() says so, to `packed`, the others to `rest`; in parts by
- * thread (a pair across a part's end stays apart) */
+/* Packs one list of operations, wave by wave and in order: every one that
+ * make() accepts, joined with the next where joins() says so, to `packed`, the
+ * others to `rest` (null: none).  The waves are cut into parts (a pair across a
+ * part's end stays apart); one pass counts per part, a second writes into
+ * arrays that its threads are the first to touch: 512 blocks (10 M
+ * operations) 170 ms with vectors that grow, 20 ms so. */
 template <class Op, class Packed, class Joins, class Make>
-void pack_range(const std::vector<Op> &ops, int b0, int b1, std::vector<Packed> &packed, std::vector<Op> &rest,
-    Joins joins, Make make)
+void pack_list(const std::vector<Op> &ops, const std::vector<int> &wave, FxArr<Packed> &packed, FxArr<Op> *rest,
+    std::vector<int> &pbegin, std::vector<int> *rbegin, Joins joins, Make make)
 {
-    const int n = b1 - b0;
-    const int nt = n < 50000 ? 1 : std::max(1, compile_threads());
-    std::vector<std::vector<Packed>> ps(nt);
-    std::vector<std::vector<Op>> rs(nt);
-    parallel_for(nt, [&](int t) {
-        const int lo = b0 + (int)((int64_t)n * t / nt), hi = b0 + (int)((int64_t)n * (t + 1) / nt);
-        ps[t].reserve((hi - lo) / 2 + 1);
-        for (int q = lo; q < hi; ++q) {
-            const bool two = q + 1 < hi && joins(ops[q], ops[q + 1]);
+    struct Part {
+        int lo, hi;
+        size_t np, nr;
+    };
+    const int nt = compile_threads();
+    const int len = std::max<int>(8192, (int)(ops.size() / (8 * (size_t)nt)) + 1);
+    std::vector<Part> parts;
+    std::vector<size_t> first; /* a wave's first part */
+    const int nw = (int)wave.size() - 1;
+    for (int w = 0; w < nw; ++w) {
+        first.push_back(parts.size());
+        for (int lo = wave[w]; lo < wave[w + 1]; lo += len) {
+            parts.push_back(Part{lo, std::min(lo + len, wave[w + 1]), 0, 0});
+        }
+    }
+    first.push_back(parts.size());
+    auto walk = [&](const Part &p, auto put, auto keep) {
+        for (int q = p.lo; q < p.hi; ++q) {
+            const bool two = q + 1 < p.hi && joins(ops[q], ops[q + 1]);
             Packed x;
             if (make(ops[q], two, x)) {
-                ps[t].push_back(x);
+                put(x);
                 q += two ? 1 : 0;
             } else {
-                rs[t].push_back(ops[q]);
+                keep(ops[q]);
             }
         }
+    };
+    const int np = (int)parts.size();
+    const int workers = std::max(1, std::min(nt, np));
+    parallel_for(workers, [&](int t) {
+        for (int n = t; n < np; n += workers) {
+            size_t a = 0, r = 0;
+            walk(parts[n], [&](const Packed &) { ++a; }, [&](const Op &) { ++r; });
+            parts[n].np = a;
+            parts[n].nr = r;
+        }
     });
-    for (int t = 0; t < nt; ++t) {
-        packed.insert(packed.end(), ps[t].begin(), ps[t].end());
-        rest.insert(rest.end(), rs[t].begin(), rs[t].end());
+    size_t a = 0, r = 0;
+    for (Part &p : parts) { /* counts -> offsets */
+        const size_t pa = p.np, pr = p.nr;
+        p.np = a;
+        p.nr = r;
+        a += pa;
+        r += pr;
+    }
+    packed.make(a);
+    if (rest) rest->make(r);
+    parallel_for(workers, [&](int t) {
+        for (int n = t; n < np; n += workers) {
+            Packed *o = packed.data() + parts[n].np;
+            Op *k = rest ? rest->data() + parts[n].nr : nullptr;
+            walk(parts[n], [&](const Packed &x) { *o++ = x; }, [&](const Op &x) { *k++ = x; });
+        }
+    });
+    for (int w = 0; w <= nw; ++w) {
+        pbegin.push_back((int)(first[w] < parts.size() ? parts[first[w]].np : a));
+        if (rbegin) rbegin->push_back((int)(first[w] < parts.size() ? parts[first[w]].nr : r));
     }
 }
 
@@ -2047,45 +2087,35 @@ int32_t pair_dst(int32_t key, bool two) { return two ? key : (int32_t)((uint32_t
 void fx_pack_program(const FxProgram &g, FxPacked &out)
 {
     out = FxPacked();
-    std::vector<FxBop> none;
-    for (auto &b : out.begin) b.assign(1, 0);
-    for (int w = 0; w < g.nwaves(); ++w) {
-        pack_range(g.cell_ops, g.cell_begin[w], g.cell_begin[w + 1], out.cp, out.cg,
-            [](const FxGop &a, const FxGop &b) {
-                return a.type == FX_GOP_COPY && b.type == FX_GOP_COPY && b.dst == a.dst + 1 && b.src == a.src + 1;
-            },
-            [](const FxGop &a, bool two, FxPair &x) {
-                x = FxPair{pair_dst(a.dst, two), a.src};
-                return a.type == FX_GOP_COPY;
-            });
-        pack_range(g.face_ops, g.face_begin[w], g.face_begin[w + 1], out.fp, out.fg,
-            [](const FxGop &a, const FxGop &b) {
-                return a.type == FX_FOP_COPY && b.type == FX_FOP_COPY && (a.aux & 3) == (b.aux & 3) &&
-                    b.dst == a.dst + 1 && b.src == a.src + 1;
-            },
-            [](const FxGop &a, bool two, FxPair &x) {
-                const int db = a.dst >> 15, sb = a.src >> 15;
-                x = FxPair{pair_dst(FX_PFACE(db, a.aux & 3, a.dst & 32767), two),
-                    FX_PFACE(sb, a.aux & 3, a.src & 32767)};
-                return a.type == FX_FOP_COPY && db < FX_PFACE_BLOCKS && sb < FX_PFACE_BLOCKS;
-            });
-        pack_range(g.b_ops, g.b_begin[w], g.b_begin[w + 1], out.b, none,
-            [](const FxBop &a, const FxBop &b) {
-                bool ok = b.dst == a.dst + 1;
-                for (int n = 0; n < 6; ++n) ok = ok && b.f[n] == a.f[n] + 1;
-                return ok;
-            },
-            [](const FxBop &a, bool two, FxBop &x) {
-                x = a;
-                x.pad = two ? 2 : 1;
-                return true;
-            });
-        out.begin[0].push_back((int)out.cp.size());
-        out.begin[1].push_back((int)out.cg.size());
-        out.begin[2].push_back((int)out.fp.size());
-        out.begin[3].push_back((int)out.fg.size());
-        out.begin[4].push_back((int)out.b.size());
-    }
+    pack_list(g.cell_ops, g.cell_begin, out.cp, &out.cg, out.begin[0], &out.begin[1],
+        [](const FxGop &a, const FxGop &b) {
+            return a.type == FX_GOP_COPY && b.type == FX_GOP_COPY && b.dst == a.dst + 1 && b.src == a.src + 1;
+        },
+        [](const FxGop &a, bool two, FxPair &x) {
+            x = FxPair{pair_dst(a.dst, two), a.src};
+            return a.type == FX_GOP_COPY;
+        });
+    pack_list(g.face_ops, g.face_begin, out.fp, &out.fg, out.begin[2], &out.begin[3],
+        [](const FxGop &a, const FxGop &b) {
+            return a.type == FX_FOP_COPY && b.type == FX_FOP_COPY && (a.aux & 3) == (b.aux & 3) &&
+                b.dst == a.dst + 1 && b.src == a.src + 1;
+        },
+        [](const FxGop &a, bool two, FxPair &x) {
+            const int db = a.dst >> 15, sb = a.src >> 15;
+            x = FxPair{pair_dst(FX_PFACE(db, a.aux & 3, a.dst & 32767), two), FX_PFACE(sb, a.aux & 3, a.src & 32767)};
+            return a.type == FX_FOP_COPY && db < FX_PFACE_BLOCKS && sb < FX_PFACE_BLOCKS;
+        });
+    pack_list(g.b_ops, g.b_begin, out.b, (FxArr<FxBop> *)nullptr, out.begin[4], nullptr,
+        [](const FxBop &a, const FxBop &b) {
+            bool ok = b.dst == a.dst + 1;
+            for (int n = 0; n < 6; ++n) ok = ok && b.f[n] == a.f[n] + 1;
+            return ok;
+        },
+        [](const FxBop &a, bool two, FxBop &x) {
+            x = a;
+            x.pad = two ? 2 : 1;
+            return true;
+        });
 }
 
 bool fx_build_plan(const fx_config &cfg, int nblocks, const fx_block_desc *blocks,

@@ -4,6 +4,7 @@
 #ifndef FX_PLAN_H
 #define FX_PLAN_H
 
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -27,13 +28,28 @@ struct FxProgram {
     int nwaves() const { return cell_begin.empty() ? 0 : (int)cell_begin.size() - 1; }
 };
 
-/* The cell, face and cell-field operations of a program's waves sorted for
- * the device (FxWave): neighbouring copies joined to pairs.  The operations
- * of a wave are conflict free, so their order is free. */
+/* an array whose memory is first touched by whoever fills it */
+template <class T>
+struct FxArr {
+    std::unique_ptr<T[]> p;
+    size_t n = 0;
+    void make(size_t count)
+    {
+        p.reset(count ? new T[count] : nullptr);
+        n = count;
+    }
+    size_t size() const { return n; }
+    T *data() { return p.get(); }
+    const T *data() const { return p.get(); }
+    const T &operator[](size_t q) const { return p[q]; }
+};
+
+/* The cell, face and cell-field operations of a program's waves as the device
+ * takes them (FxWave): neighbouring copies joined to pairs. */
 struct FxPacked {
-    std::vector<FxPair> cp, fp;
-    std::vector<FxGop> cg, fg;
-    std::vector<FxBop> b;
+    FxArr<FxPair> cp, fp;
+    FxArr<FxGop> cg, fg;
+    FxArr<FxBop> b;
     std::vector<int> begin[5]; /* per list (in FxWave's order): wave offsets, one more than waves */
 };
 
