@@ -606,6 +606,9 @@ __device__ __noinline__ double fx_edge_eta(FxErr *err, const double *Wb, int b, 
     return eta;
 }
 
+/* two buffers of planes */
+constexpr int kEmfSmem = 2 * FX_EP_COUNT * kEmfNodes * (int)sizeof(double);
+
 /* curl B term of one edge, src/prj_mhd.c:682-709 */
 __device__ __noinline__ double fx_edge_curl_b(const double *bf, const FxBlockDev &B, int bfslot, int dir, int i, int j, int k)
 {
@@ -2125,10 +2128,12 @@ void fx_launch_emf(const FxDev &D, const int *blist, int nlist, int wslot, int b
      * blocks 20.6 us with 10 chunks, 22.7 with 14 */
     constexpr int fill = 592;
     const int nchunk = nlist * 17 <= fill ? 17 : nlist * 2 >= fill ? 2 : (fill + nlist - 1) / nlist;
-    constexpr int smem = 2 * FX_EP_COUNT * kEmfNodes * (int)sizeof(double);
-    static const cudaError_t opted = cudaFuncSetAttribute(k_emf, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    (void)opted;
-    k_emf<<<dim3(nchunk, nlist), kEmfThreads, smem, s>>>(D, blist, wslot, bfslot, nchunk);
+    k_emf<<<dim3(nchunk, nlist), kEmfThreads, kEmfSmem, s>>>(D, blist, wslot, bfslot, nchunk);
+}
+
+cudaError_t fx_prepare_kernels()
+{
+    return cudaFuncSetAttribute(k_emf, cudaFuncAttributeMaxDynamicSharedMemorySize, kEmfSmem);
 }
 
 void fx_launch_bf_update(const FxDev &D, const int *blist, int nlist, int stage, cudaStream_t s)

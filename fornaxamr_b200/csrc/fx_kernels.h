@@ -199,6 +199,10 @@ struct FxXent {
 #define FX_CELL_BLOCK(key) ((key) >> FX_CELL_BITS)
 #define FX_CELL_IDX(key) ((key) & ((1 << FX_CELL_BITS) - 1))
 
+/* per device, before the first launch: k_emf's opt-in to more than 48 KB of
+ * shared memory */
+cudaError_t fx_prepare_kernels();
+
 /* launchers (fx_kernels.cu); all asynchronous on `s` */
 void fx_launch_flux(const FxDev &D, const int *blist, int nlist, int ndir, int wslot, int bfslot,
     int full, cudaStream_t s);

@@ -1200,7 +1200,7 @@ int fx_create(int device, const fx_config *cfg, fx_ctx **out)
     c->device = device;
     c->cfg = *cfg;
     c->nv = cfg->mhd ? 9 : 6;
-    if (cudaSetDevice(device) != cudaSuccess ||
+    if (cudaSetDevice(device) != cudaSuccess || fx_prepare_kernels() != cudaSuccess ||
         cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaMalloc((void **)&c->d_err, sizeof(FxErr)) != cudaSuccess ||
         cudaMalloc((void **)&c->d_red, 3 * sizeof(unsigned long long)) != cudaSuccess ||
