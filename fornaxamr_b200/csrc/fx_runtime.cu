@@ -49,7 +49,13 @@ enum { FX_XG = 0, FX_XF = 1, FX_XE = 2 }; /* ghost fill (cells + faces), flux, E
  * latency each */
 constexpr int FX_LANES = 8;
 
-constexpr size_t FX_STAGE_BYTES = 1 << 20;
+/* staging of large copies from and to pageable memory: host threads and the
+ * size of each thread's two page-locked buffers.  8 MB in all, since locking
+ * pages costs a context's first such copy about 1.5 ms per MB: the 64-block
+ * adjoint's reverse 20.4 ms the first time and 14.3 after it, 26 and 14.7 with
+ * 16 MB, 21 and 15.5 with 4 MB (16 threads 15), 33 and 30 without */
+constexpr int FX_STAGE_THREADS = 8;
+constexpr size_t FX_STAGE_BYTES = (size_t)512 << 10;
 
 struct fx_ctx {
     int device = 0;
@@ -91,10 +97,9 @@ struct fx_ctx {
      * block always on the same one) between lanes_open and lanes_close */
     cudaStream_t lane[FX_LANES] = {};
     cudaEvent_t ev_lane[FX_LANES] = {};
-    /* page-locked staging of large copies from and to pageable memory, two
-     * buffers per lane (allocated by the first one) */
+    /* page-locked staging buffers, two per thread (allocated by the first copy) */
     char *h_stage = nullptr;
-    cudaEvent_t ev_stage[FX_LANES][2] = {};
+    cudaEvent_t ev_stage[FX_STAGE_THREADS][2] = {};
     bool lanes = false;
     cudaStream_t side = nullptr;      /* a wave's face-prolongation groups, beside its copies */
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
@@ -1059,7 +1064,7 @@ void child_groups(const FxAmrRefine &r, bool use_bj, std::vector<FxPop> &out)
 /* Copies `bytes` between host and device in the order of the context's
  * stream; the host side is done when the call returns.  A large copy from
  * or to pageable memory goes through page-locked buffers, a share of the
- * array per host thread and lane (the driver's own staging copies with one
+ * array per host thread (the driver's own staging copies with one
  * thread, 5 to 8 GB/s, and faults a fresh array's pages in one by one).
  * The 64-block adjoint's 74 MB in and 100 MB out: 33 -> 18 ms
  * for the whole gradient. */
@@ -1069,13 +1074,13 @@ int copy_pageable(fx_ctx *c, void *host, void *dev, size_t bytes, bool to_host)
     cudaPointerAttributes at{};
     const bool pageable = cudaPointerGetAttributes(&at, host) != cudaSuccess || at.type == cudaMemoryTypeUnregistered;
     cudaGetLastError();
-    const int lanes = (int)std::min<size_t>(FX_LANES, std::max(1u, std::thread::hardware_concurrency()));
-    bool staged = pageable && bytes >= 8 * FX_STAGE_BYTES && lanes > 1 && make_lanes(c);
+    const int threads = (int)std::min<size_t>(FX_STAGE_THREADS, std::max(1u, std::thread::hardware_concurrency()));
+    bool staged = pageable && bytes >= ((size_t)8 << 20) && threads > 1;
     for (auto &pair : c->ev_stage) {
         for (cudaEvent_t &e : pair) staged = staged && make_event(&e);
     }
     if (staged && !c->h_stage &&
-        cudaMallocHost((void **)&c->h_stage, 2 * FX_LANES * FX_STAGE_BYTES) != cudaSuccess) {
+        cudaMallocHost((void **)&c->h_stage, 2 * FX_STAGE_THREADS * FX_STAGE_BYTES) != cudaSuccess) {
         cudaGetLastError();
         c->h_stage = nullptr;
         staged = false;
@@ -1085,15 +1090,14 @@ int copy_pageable(fx_ctx *c, void *host, void *dev, size_t bytes, bool to_host)
         FX_CUDA(c, cudaStreamSynchronize(c->stream));
         return FX_SUCCESS;
     }
-    FX_CUDA(c, cudaEventRecord(c->ev_fork, c->stream));
     std::atomic<int> failed{0};
     auto share = [&](int l) {
         cudaSetDevice(c->device);
-        const size_t lo = bytes / lanes * l;
-        const size_t hi = l + 1 == lanes ? bytes : bytes / lanes * (l + 1);
+        const size_t lo = bytes / threads * l;
+        const size_t hi = l + 1 == threads ? bytes : bytes / threads * (l + 1);
         const size_t n = (hi - lo + FX_STAGE_BYTES - 1) / FX_STAGE_BYTES;
-        cudaStream_t s = c->lane[l];
-        cudaError_t e = cudaStreamWaitEvent(s, c->ev_fork, 0);
+        cudaStream_t s = c->stream;
+        cudaError_t e = cudaSuccess;
         auto part = [&](size_t q, size_t &off) {
             off = lo + q * FX_STAGE_BYTES;
             return std::min(FX_STAGE_BYTES, hi - off);
@@ -1123,20 +1127,18 @@ int copy_pageable(fx_ctx *c, void *host, void *dev, size_t bytes, bool to_host)
                 put(q);
             }
         }
-        if (e == cudaSuccess) e = cudaEventRecord(c->ev_lane[l], s);
         if (e != cudaSuccess) failed = (int)e;
     };
     std::vector<std::thread> pool;
     int started = 1;
     try {
-        for (; started < lanes; ++started) pool.emplace_back(share, started);
+        for (; started < threads; ++started) pool.emplace_back(share, started);
     } catch (const std::exception &) { /* no more threads: the shares left are done here */
     }
     share(0);
-    for (int l = started; l < lanes; ++l) share(l);
+    for (int l = started; l < threads; ++l) share(l);
     for (std::thread &t : pool) t.join();
     if (failed) return set_err(c, FX_ECUDA, "staged copy: %s", cudaGetErrorString((cudaError_t)failed.load()));
-    for (int l = 0; l < lanes; ++l) FX_CUDA(c, cudaStreamWaitEvent(c->stream, c->ev_lane[l], 0));
     return FX_SUCCESS;
 }
 
