@@ -694,6 +694,8 @@ bool plain_graph(fx_ctx *c)
     const size_t per_block = c->cfg.integrator == FX_INT_ESSPRK10_4 ? 80 : 12; /* launches of a step */
     const size_t n = c->plan.active.size();
     if (c->D.br_mode || c->nranks > 1 || n < 2 || n * per_block > 8192) return false;
+    cudaStreamCaptureStatus caller = cudaStreamCaptureStatusNone; /* a capture of the caller's takes the launches */
+    if (cudaStreamIsCapturing(c->stream, &caller) != cudaSuccess || caller != cudaStreamCaptureStatusNone) return false;
     if (c->g_plain) return true;
     if (++c->plain_steps <= 3 || !make_lanes(c)) return false;
     cudaGraph_t g = nullptr;

@@ -342,8 +342,9 @@ int fx_stage(fx_ctx *ctx, int form, int stage, double dt, double *dt_src);
 /* prj_timeint_step (src/prj_timeint.h:31-33): one RK2 step, or one
  * eSSPRK10_4 step (prj_timeint_eSSPRK10_4_advance, src/prj_timeint.c:2671-2729).
  * *dt_src (may be NULL) receives the minimum source time step.
- * FX_FORM_BATCHED replays a captured CUDA graph; it does not synchronise
- * unless dt_src != NULL. */
+ * FX_FORM_BATCHED replays a captured CUDA graph, FX_FORM_PLAIN one of its
+ * per-block launches from the fourth step of a mesh on (not while the caller
+ * captures the stream); it does not synchronise unless dt_src != NULL. */
 int fx_step(fx_ctx *ctx, int form, double dt, double *dt_src);
 /* The driver loop of src/main.c:485-562 without I/O: calc_dt, dt growth
  * limit dt_factor, clip to t_end, step, dt_src clamp; device resident.

@@ -220,3 +220,32 @@ def test_driver_loop_stops_and_goes_on_as_the_plain_form():
     assert got[0][0] == got[1][0]
     assert got[0][0][2] == got[0][0][1]
     _same(got[0][1], got[1][1])
+
+
+@pytest.mark.parametrize("before", [1, 5])
+def test_plain_step_inside_a_capture_of_the_callers(before):
+    """A plain step that the caller captures on the context's stream, before
+    and after the library keeps a graph of its own: launched, it is the step."""
+    import torch
+    got = []
+    for captured in (False, True):
+        ctx, n = _context((2, 2, 1))
+        dt = 0.3 * ctx.calc_dt(0.4)
+        for _ in range(before):
+            ctx.step(fx.FORM_PLAIN, dt)
+        if captured:
+            g = torch.cuda.CUDAGraph()
+            torch.cuda.synchronize()
+            with torch.cuda.stream(torch.cuda.ExternalStream(ctx.stream())):
+                g.capture_begin(capture_error_mode="thread_local")
+                ctx.step(fx.FORM_PLAIN, dt, want_dt_src=False)
+                g.capture_end()
+                g.replay()
+                g.replay()
+        else:
+            for _ in range(2):
+                ctx.step(fx.FORM_PLAIN, dt)
+        ctx.sync()
+        got.append(_state(ctx, n))
+        ctx.close()
+    _same(got[0], got[1])
