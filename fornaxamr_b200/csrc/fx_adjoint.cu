@@ -287,7 +287,10 @@ struct AdjCellAcc {
  * and reverse it.  Bounded to 128 registers (four resident CTAs per SM): the
  * reverse HLLD is latency-bound on dependent FP64 operations, and the
  * occupancy gained outweighs the spills (measured: 20 % faster than 255
- * registers). */
+ * registers; 168 registers 3 % slower, 64 x 9 at 96 registers 10 %).  64
+ * blocks, reverse sweep of five steps: 6.32 -> 5.38 ms with the two sides'
+ * adjoints held by value (the stack held both structures) and 14 divisions
+ * per face instead of 37 in the fast speeds and outer stars. */
 __global__ void __launch_bounds__(128, 4) k_adj_flux(FxAdjDev A, const int *__restrict__ blist, int stage)
 {
     const int dir = blockIdx.y;

@@ -106,7 +106,8 @@ FX_HD void fxa_state_vjp(const double *w, const FxaS &sb, double *wb, double &pb
     pb += sb.p + sb.pt;
 }
 
-/* fx_hlld_fast_speed */
+/* fx_hlld_fast_speed.  Adjoints are divided by rho once, before the products
+ * they go into: as many roundings as dividing each product. */
 FX_HD void fxa_fast_speed_vjp(const FxHlldState &s, double cfb, FxaS &sb)
 {
     if (cfb == 0.0) {
@@ -132,14 +133,17 @@ FX_HD void fxa_fast_speed_vjp(const FxHlldState &s, double cfb, FxaS &sb)
     const double bx2rb = -4.0 * a2 * discb;
     a2b += s1b;
     const double b2rb = s1b;
-    sb.p += a2b * s.gamma / s.rho;
-    sb.rho -= a2b * a2 / s.rho;
-    sb.rho -= b2rb * b2r / s.rho;
-    sb.bx += b2rb * 2.0 * s.bx / s.rho;
-    sb.by += b2rb * 2.0 * s.by / s.rho;
-    sb.bz += b2rb * 2.0 * s.bz / s.rho;
-    sb.bx += bx2rb * 2.0 * s.bx / s.rho;
-    sb.rho -= bx2rb * bx2r / s.rho;
+    const double a2r = a2b / s.rho;
+    const double b2rr = b2rb / s.rho;
+    const double bx2rr = bx2rb / s.rho;
+    sb.p += a2r * s.gamma;
+    sb.rho -= a2r * a2;
+    sb.rho -= b2rr * b2r;
+    sb.bx += b2rr * 2.0 * s.bx;
+    sb.by += b2rr * 2.0 * s.by;
+    sb.bz += b2rr * 2.0 * s.bz;
+    sb.bx += bx2rr * 2.0 * s.bx;
+    sb.rho -= bx2rr * bx2r;
 }
 
 /* fx_hlld_state_f, all nine components */
@@ -273,7 +277,7 @@ FX_HD void fxa_outer_star_vjp(const FxHlldState &s, double S, double SM, double 
     const double es = num / sd;
 
     const double numb = stb.e / sd;
-    double sdb = -stb.e * es / sd;
+    double sdb = -numb * es;
     double alphab = numb * s.e;
     sb.e += numb * alpha;
     sb.pt -= numb * s.vx;
@@ -313,13 +317,14 @@ FX_HD void fxa_outer_star_vjp(const FxHlldState &s, double S, double SM, double 
         double mfb = bysb * s.by;
         sb.bz += bzsb * mf;
         mfb += bzsb * s.bz;
-        SMb += qb / den;
-        sb.vx -= qb / den;
-        double denb = -qb * q / den;
-        sb.rho += mfb * alpha * alpha / den;
-        alphab += mfb * 2.0 * s.rho * alpha / den;
-        sb.bx -= mfb * 2.0 * s.bx / den;
-        denb -= mfb * mf / den;
+        qb /= den;
+        mfb /= den;
+        SMb += qb;
+        sb.vx -= qb;
+        const double denb = -qb * q - mfb * mf;
+        sb.rho += mfb * alpha * alpha;
+        alphab += mfb * 2.0 * s.rho * alpha;
+        sb.bx -= mfb * 2.0 * s.bx;
         sb.rho += denb * alpha * sd;
         alphab += denb * s.rho * sd;
         sdb += denb * s.rho * alpha;
@@ -328,9 +333,10 @@ FX_HD void fxa_outer_star_vjp(const FxHlldState &s, double S, double SM, double 
     SMb += stb.vx;
     sb.bx += stb.bx;
     sb.ye += stb.ye;
-    sb.rho += stb.rho * alpha / sd;
-    alphab += stb.rho * s.rho / sd;
-    sdb -= stb.rho * rhos / sd;
+    const double rb = stb.rho / sd;
+    sb.rho += rb * alpha;
+    alphab += rb * s.rho;
+    sdb -= rb * rhos;
     Sb += alphab;
     sb.vx -= alphab;
     Sb += sdb;
@@ -369,10 +375,16 @@ FX_HD void fxa_hlld_vjp(const double *WL, const double *WR, double pL, double pR
     if (0.0 <= SL || SR <= 0.0) {
         const bool isL = 0.0 <= SL;
         const FxHlldState &X = isL ? L : R;
-        FxaS &Xb = isL ? Lb : Rb;
+        FxaS Xb;
+        fxa_clear(Xb);
         fxa_flux_vjp(X, Fb, Xb);
         fxa_outputs_vjp(X.vx, X.vy, X.vz, X.bx, X.by, X.bz, outb, xb);
         Xb.vx += xb[0]; Xb.vy += xb[1]; Xb.vz += xb[2]; Xb.bx += xb[3]; Xb.by += xb[4]; Xb.bz += xb[5];
+        if (isL) {
+            Lb = Xb;
+        } else {
+            Rb = Xb;
+        }
     } else {
         const double denom = R.rho * (SR - R.vx) - L.rho * (SL - L.vx);
         const double smnum = R.rho * R.vx * (SR - R.vx) - L.rho * L.vx * (SL - L.vx) + (L.pt - R.pt);
@@ -385,7 +397,11 @@ FX_HD void fxa_hlld_vjp(const double *WL, const double *WR, double pL, double pR
             /* HLL fallback: Uh_v = (SR ru - SL lu + lf - rf) / (SR - SL),
              * F_v = (SR lf - SL rf + SL SR (ru - lu)) / (SR - SL) */
             const double inv = 1.0 / (SR - SL);
-            double Uh[9];
+            double Uh[9], Fq[9]; /* Fb copied: an index of run time keeps an array in local memory */
+#pragma unroll
+            for (int v = 0; v < 9; ++v) {
+                Fq[v] = Fb[v];
+            }
             for (int v = 0; v < 9; ++v) {
                 Uh[v] = (SR * fx_hlld_state_u(R, v) - SL * fx_hlld_state_u(L, v) + fx_hlld_state_f(L, v) -
                     fx_hlld_state_f(R, v)) * inv;
@@ -406,7 +422,7 @@ FX_HD void fxa_hlld_vjp(const double *WL, const double *WR, double pL, double pR
             for (int v = 0; v < 9; ++v) {
                 const double lf = fx_hlld_state_f(L, v), rf = fx_hlld_state_f(R, v);
                 const double lu = fx_hlld_state_u(L, v), ru = fx_hlld_state_u(R, v);
-                const double fb = Fb[v];
+                const double fb = Fq[v];
                 const double du = ru - lu;
                 SRb += fb * (lf + SL * du) * inv + Uhb[v] * ru * inv;
                 SLb += fb * (-rf + SR * du) * inv - Uhb[v] * lu * inv;
@@ -422,7 +438,12 @@ FX_HD void fxa_hlld_vjp(const double *WL, const double *WR, double pL, double pR
             const bool bn_small = (0.5 * bn * bn < FX_HLLD_SMALL * pts);
             const bool left = (0.0 <= SM);
             const FxHlldState &N = left ? L : R;
-            FxaS &Nb = left ? Lb : Rb;
+            /* the near and the far side's adjoints, given to left and right
+             * at the end: references chosen at run time would keep all four
+             * structures in local memory */
+            FxaS Nb, Frb;
+            fxa_clear(Nb);
+            fxa_clear(Frb);
             const double SN = left ? SL : SR;
             double SNb = 0.0;
             FxHlldStar Ns;
@@ -443,7 +464,6 @@ FX_HD void fxa_hlld_vjp(const double *WL, const double *WR, double pL, double pR
                 fxa_ustar_vjp(Ns, Fb, SN, Nsb);
             } else {
                 const FxHlldState &Fr = left ? R : L;
-                FxaS &Frb = left ? Rb : Lb;
                 const double SF = left ? SR : SL;
                 double SFb = 0.0;
                 FxHlldStar Fs;
@@ -571,10 +591,13 @@ FX_HD void fxa_hlld_vjp(const double *WL, const double *WR, double pL, double pR
             fxa_outer_star_vjp(N, SN, SM, pts, Nsb, Nb, SNb, SMb, ptsb);
             if (left) {
                 SLb += SNb;
+                Lb = Nb;
+                Rb = Frb;
             } else {
                 SRb += SNb;
+                Rb = Nb;
+                Lb = Frb;
             }
-            (void)bn_small;
         }
         /* pts = 0.5 (ptl + ptr) */
         const double ptlb = 0.5 * ptsb;
@@ -591,7 +614,7 @@ FX_HD void fxa_hlld_vjp(const double *WL, const double *WR, double pL, double pR
         Rb.vx -= ptrb * R.rho * ((SM - R.vx) + (SR - R.vx));
         /* SM = smnum / denom */
         const double smnb = SMb / denom;
-        const double denb = -SMb * SM / denom;
+        const double denb = -smnb * SM;
         Rb.rho += smnb * R.vx * (SR - R.vx);
         Rb.vx += smnb * R.rho * (SR - 2.0 * R.vx);
         SRb += smnb * R.rho * R.vx;
