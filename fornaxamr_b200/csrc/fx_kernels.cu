@@ -28,6 +28,10 @@ namespace {
 
 constexpr int kPlane = FX_NSTAGES * FX_NCELLS; /* stride between variables of W */
 
+/* the face arrays take no more memory than the reference's tiles would */
+static_assert(FX_CF_COUNT + FX_CX_COUNT + FX_VN_COUNT + FX_VT_COUNT <= (3 * 9 + 9) * FX_NCELLS, "MHD");
+static_assert(FX_CF_COUNT + FX_VN_COUNT + FX_VT_COUNT <= (3 * 6 + 9) * FX_NCELLS, "hydro");
+
 __device__ __forceinline__ int fx_axis_stride(int dir)
 {
     return dir == 0 ? FX_PBS * FX_PBS : dir == 1 ? FX_PBS : 1;
@@ -275,8 +279,8 @@ __device__ __forceinline__ void fx_flux_dir(const FxDev &D, const int *__restric
         /* the pressure takes the normal field's (unreconstructed) bits */
         fx_recon_pair_br(pS, pL, pR, br, 4 * FX_B1);
     }
-    const size_t fbase = (size_t)b * FX_FLUX_COUNT(nv) + (size_t)dir * nv * FX_NCELLS;
-    const size_t vbase = (size_t)b * FX_VR_COUNT + (size_t)dir * 3 * FX_NCELLS;
+    /* the transverse velocities of the plain form */
+    double *vt = D.vt + (size_t)b * FX_VT_COUNT + (size_t)dir * 2 * FX_NCELLS + cR;
     if (MHD) {
         const double *bnp = D.Bf + (size_t)b * FX_BF_COUNT + ((size_t)dir * FX_NSTAGES + bfslot) * FX_NFACES +
             fx_face_idx(dir, i, j, k);
@@ -304,29 +308,25 @@ __device__ __forceinline__ void fx_flux_dir(const FxDev &D, const int *__restric
                 atomicAdd(D.br_flips, (unsigned long long)br.flips);
             }
         }
-        if constexpr (FULL) {
-#pragma unroll
-            for (int lv = 0; lv < 9; ++lv) {
-                D.flux[fbase + fx_bidx(9, fx_gmap(dir, lv), i, j, k)] = o.F[lv];
-            }
-        } else if ((unsigned)i < (dir == 0 ? FX_BS + 1u : FX_BS) && (unsigned)j < (dir == 1 ? FX_BS + 1u : FX_BS) &&
-            (unsigned)k < (dir == 2 ? FX_BS + 1u : FX_BS)) {
-            /* the transverse ghost ring serves the EMFs only */
-            double *cf = D.cf + (size_t)b * FX_CF_COUNT + fx_cf_idx(dir, i, j, k);
-            const int plane = fx_cf_plane(dir);
+        const bool own = fx_is_face(dir, 0, i, j, k); /* the ghost layer serves the EMFs only */
+        if (FULL || own) {
+            double *f = own ? D.cf + (size_t)b * FX_CF_COUNT + fx_cf_idx(dir, i, j, k)
+                            : D.cx + (size_t)b * FX_CX_COUNT + fx_cx_idx(dir, i, j, k);
+            const int plane = own ? fx_cf_plane(dir) : fx_cx_plane(dir);
 #pragma unroll
             for (int lv = 0; lv < 6; ++lv) {
-                cf[fx_gmap(dir, lv) * plane] = o.F[lv];
+                f[fx_gmap(dir, lv) * plane] = o.F[lv];
             }
         }
         const size_t bvi = (size_t)b * FX_BV_COUNT + (size_t)dir * FX_NCELLS + cR;
+        D.vn[bvi] = o.v[0];
         if constexpr (FULL) {
 #pragma unroll
-            for (int m = 0; m < 3; ++m) {
-                D.vr[vbase + fx_bidx(3, (dir + m) % 3, i, j, k)] = o.v[m];
+            for (int lv = 6; lv < 9; ++lv) {
+                D.cx[(size_t)b * FX_CX_COUNT + fx_cx_field(dir, fx_gmap(dir, lv), i, j, k)] = o.F[lv];
             }
-        } else {
-            D.vn[bvi] = o.v[0];
+            vt[0] = o.v[1];
+            vt[FX_NCELLS] = o.v[2];
         }
         D.bv1[bvi] = o.bv1;
         D.bv2[bvi] = o.bv2;
@@ -357,19 +357,12 @@ __device__ __forceinline__ void fx_flux_dir(const FxDev &D, const int *__restric
         const int plane = fx_cf_plane(dir);
 #pragma unroll
         for (int lv = 0; lv < 6; ++lv) {
-            if constexpr (FULL) {
-                D.flux[fbase + fx_bidx(6, fx_gmap(dir, lv), i, j, k)] = F[lv];
-            } else {
-                cf[fx_gmap(dir, lv) * plane] = F[lv];
-            }
+            cf[fx_gmap(dir, lv) * plane] = F[lv];
         }
+        D.vn[(size_t)b * FX_VN_COUNT + (size_t)dir * FX_NCELLS + cR] = v[0];
         if constexpr (FULL) {
-#pragma unroll
-            for (int m = 0; m < 3; ++m) {
-                D.vr[vbase + fx_bidx(3, (dir + m) % 3, i, j, k)] = v[m];
-            }
-        } else {
-            D.vn[(size_t)b * FX_VN_COUNT + (size_t)dir * FX_NCELLS + cR] = v[0];
+            vt[0] = v[1];
+            vt[FX_NCELLS] = v[2];
         }
     }
 }
@@ -435,9 +428,7 @@ __device__ __forceinline__ double fx_cell_emf(const double *Wb, int dir, int c)
     return bA * vB - bB * vA;
 }
 
-/* FULL: the plain form, normal velocities in vr; else the batched form
- * on a short list, in vn */
-template <bool FULL>
+/* the plain form, and the batched form on a short list */
 __global__ void __launch_bounds__(128) k_emf_edges(FxDev D, const int *__restrict__ blist, int wslot, int bfslot)
 {
     if (D.ctl->skip) {
@@ -470,6 +461,8 @@ __global__ void __launch_bounds__(128) k_emf_edges(FxDev D, const int *__restric
     const double *Wb = D.W + (size_t)b * FX_W_COUNT(9) + (size_t)wslot * FX_NCELLS;
     const double *bv1r = D.bv1 + (size_t)b * FX_BV_COUNT + (size_t)right * FX_NCELLS;
     const double *bv2u = D.bv2 + (size_t)b * FX_BV_COUNT + (size_t)up * FX_NCELLS;
+    const double *vnr = D.vn + (size_t)b * FX_VN_COUNT + (size_t)right * FX_NCELLS;
+    const double *vnu = D.vn + (size_t)b * FX_VN_COUNT + (size_t)up * FX_NCELLS;
     double f[4], c[4], vn[4];
     /* face0 = e (right-normal), face1 = e (up-normal), face2 = e - up
      * (right-normal), face3 = e - right (up-normal) */
@@ -481,21 +474,10 @@ __global__ void __launch_bounds__(128) k_emf_edges(FxDev D, const int *__restric
     c[1] = fx_cell_emf(Wb, dir, c1);
     c[2] = fx_cell_emf(Wb, dir, c2);
     c[3] = fx_cell_emf(Wb, dir, c3);
-    if constexpr (FULL) {
-        const double *vrr = D.vr + (size_t)b * FX_VR_COUNT + (size_t)right * 3 * FX_NCELLS;
-        const double *vru = D.vr + (size_t)b * FX_VR_COUNT + (size_t)up * 3 * FX_NCELLS;
-        vn[0] = vrr[fx_bidx_cell(3, right, c0)];
-        vn[1] = vru[fx_bidx_cell(3, up, c0)];
-        vn[2] = vrr[fx_bidx_cell(3, right, c1)];
-        vn[3] = vru[fx_bidx_cell(3, up, c3)];
-    } else {
-        const double *vrr = D.vn + (size_t)b * FX_VN_COUNT + (size_t)right * FX_NCELLS;
-        const double *vru = D.vn + (size_t)b * FX_VN_COUNT + (size_t)up * FX_NCELLS;
-        vn[0] = vrr[c0];
-        vn[1] = vru[c0];
-        vn[2] = vrr[c1];
-        vn[3] = vru[c3];
-    }
+    vn[0] = vnr[c0];
+    vn[1] = vnu[c0];
+    vn[2] = vnr[c1];
+    vn[3] = vnu[c3];
     const int eidx = fx_edge_idx(dir, e[0], e[1], e[2]);
     for (int n = 0; n < 4; ++n) {
         if (!isfinite(f[n]) || !isfinite(c[n]) || !isfinite(vn[n])) {
@@ -867,8 +849,7 @@ __device__ __forceinline__ double fx_cell_dt(double cfl, double g, double rho, d
     return cfl / denom;
 }
 
-/* FULL: the plain form (face velocities in vr, rhs stored), else the batched
- * one.  DT (the RK2 driver loop): the new state's timestep minimum goes to
+/* FULL: the plain form (rhs stored), else the batched one.  DT (the RK2 driver loop): the new state's timestep minimum goes to
  * D.red[0] for the next step, which then needs no pass over the state for it
  * (the ghost fill leaves active cells alone): a step of 8 blocks 68.1 -> 65.1
  * us, of 512 blocks 2025 -> 1983. */
@@ -898,21 +879,12 @@ __global__ void __launch_bounds__(128) k_cell_update(FxDev D, const int *__restr
 #pragma unroll
     for (int v = 0; v < 6; ++v) {
         double f[3][2];
-        if constexpr (FULL) {
-            const double *fl = D.flux + (size_t)b * FX_FLUX_COUNT(nv);
+        const double *cf = D.cf + (size_t)b * FX_CF_COUNT;
 #pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                f[d][0] = fl[(size_t)d * nv * FX_NCELLS + fx_bidx(nv, v, i, j, k)];
-                f[d][1] = fl[(size_t)d * nv * FX_NCELLS + fx_bidx(nv, v, i + (d == 0), j + (d == 1), k + (d == 2))];
-            }
-        } else {
-            const double *cf = D.cf + (size_t)b * FX_CF_COUNT;
-#pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                const double *q = cf + v * fx_cf_plane(d) + fx_cf_idx(d, i, j, k);
-                f[d][0] = q[0];
-                f[d][1] = q[d == 0 ? FX_BS * FX_BS : d == 1 ? FX_BS : 1];
-            }
+        for (int d = 0; d < 3; ++d) {
+            const double *q = cf + v * fx_cf_plane(d) + fx_cf_idx(d, i, j, k);
+            f[d][0] = q[0];
+            f[d][1] = q[d == 0 ? FX_BS * FX_BS : d == 1 ? FX_BS : 1];
         }
         fluxdiv[v] = -(B.area[0] * (f[0][1] - f[0][0]) + B.area[1] * (f[1][1] - f[1][0]) +
             B.area[2] * (f[2][1] - f[2][0])) / B.vol;
@@ -944,20 +916,11 @@ __global__ void __launch_bounds__(128) k_cell_update(FxDev D, const int *__restr
         rhs[FX_V2] += rho * g2;
         rhs[FX_V3] += rho * g3;
         double vf[3][2];
-        if constexpr (FULL) {
-            const double *vr = D.vr + (size_t)b * FX_VR_COUNT;
+        const double *vn = D.vn + (size_t)b * FX_VN_COUNT + c;
 #pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                vf[d][0] = vr[d * 3 * FX_NCELLS + fx_bidx(3, d, i, j, k)];
-                vf[d][1] = vr[d * 3 * FX_NCELLS + fx_bidx(3, d, i + (d == 0), j + (d == 1), k + (d == 2))];
-            }
-        } else {
-            const double *vn = D.vn + (size_t)b * FX_VN_COUNT + c;
-#pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                vf[d][0] = vn[d * FX_NCELLS];
-                vf[d][1] = vn[d * FX_NCELLS + fx_axis_stride(d)];
-            }
+        for (int d = 0; d < 3; ++d) {
+            vf[d][0] = vn[d * FX_NCELLS];
+            vf[d][1] = vn[d * FX_NCELLS + fx_axis_stride(d)];
         }
         const double v_avg1 = (vf[0][0] + vf[0][1]) * 0.5;
         const double v_avg2 = (vf[1][0] + vf[1][1]) * 0.5;
@@ -1672,18 +1635,21 @@ __global__ void __launch_bounds__(256, BJ ? 4 : 6) k_ghost_wave(FxDev D, FxWave 
     }
 }
 
-/* compact position (variable 0, and the stride between variables) of a flux
- * entry given as direction * nv * cells + AoSoA index of component 0 */
-__device__ __forceinline__ int fx_cf_of_entry(int nv, int entry, int &plane)
+/* component v of block b's flux entry given as direction * nv * cells + AoSoA
+ * index of component 0: a face of the block itself (corrections and
+ * exchanges reach no other) */
+__device__ __forceinline__ double *fx_flux_entry(const FxDev &D, int b, int entry, int v)
 {
+    const int nv = D.nv;
     const int dir = entry / (nv * FX_NCELLS);
     const int r = entry - dir * nv * FX_NCELLS;
     const int u = r / (FX_AOSOA_W * nv);
     const int row = u / FX_AOSOA_KT;
     const int k = (u - row * FX_AOSOA_KT) * FX_AOSOA_W + r % FX_AOSOA_W - FX_NG;
-    const int i = row / FX_PBS;
-    plane = fx_cf_plane(dir);
-    return fx_cf_idx(dir, i - FX_NG, row - i * FX_PBS - FX_NG, k);
+    const int i = row / FX_PBS - FX_NG;
+    const int j = row % FX_PBS - FX_NG;
+    if (v >= 6) return D.cx + (size_t)b * FX_CX_COUNT + fx_cx_field(dir, v, i, j, k);
+    return D.cf + (size_t)b * FX_CF_COUNT + fx_cf_idx(dir, i, j, k) + v * fx_cf_plane(dir);
 }
 
 /* exchanges of a sharded mesh: one thread per listed element */
@@ -1697,11 +1663,8 @@ __device__ __forceinline__ double *fx_xelem(const FxDev &D, const FxXent &x, int
         return D.Bf + (size_t)x.block * FX_BF_COUNT + ((size_t)dir * FX_NSTAGES + slot) * FX_NFACES +
             (x.idx - dir * FX_NFACES);
     }
-    case 2: {
-        int plane;
-        const int e = fx_cf_of_entry(D.nv, x.idx, plane);
-        return D.cf + (size_t)x.block * FX_CF_COUNT + e + q * plane;
-    }
+    case 2:
+        return fx_flux_entry(D, x.block, x.idx, q);
     default:
         return D.emf + (size_t)x.block * FX_EMF_COUNT + x.idx;
     }
@@ -1725,9 +1688,7 @@ __global__ void k_xunpack(FxDev D, const FxXent *__restrict__ ents, int n, const
     for (int q = 0; q < fx_xwidth(x.kind); ++q) *fx_xelem(D, x, slot, q) = buf[x.off + q];
 }
 
-/* coarse/fine corrections; FULL: in the plain form's flux arrays, else the
- * batched form's */
-template <bool FULL>
+/* coarse/fine corrections */
 __global__ void k_flux_correct(FxDev D, const FxCorr *__restrict__ recs, int n, int ncomp)
 {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1738,24 +1699,12 @@ __global__ void k_flux_correct(FxDev D, const FxCorr *__restrict__ recs, int n, 
     const int v = t - r * ncomp;
     const FxCorr rec = recs[r];
     /* sum order of src/prj_riemann.c:1756-1761 */
-    if constexpr (FULL) {
-        /* component v sits FX_AOSOA_W * v further in the AoSoA tile */
-        const double *s = D.flux + (size_t)rec.src_block * FX_FLUX_COUNT(D.nv) + (size_t)v * FX_AOSOA_W;
-        double *d = D.flux + (size_t)rec.dst_block * FX_FLUX_COUNT(D.nv) + (size_t)v * FX_AOSOA_W;
-        d[rec.dst] = 0.25 * (s[rec.src[0]] + s[rec.src[1]] + s[rec.src[2]] + s[rec.src[3]]);
-    } else {
-        const double *s = D.cf + (size_t)rec.src_block * FX_CF_COUNT;
-        double f[4];
+    double f[4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            int plane;
-            const int e = fx_cf_of_entry(D.nv, rec.src[q], plane);
-            f[q] = s[e + v * plane];
-        }
-        int plane;
-        const int e = fx_cf_of_entry(D.nv, rec.dst, plane);
-        D.cf[(size_t)rec.dst_block * FX_CF_COUNT + e + v * plane] = 0.25 * (f[0] + f[1] + f[2] + f[3]);
+    for (int q = 0; q < 4; ++q) {
+        f[q] = *fx_flux_entry(D, rec.src_block, rec.src[q], v);
     }
+    *fx_flux_entry(D, rec.dst_block, rec.dst, v) = 0.25 * (f[0] + f[1] + f[2] + f[3]);
 }
 
 __global__ void k_emf_correct(FxDev D, const FxCorr *__restrict__ recs, int n)
@@ -2085,42 +2034,50 @@ void fx_launch_cell_field_active(const FxDev &D, const int *blist, int nlist, cu
     k_cell_field_active<<<dim3(fx_blocks(NC, 256), nlist), 256, 0, s>>>(D, blist);
 }
 
-/* the batched form's face arrays written in the reference's layout, for a
- * caller that goes on with the plain entry points or downloads them */
-__global__ void __launch_bounds__(256) k_expand_faces(FxDev D, const int *__restrict__ blist)
+/* one block's face arrays in the reference's tiles, for a download */
+__global__ void __launch_bounds__(256) k_face_tiles(FxDev D, int b, int dir, int velocities, double *__restrict__ out)
 {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= FX_NCELLS) {
         return;
     }
-    const int b = blist[blockIdx.y];
-    const int i = t / (FX_PBS * FX_PBS) - FX_NG, j = (t / FX_PBS) % FX_PBS - FX_NG, k = t % FX_PBS - FX_NG;
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        if (i >= 0 && j >= 0 && k >= 0 && i < FX_BS + (d == 0) && j < FX_BS + (d == 1) && k < FX_BS + (d == 2)) {
-            for (int v = 0; v < 6; ++v) {
-                D.flux[(size_t)b * FX_FLUX_COUNT(D.nv) + (size_t)d * D.nv * FX_NCELLS + fx_bidx(D.nv, v, i, j, k)] =
-                    D.cf[(size_t)b * FX_CF_COUNT + v * fx_cf_plane(d) + fx_cf_idx(d, i, j, k)];
-            }
+    if (velocities) {
+        for (int v = 0; v < 3; ++v) {
+            const int m = (v + 3 - dir) % 3;
+            out[fx_bidx_cell(3, v, t)] = m == 0 ? D.vn[(size_t)b * FX_VN_COUNT + dir * FX_NCELLS + t]
+                : D.vt[(size_t)b * FX_VT_COUNT + (2 * dir + m - 1) * FX_NCELLS + t];
         }
-        D.vr[(size_t)b * FX_VR_COUNT + d * 3 * FX_NCELLS + fx_bidx_cell(3, d, t)] =
-            D.vn[(size_t)b * FX_VN_COUNT + d * FX_NCELLS + t];
+        return;
+    }
+    const int i = t / (FX_PBS * FX_PBS) - FX_NG, j = (t / FX_PBS) % FX_PBS - FX_NG, k = t % FX_PBS - FX_NG;
+    const bool own = fx_is_face(dir, 0, i, j, k);
+    const bool ring = D.nv == 9 && fx_is_face(dir, 1, i, j, k); /* own faces too */
+    const double *cf = D.cf + (size_t)b * FX_CF_COUNT;
+    const double *cx = D.cx + (size_t)b * FX_CX_COUNT;
+    for (int v = 0; v < D.nv; ++v) {
+        double f = 0.0;
+        if (v >= 6) {
+            if (ring) f = cx[fx_cx_field(dir, v, i, j, k)];
+        } else if (own) {
+            f = cf[fx_cf_idx(dir, i, j, k) + v * fx_cf_plane(dir)];
+        } else if (ring) {
+            f = cx[fx_cx_idx(dir, i, j, k) + v * fx_cx_plane(dir)];
+        }
+        out[fx_bidx_cell(D.nv, v, t)] = f;
     }
 }
 
-void fx_launch_expand_faces(const FxDev &D, const int *blist, int nlist, cudaStream_t s)
+void fx_launch_face_tiles(const FxDev &D, int b, int dir, int velocities, double *out, cudaStream_t s)
 {
-    if (nlist <= 0) return;
-    k_expand_faces<<<dim3(fx_blocks(FX_NCELLS, 256), nlist), 256, 0, s>>>(D, blist);
+    k_face_tiles<<<fx_blocks(FX_NCELLS, 256), 256, 0, s>>>(D, b, dir, velocities, out);
 }
 
-void fx_launch_emf(const FxDev &D, const int *blist, int nlist, int wslot, int bfslot, int full, cudaStream_t s)
+void fx_launch_emf(const FxDev &D, const int *blist, int nlist, int wslot, int bfslot, cudaStream_t s)
 {
     if (nlist <= 0) return;
-    if (full || nlist < 16) {
+    if (nlist < 16) {
         const dim3 grid(fx_blocks(3 * FX_BS * (FX_BS + 1) * (FX_BS + 1), 128), nlist);
-        if (full) k_emf_edges<true><<<grid, 128, 0, s>>>(D, blist, wslot, bfslot);
-        else k_emf_edges<false><<<grid, 128, 0, s>>>(D, blist, wslot, bfslot);
+        k_emf_edges<<<grid, 128, 0, s>>>(D, blist, wslot, bfslot);
         return;
     }
     /* chunks of edge layers: two rounds of the 296 CTAs that fit (two per
@@ -2211,12 +2168,10 @@ void fx_launch_prolong_groups(const FxDev &D, const FxPop *pops, int np, int slo
     }
 }
 
-void fx_launch_flux_correct(const FxDev &D, const FxCorr *recs, int n, int ncomp, int full, cudaStream_t s)
+void fx_launch_flux_correct(const FxDev &D, const FxCorr *recs, int n, int ncomp, cudaStream_t s)
 {
     if (n <= 0) return;
-    const unsigned grid = fx_blocks(n * ncomp, 256);
-    if (full) k_flux_correct<true><<<grid, 256, 0, s>>>(D, recs, n, ncomp);
-    else k_flux_correct<false><<<grid, 256, 0, s>>>(D, recs, n, ncomp);
+    k_flux_correct<<<fx_blocks(n * ncomp, 256), 256, 0, s>>>(D, recs, n, ncomp);
 }
 
 void fx_launch_emf_correct(const FxDev &D, const FxCorr *recs, int n, cudaStream_t s)

@@ -46,13 +46,13 @@ struct FxDev {
     const FxBlockDev *blk;
     double *W;    /* [b][v][stage][cell]           (WIDX) */
     double *Bf;   /* [b][dir][stage][face]         (FACE_IDX) */
-    double *flux; /* [b][dir][AoSoA nc=nv]         (VIDX) */
-    double *vr;   /* [b][dir][AoSoA nc=3]          (VRIDX) */
-    double *cf;   /* the batched form's face fluxes [b][...] (fx_cf_idx) */
-    /* the batched form's face velocities, normal component only: the
-     * reference's AoSoA tile holds three components of which later phases
-     * read one, and DRAM moves whole tiles */
+    double *cf;   /* face fluxes [b][...]          (fx_cf_idx) */
+    double *cx;   /* the rest of them, MHD         (fx_cx_idx, fx_cx_field) */
+    /* face velocities, the normal component by itself: the reference's AoSoA
+     * tile holds three components of which later phases read one, and DRAM
+     * moves whole tiles */
     double *vn;   /* [b][dir][cell]                (IDX) */
+    double *vt;   /* [b][dir][2][cell], plain form (IDX) */
     double *bv1;  /* [b][dir][cell]                (IDX) */
     double *bv2;
     double *emf;  /* [b][dir][edge]                (EDGE_IDX) */
@@ -206,11 +206,10 @@ cudaError_t fx_prepare_kernels();
 /* launchers (fx_kernels.cu); all asynchronous on `s` */
 void fx_launch_flux(const FxDev &D, const int *blist, int nlist, int ndir, int wslot, int bfslot,
     int full, cudaStream_t s);
-/* full: the plain form (velocities in vr), else the batched one (vn) */
-void fx_launch_emf(const FxDev &D, const int *blist, int nlist, int wslot, int bfslot, int full, cudaStream_t s);
-/* the batched form's face arrays of the listed blocks in the reference's
- * layout (the entries the batched form has) */
-void fx_launch_expand_faces(const FxDev &D, const int *blist, int nlist, cudaStream_t s);
+void fx_launch_emf(const FxDev &D, const int *blist, int nlist, int wslot, int bfslot, cudaStream_t s);
+/* one block's fluxes (nv components) or face velocities (3) of one direction
+ * in the reference's tiles, zero where the block has no face */
+void fx_launch_face_tiles(const FxDev &D, int b, int dir, int velocities, double *out, cudaStream_t s);
 /* stage 1, 2: the RK2 stages; stage 0: an eSSPRK forward-Euler substep in
  * place on slot 0 (prj_timeint_mhd_update_bf stage 0 and the stage-1 cell
  * update writing slot 0) */
@@ -238,14 +237,13 @@ void fx_launch_ghost_wave(const FxDev &D, const FxWave &w, int slot, cudaStream_
 /* gather the listed elements into buf / scatter buf into them */
 void fx_launch_xpack(const FxDev &D, const FxXent *ents, int n, double *buf, int slot, cudaStream_t s);
 void fx_launch_xunpack(const FxDev &D, const FxXent *ents, int n, const double *buf, int slot, cudaStream_t s);
-/* one wave of correction records; ncomp flux components per record */
 /* the dump rows (Data, Eos, optionally Bf) of the listed blocks, packed
  * contiguously per list position */
 void fx_launch_dump_pack(const FxDev &D, const int *blist, int nlist, int faces, double *out, cudaStream_t s);
 /* cell-centred field of the listed blocks' active cells from the faces (slot 0) */
 void fx_launch_cell_field_active(const FxDev &D, const int *blist, int nlist, cudaStream_t s);
-/* full: in the plain form's flux arrays, else the batched form's */
-void fx_launch_flux_correct(const FxDev &D, const FxCorr *recs, int n, int ncomp, int full, cudaStream_t s);
+/* one wave of correction records; ncomp flux components per record */
+void fx_launch_flux_correct(const FxDev &D, const FxCorr *recs, int n, int ncomp, cudaStream_t s);
 void fx_launch_emf_correct(const FxDev &D, const FxCorr *recs, int n, cudaStream_t s);
 void fx_launch_reset_reductions(const FxDev &D, int which, cudaStream_t s);
 /* device-resident driver: dt selection before a step, dt_src clamp and time

@@ -94,7 +94,11 @@ FX_HD int fx_bidx_cell(int nc, int v, int cell)
     return ((row * FX_AOSOA_KT + kk / FX_AOSOA_W) * nc + v) * FX_AOSOA_W + kk % FX_AOSOA_W;
 }
 
-/* Face fluxes of the batched form, [dir][variable 0-5][i][j][k]: the faces of
+/* Face arrays.  Both forms keep theirs in the same four arrays, laid out for
+ * the kernels that read them; a download puts them into the reference's
+ * VIDX / VRIDX tiles.
+ *
+ * cf: fluxes of variables 0-5, [dir][variable][i][j][k]: the faces of
  * the block itself only, in rows of 16 (20 along the sweep direction 2, 17 of
  * them used), so rows start on 32-byte sectors and a variable's plane is
  * read end to end. */
@@ -113,12 +117,55 @@ FX_HD int fx_cf_idx(int dir, int i, int j, int k)
                                              : (i * FX_BS + j) * FX_CF_ROW2 + k);
 }
 
-/* per-block element counts of the stacked device arrays */
+/* cx (MHD): the fluxes no later phase reads.  First variables 0-5 on the
+ * transverse ghost layer of faces that the EMFs need, [dir][variable][s][r]
+ * ([r][s] along direction 2, rows of 20), s along the sweep and r around the
+ * block: the rows at -1 and 16 of the first transverse axis, then the
+ * columns at -1 and 16 of the second.  Then the field components, which the
+ * plain form alone stores, [dir][component][i][j][k] with the ghost layer. */
+#define FX_CX_RING (4 * (FX_BS + 1))
+#define FX_CX_PLANE (FX_CX_RING * (FX_BS + 1))          /* directions 0 and 1 */
+#define FX_CX_PLANE2 (FX_CX_RING * FX_CF_ROW2)
+#define FX_CX_FIELD (12 * FX_CX_PLANE + 6 * FX_CX_PLANE2)
+#define FX_CX_BOX ((FX_BS + 1) * (FX_BS + 2) * (FX_BS + 2))
+#define FX_CX_COUNT (FX_CX_FIELD + 9 * FX_CX_BOX)
+
+FX_HD int fx_cx_plane(int dir) { return dir == 2 ? FX_CX_PLANE2 : FX_CX_PLANE; }
+
+/* variable 0 of a face of the ghost layer */
+FX_HD int fx_cx_idx(int dir, int i, int j, int k)
+{
+    const int s = dir == 0 ? i : dir == 1 ? j : k;
+    const int a = dir == 0 ? j : i, b = dir == 2 ? j : k;
+    const int r = a < 0 ? b + 1 : a == FX_BS ? FX_BS + 3 + b : (b < 0 ? 2 : 3) * FX_BS + 4 + a;
+    return dir * 6 * FX_CX_PLANE + (dir == 2 ? r * FX_CF_ROW2 + s : s * FX_CX_RING + r);
+}
+
+/* field component v (6-8) of a face, ghost layer or not */
+FX_HD int fx_cx_field(int dir, int v, int i, int j, int k)
+{
+    const int ej = dir == 1 ? FX_BS + 1 : FX_BS + 2, ek = dir == 2 ? FX_BS + 1 : FX_BS + 2;
+    return FX_CX_FIELD + (3 * dir + v - 6) * FX_CX_BOX +
+        ((i + (dir != 0)) * ej + j + (dir != 1)) * ek + k + (dir != 2);
+}
+
+/* whether (i, j, k) is a face of direction dir of the block itself (ring 0),
+ * or one of these or of the transverse ghost layer (ring 1) */
+FX_HD bool fx_is_face(int dir, int ring, int i, int j, int k)
+{
+    const int n = FX_BS + 2 * ring;
+    return (dir == 0 ? (unsigned)i < FX_BS + 1u : (unsigned)(i + ring) < (unsigned)n) &&
+        (dir == 1 ? (unsigned)j < FX_BS + 1u : (unsigned)(j + ring) < (unsigned)n) &&
+        (dir == 2 ? (unsigned)k < FX_BS + 1u : (unsigned)(k + ring) < (unsigned)n);
+}
+
+/* per-block element counts of the stacked device arrays: vn the face
+ * velocities along the sweep, [dir][cell], vt the transverse ones (plain
+ * form), [dir][2][cell] with component (dir + 1 + m) % 3 at m */
 #define FX_W_COUNT(nv) ((nv) * FX_NSTAGES * FX_NCELLS)
 #define FX_BF_COUNT (3 * FX_NSTAGES * FX_NFACES)
-#define FX_FLUX_COUNT(nv) (3 * (nv) * FX_NCELLS)
-#define FX_VR_COUNT (3 * 3 * FX_NCELLS)
 #define FX_VN_COUNT (3 * FX_NCELLS)
+#define FX_VT_COUNT (6 * FX_NCELLS)
 #define FX_BV_COUNT (3 * FX_NCELLS)
 #define FX_EMF_COUNT (3 * FX_NEDGES)
 #define FX_EOS_COUNT (3 * FX_NCELLS)

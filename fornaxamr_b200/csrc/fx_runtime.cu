@@ -75,8 +75,8 @@ struct fx_ctx {
     FxDev D{};
 
     FxBlockDev *d_blk = nullptr;
-    double *d_W = nullptr, *d_Bf = nullptr, *d_flux = nullptr, *d_vr = nullptr, *d_vn = nullptr, *d_cf = nullptr;
-    bool compact_faces = false; /* the last face fluxes are the batched form's (cf, vn) */
+    double *d_W = nullptr, *d_Bf = nullptr, *d_cf = nullptr, *d_cx = nullptr, *d_vn = nullptr, *d_vt = nullptr;
+    double *d_tiles = nullptr; /* one direction's face array of one block, for a download (made by the first) */
     double *d_bv1 = nullptr, *d_bv2 = nullptr, *d_emf = nullptr, *d_eos = nullptr;
     double *d_rhs = nullptr, *d_grav = nullptr;
     double *d_W2 = nullptr, *d_Bf2 = nullptr; /* eSSPRK10_4 stage slot 2 */
@@ -272,10 +272,10 @@ void free_mesh(fx_ctx *c)
     cudaFree(c->d_blk);
     cudaFree(c->d_W);
     cudaFree(c->d_Bf);
-    cudaFree(c->d_flux);
-    cudaFree(c->d_vr);
-    cudaFree(c->d_vn);
     cudaFree(c->d_cf);
+    cudaFree(c->d_cx);
+    cudaFree(c->d_vn);
+    cudaFree(c->d_vt);
     cudaFree(c->d_bv1);
     cudaFree(c->d_bv2);
     cudaFree(c->d_emf);
@@ -297,12 +297,11 @@ void free_mesh(fx_ctx *c)
     c->d_pops = nullptr;
     c->d_bops = nullptr;
     c->waves.clear();
-    c->compact_faces = false;
     cudaFree(c->d_fcorr);
     cudaFree(c->d_ecorr);
     for (size_t &cap : c->tab_cap) cap = 0;
     c->d_blk = nullptr;
-    c->d_W = c->d_Bf = c->d_flux = c->d_vr = c->d_vn = c->d_cf = c->d_bv1 = c->d_bv2 = nullptr;
+    c->d_W = c->d_Bf = c->d_cf = c->d_cx = c->d_vn = c->d_vt = c->d_bv1 = c->d_bv2 = nullptr;
     c->d_emf = c->d_eos = c->d_rhs = c->d_grav = nullptr;
     c->d_ids = c->d_active = nullptr;
     c->d_cg = c->d_fg = nullptr;
@@ -436,16 +435,6 @@ void per_block(fx_ctx *c, int form, F &&fn)
     }
 }
 
-/* Face arrays: the batched form keeps its own (compact) ones.  A plain entry
- * point, or a download, after batched stages first gets what they hold in
- * the reference's layout. */
-void expand_faces(fx_ctx *c)
-{
-    if (!c->compact_faces) return;
-    fx_launch_expand_faces(c->D, c->d_active, c->nactive, c->stream);
-    c->compact_faces = false;
-}
-
 /* the whole ghost fill of prj_boundary_fill_ghosts_and_bf: one launch per
  * conflict-free wave of the compiled program (a single launch on
  * single-level meshes) */
@@ -468,14 +457,12 @@ void ghost_fill(fx_ctx *c, int slot)
 }
 
 /* coarse/fine flux corrections (prj_riemann_flux_send), wave by wave;
- * full: the plain form's arrays, every component, else the six the batched
- * form keeps */
-void flux_correct(fx_ctx *c, int full, cudaStream_t s)
+ * ncomp: flux components the face kernel stored */
+void flux_correct(fx_ctx *c, int ncomp, cudaStream_t s)
 {
-    const int ncomp = full ? c->nv : 6;
     const std::vector<int> &wb = c->plan.flux_corr_begin;
     for (size_t w = 0; w + 1 < wb.size(); ++w) {
-        fx_launch_flux_correct(c->D, c->d_fcorr + wb[w], wb[w + 1] - wb[w], ncomp, full, s);
+        fx_launch_flux_correct(c->D, c->d_fcorr + wb[w], wb[w + 1] - wb[w], ncomp, s);
     }
 }
 
@@ -542,15 +529,14 @@ void stage_phases(fx_ctx *c, int form, int wslot, int bfslot, int stage, int dst
     const int full = form == FX_FORM_PLAIN ? 1 : 0;
     lanes_open(c, form);
     per_block(c, form, [&](const int *l, int n, cudaStream_t s) { fx_launch_flux(c->D, l, n, 3, wslot, bfslot, full, s); });
-    c->compact_faces = !full;
     shard_exchange(c, FX_XF, wslot);
     if (!c->plan.flux_corr.empty()) {
         lanes_close(c);
-        flux_correct(c, full, c->stream);
+        flux_correct(c, full ? c->nv : 6, c->stream);
         lanes_open(c, form);
     }
     if (c->cfg.mhd) {
-        per_block(c, form, [&](const int *l, int n, cudaStream_t s) { fx_launch_emf(c->D, l, n, wslot, bfslot, full, s); });
+        per_block(c, form, [&](const int *l, int n, cudaStream_t s) { fx_launch_emf(c->D, l, n, wslot, bfslot, s); });
         shard_exchange(c, FX_XE, wslot);
         if (!c->plan.emf_corr.empty()) {
             lanes_close(c);
@@ -858,14 +844,14 @@ int alloc_block_arrays(fx_ctx *c, int cap, int keep)
     int rc;
     if ((rc = regrow(c, &c->d_blk, 1, cap, keep))) return rc;
     if ((rc = regrow(c, &c->d_W, w_count(c), cap, keep))) return rc;
-    if ((rc = regrow(c, &c->d_flux, (size_t)FX_FLUX_COUNT(c->nv), cap, keep))) return rc;
-    if ((rc = regrow(c, &c->d_vr, (size_t)FX_VR_COUNT, cap, keep))) return rc;
-    if ((rc = regrow(c, &c->d_vn, (size_t)FX_VN_COUNT, cap, keep))) return rc;
     if ((rc = regrow(c, &c->d_cf, (size_t)FX_CF_COUNT, cap, keep))) return rc;
+    if ((rc = regrow(c, &c->d_vn, (size_t)FX_VN_COUNT, cap, keep))) return rc;
+    if ((rc = regrow(c, &c->d_vt, (size_t)FX_VT_COUNT, cap, keep))) return rc;
     if ((rc = regrow(c, &c->d_eos, (size_t)FX_EOS_COUNT, cap, keep))) return rc;
     if ((rc = regrow(c, &c->d_rhs, (size_t)FX_RHS_COUNT(c->nv), cap, keep))) return rc;
     if (c->cfg.mhd) {
         if ((rc = regrow(c, &c->d_Bf, (size_t)FX_BF_COUNT, cap, keep))) return rc;
+        if ((rc = regrow(c, &c->d_cx, (size_t)FX_CX_COUNT, cap, keep))) return rc;
         if ((rc = regrow(c, &c->d_bv1, (size_t)FX_BV_COUNT, cap, keep))) return rc;
         if ((rc = regrow(c, &c->d_bv2, (size_t)FX_BV_COUNT, cap, keep))) return rc;
         if ((rc = regrow(c, &c->d_emf, (size_t)FX_EMF_COUNT, cap, keep))) return rc;
@@ -880,6 +866,27 @@ int alloc_block_arrays(fx_ctx *c, int cap, int keep)
     if ((rc = regrow(c, &c->d_ids, 1, cap, 0))) return rc;
     c->cap = cap;
     return FX_SUCCESS;
+}
+
+/* the kernels' view of the block arrays */
+void point_view(fx_ctx *c)
+{
+    FxDev &D = c->D;
+    D.blk = c->d_blk;
+    D.W = c->d_W;
+    D.Bf = c->d_Bf;
+    D.cf = c->d_cf;
+    D.cx = c->d_cx;
+    D.vn = c->d_vn;
+    D.vt = c->d_vt;
+    D.bv1 = c->d_bv1;
+    D.bv2 = c->d_bv2;
+    D.emf = c->d_emf;
+    D.eos = c->d_eos;
+    D.rhs = c->d_rhs;
+    D.grav = c->d_grav;
+    D.W2 = c->d_W2;
+    D.Bf2 = c->d_Bf2;
 }
 
 /* Uploads the block geometry, the block and active lists and the compiled
@@ -959,21 +966,7 @@ int install_tables(fx_ctx *c)
     /* the host vectors must outlive the copies */
     FX_CUDA(c, cudaStreamSynchronize(s));
     c->D.nblocks = nblocks;
-    c->D.blk = c->d_blk;
-    c->D.W = c->d_W;
-    c->D.Bf = c->d_Bf;
-    c->D.flux = c->d_flux;
-    c->D.vr = c->d_vr;
-    c->D.vn = c->d_vn;
-    c->D.cf = c->d_cf;
-    c->D.bv1 = c->d_bv1;
-    c->D.bv2 = c->d_bv2;
-    c->D.emf = c->d_emf;
-    c->D.eos = c->d_eos;
-    c->D.rhs = c->d_rhs;
-    c->D.grav = c->d_grav;
-    c->D.W2 = c->d_W2;
-    c->D.Bf2 = c->d_Bf2;
+    point_view(c);
     return FX_SUCCESS;
 }
 
@@ -1305,6 +1298,7 @@ void fx_destroy(fx_ctx *c)
     cudaFreeHost(c->h_red);
     cudaFreeHost(c->h_ctl);
     cudaFreeHost(c->h_stage);
+    cudaFree(c->d_tiles);
     for (auto &pair : c->ev_stage) {
         for (cudaEvent_t e : pair) {
             if (e) cudaEventDestroy(e);
@@ -1851,7 +1845,6 @@ int fx_download_array(fx_ctx *c, int b, int which, int dir, double *out)
     const double *src = nullptr;
     size_t count = 0;
     const size_t nv = (size_t)c->nv;
-    if (which == FX_ARR_FLUX || which == FX_ARR_VRIEMANN) expand_faces(c);
     switch (which) {
     case FX_ARR_W: {
         int rc = xfer_w(c, b, 1, out, cudaMemcpyDeviceToHost, false);
@@ -1859,10 +1852,15 @@ int fx_download_array(fx_ctx *c, int b, int which, int dir, double *out)
     }
     case FX_ARR_EOSVAR: src = c->d_eos + (size_t)b * FX_EOS_COUNT; count = FX_EOS_COUNT; break;
     case FX_ARR_RHS: src = c->d_rhs + (size_t)b * FX_RHS_COUNT(nv); count = FX_RHS_COUNT(nv); break;
-    case FX_ARR_FLUX: src = c->d_flux + (size_t)b * FX_FLUX_COUNT(nv) + (size_t)dir * nv * FX_NCELLS;
-        count = nv * FX_NCELLS; break;
-    case FX_ARR_VRIEMANN: src = c->d_vr + (size_t)b * FX_VR_COUNT + (size_t)dir * 3 * FX_NCELLS;
-        count = 3 * FX_NCELLS; break;
+    case FX_ARR_FLUX:
+    case FX_ARR_VRIEMANN: {
+        int rc;
+        if (!c->d_tiles && (rc = dev_alloc(c, &c->d_tiles, nv * FX_NCELLS))) return rc;
+        fx_launch_face_tiles(c->D, b, dir, which == FX_ARR_VRIEMANN, c->d_tiles, c->stream);
+        src = c->d_tiles;
+        count = (which == FX_ARR_FLUX ? nv : 3) * FX_NCELLS;
+        break;
+    }
     case FX_ARR_GRAV:
         if (!c->d_grav) return set_err(c, FX_EINVAL, "no gravity arrays");
         src = c->d_grav + (size_t)b * FX_GRAV_COUNT + (size_t)dir * FX_NCELLS; count = FX_NCELLS; break;
@@ -1904,7 +1902,6 @@ int fx_flux_update(fx_ctx *c, int b, int w_slot, int use_bf1)
     int rc = check_block(c, b);
     if (rc) return rc;
     if (w_slot < 0 || w_slot > 1 || use_bf1 < 0 || use_bf1 > 1) return set_err(c, FX_EINVAL, "bad slot");
-    expand_faces(c);
     fx_launch_set_dt(c->D, 0.0, c->stream);
     fx_launch_flux(c->D, c->d_ids + b, 1, 3, w_slot, use_bf1, 1, c->stream);
     return FX_SUCCESS;
@@ -1916,9 +1913,8 @@ int fx_mhd_update_emf(fx_ctx *c, int b, int stage)
     int rc = check_block(c, b);
     if (rc) return rc;
     if (!c->cfg.mhd || stage < 0 || stage > 1) return set_err(c, FX_EINVAL, "bad emf call");
-    expand_faces(c);
     fx_launch_set_dt(c->D, 0.0, c->stream);
-    fx_launch_emf(c->D, c->d_ids + b, 1, stage, stage, 1, c->stream);
+    fx_launch_emf(c->D, c->d_ids + b, 1, stage, stage, c->stream);
     return FX_SUCCESS;
 }
 
@@ -1939,7 +1935,6 @@ int fx_update_cells(fx_ctx *c, int b, int stage, double dt, double *dt_src)
     int rc = check_block(c, b);
     if (rc) return rc;
     if (stage != 1 && stage != 2) return set_err(c, FX_EINVAL, "bad stage");
-    expand_faces(c);
     fx_launch_set_dt(c->D, dt, c->stream);
     if (dt_src) fx_launch_reset_reductions(c->D, 2, c->stream);
     fx_launch_cell_update(c->D, c->d_ids + b, 1, stage, c->cfg.gravity, 1, 0, c->stream);
@@ -1957,9 +1952,8 @@ int fx_riemann_flux_send(fx_ctx *c)
 {
     if (c && c->nranks > 1) return set_err(c, FX_EINVAL, "%s: not available on a sharded mesh", __func__);
     if (!has_mesh(c)) return c ? set_err(c, FX_ENOMESH, "no mesh") : FX_EINVAL;
-    expand_faces(c);
     fx_launch_set_dt(c->D, 0.0, c->stream);
-    flux_correct(c, 1, c->stream);
+    flux_correct(c, c->nv, c->stream);
     return FX_SUCCESS;
 }
 
@@ -2061,7 +2055,6 @@ int fx_step(fx_ctx *c, int form, double dt, double *dt_src)
     fx_launch_set_dt(c->D, dt, c->stream);
     if (form == FX_FORM_PLAIN && plain_graph(c)) {
         FX_CUDA(c, cudaGraphLaunch(c->g_plain, c->stream));
-        c->compact_faces = false;
         c->last_slot = 0;
     } else if (form == FX_FORM_PLAIN || eager(c)) {
         fx_launch_reset_reductions(c->D, 2, c->stream);
@@ -2070,7 +2063,6 @@ int fx_step(fx_ctx *c, int form, double dt, double *dt_src)
         int rc = build_step_graph(c);
         if (rc) return rc;
         FX_CUDA(c, cudaGraphLaunch(c->g_step, c->stream));
-        c->compact_faces = true;
         c->last_slot = 0;
     }
     shard_min(c, 1, 1);
@@ -2139,7 +2131,6 @@ int fx_run(fx_ctx *c, int form, int nsteps, double cfl, double dt_factor, double
         for (int n = 0; n < nsteps; ++n) {
             FX_CUDA(c, cudaGraphLaunch(c->g_run, c->stream));
         }
-        if (nsteps > 0) c->compact_faces = true;
     }
     c->last_slot = 0;
     FX_CUDA(c, cudaMemcpyAsync(c->h_ctl, c->d_ctl, sizeof(FxCtl), cudaMemcpyDeviceToHost, c->stream));
@@ -2167,7 +2158,7 @@ int fx_time_phase(fx_ctx *c, int phase, int reps, double dt, double *ms)
     auto launch = [&]() {
         switch (phase) {
         case FX_PHASE_FLUX: fx_launch_flux(c->D, c->d_active, c->nactive, 3, 0, 0, 0, s); break;
-        case FX_PHASE_EMF: fx_launch_emf(c->D, c->d_active, c->nactive, 0, 0, 0, s); break;
+        case FX_PHASE_EMF: fx_launch_emf(c->D, c->d_active, c->nactive, 0, 0, s); break;
         case FX_PHASE_CT: fx_launch_bf_update(c->D, c->d_active, c->nactive, 1, s); break;
         case FX_PHASE_CELLS: fx_launch_cell_update(c->D, c->d_active, c->nactive, 1, c->cfg.gravity, 0, 0, s); break;
         case FX_PHASE_GHOST: ghost_fill(c, 1); break;
@@ -2175,7 +2166,6 @@ int fx_time_phase(fx_ctx *c, int phase, int reps, double dt, double *ms)
         }
     };
     fx_launch_set_dt(c->D, dt, s);
-    if (phase == FX_PHASE_FLUX || phase == FX_PHASE_STEP) c->compact_faces = true;
     launch();
     cudaEvent_t e0, e1;
     FX_CUDA(c, cudaEventCreate(&e0));
@@ -2203,7 +2193,6 @@ int fx_autotune(fx_ctx *c, double *times_ms, int n, int *choice)
     FX_CUDA(c, cudaEventCreate(&e0));
     FX_CUDA(c, cudaEventCreate(&e1));
     fx_launch_set_dt(c->D, 0.0, s);
-    c->compact_faces = true;
     int best = 0;
     double best_ms = 1.0e30;
     for (int v = 0; v < FX_FLUX_VARIANTS; ++v) {
@@ -2368,21 +2357,7 @@ int fx_amr_adapt(fx_ctx *c, int *changed)
     if (nb > c->cap) {
         const int grown = std::min(std::max(nb, c->cap + c->cap / 4), capacity);
         if ((rc = alloc_block_arrays(c, grown, c->nblocks))) return rc;
-        c->D.blk = c->d_blk;
-        c->D.W = c->d_W;
-        c->D.Bf = c->d_Bf;
-        c->D.flux = c->d_flux;
-        c->D.vr = c->d_vr;
-    c->D.vn = c->d_vn;
-    c->D.cf = c->d_cf;
-        c->D.bv1 = c->d_bv1;
-        c->D.bv2 = c->d_bv2;
-        c->D.emf = c->d_emf;
-        c->D.eos = c->d_eos;
-        c->D.rhs = c->d_rhs;
-        c->D.grav = c->d_grav;
-        c->D.W2 = c->d_W2;
-        c->D.Bf2 = c->d_Bf2;
+        point_view(c);
     }
     /* geometry of the new block list, read by the data kernels */
     std::vector<FxBlockDev> hb(nb);

@@ -1,6 +1,6 @@
 """The batched form against the plain form on the same uploaded state, bit for
 bit: where the two run different kernels (edge EMFs by marching CTAs against
-one thread per edge; compact face arrays against the reference's tiles), at
+one thread per edge; flux kernels that store more or less), at
 block counts on both sides of each launch rule."""
 import numpy as np
 import pytest
