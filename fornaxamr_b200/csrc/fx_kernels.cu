@@ -170,16 +170,13 @@ __device__ __noinline__ void fx_face_recheck(FxErr *err, const double *q0, const
     }
 }
 
-/* BRM: 0 the solver as it stands; 1 record / 2 replay every face's
- * decisions in D.br_words (FxBrRecord / FxBrReplay; MHD, MC and the plain
- * form only), the branch-frozen map the adjoint checks use */
 /* The faces of one sweep direction: DIR, or blockIdx.y's if DIR is -1.  With a
  * compile-time direction the strides, rotated variables and output planes are
  * immediate offsets, but the kernel holds three copies of the body, run side by
  * side.  Hydro gains (216 blocks 106 -> 92 us); three MHD bodies overrun the
  * instruction cache (512 blocks 503 -> 583 us; with the directions one after
  * the other 525 us, the stencils then read from DRAM three times). */
-template <bool MHD, bool FULL, int TPB, int RECON, int BRM, int DIR, class Br>
+template <bool MHD, bool FULL, bool RING, int TPB, int RECON, int BRM, int DIR, class Br>
 __device__ __forceinline__ void fx_flux_dir(const FxDev &D, const int *__restrict__ blist, int wslot, int bfslot,
     double gL, double gR, Br &br)
 {
@@ -309,7 +306,7 @@ __device__ __forceinline__ void fx_flux_dir(const FxDev &D, const int *__restric
             }
         }
         const bool own = fx_is_face(dir, 0, i, j, k); /* the ghost layer serves the EMFs only */
-        if (FULL || own) {
+        if (RING || own) {
             double *f = own ? D.cf + (size_t)b * FX_CF_COUNT + fx_cf_idx(dir, i, j, k)
                             : D.cx + (size_t)b * FX_CX_COUNT + fx_cx_idx(dir, i, j, k);
             const int plane = own ? fx_cf_plane(dir) : fx_cx_plane(dir);
@@ -367,7 +364,15 @@ __device__ __forceinline__ void fx_flux_dir(const FxDev &D, const int *__restric
     }
 }
 
-template <bool MHD, bool FULL, int TPB, int MINB, int RECON, int BRM = 0>
+/* BRM: 0 the solver as it stands; 1 record / 2 replay every face's
+ * decisions in D.br_words (FxBrRecord / FxBrReplay; MHD, MC and the plain
+ * form only), the branch-frozen map the adjoint checks use.
+ * RING (MHD): the fluxes of the transverse ghost layer are stored too.
+ * Downloads alone read them, and they cost a launch 500 -> 541 us at 512
+ * blocks, so only the last launch of a call has them.  A kernel of its own:
+ * with the store behind a run-time test the launches without it take 522 us,
+ * with both bodies in one kernel a run of 105 blocks 0.8 % longer. */
+template <bool MHD, bool FULL, bool RING, int TPB, int MINB, int RECON, int BRM = 0>
 __global__ void __launch_bounds__(TPB, MINB) k_flux(FxDev D, const int *__restrict__ blist,
     int wslot, int bfslot)
 {
@@ -401,12 +406,12 @@ __global__ void __launch_bounds__(TPB, MINB) k_flux(FxDev D, const int *__restri
         gR = s_gface[1];
     }
     if constexpr (MHD) {
-        fx_flux_dir<MHD, FULL, TPB, RECON, BRM, -1>(D, blist, wslot, bfslot, gL, gR, br);
+        fx_flux_dir<MHD, FULL, RING, TPB, RECON, BRM, -1>(D, blist, wslot, bfslot, gL, gR, br);
     } else {
         switch (blockIdx.y) {
-        case 0: fx_flux_dir<MHD, FULL, TPB, RECON, BRM, 0>(D, blist, wslot, bfslot, gL, gR, br); break;
-        case 1: fx_flux_dir<MHD, FULL, TPB, RECON, BRM, 1>(D, blist, wslot, bfslot, gL, gR, br); break;
-        default: fx_flux_dir<MHD, FULL, TPB, RECON, BRM, 2>(D, blist, wslot, bfslot, gL, gR, br); break;
+        case 0: fx_flux_dir<MHD, FULL, RING, TPB, RECON, BRM, 0>(D, blist, wslot, bfslot, gL, gR, br); break;
+        case 1: fx_flux_dir<MHD, FULL, RING, TPB, RECON, BRM, 1>(D, blist, wslot, bfslot, gL, gR, br); break;
+        default: fx_flux_dir<MHD, FULL, RING, TPB, RECON, BRM, 2>(D, blist, wslot, bfslot, gL, gR, br); break;
         }
     }
 }
@@ -1856,14 +1861,11 @@ static inline unsigned fx_blocks(int n, int tpb) { return (unsigned)((n + tpb - 
 /* launch shapes of the face kernel: {threads per CTA, min CTAs per SM} */
 static const int kFluxShapes[FX_FLUX_VARIANTS][2] = {{64, 9}, {64, 8}, {32, 18}, {128, 5}, {64, 12}, {256, 3}};
 
-template <bool MHD, bool FULL, int TPB, int MINB, int RECON = FX_RECON_MC>
-static void launch_flux_shape(const FxDev &D, const int *blist, int nlist, int ndir, int wslot,
-    int bfslot, cudaStream_t s)
-{
-    const int nf = MHD ? (FX_BS + 1) * (FX_BS + 2) * (FX_BS + 2) : (FX_BS + 1) * FX_BS * FX_BS;
-    const dim3 g(fx_blocks(nf, TPB), ndir, nlist);
-    k_flux<MHD, FULL, TPB, MINB, RECON><<<g, TPB, 0, s>>>(D, blist, wslot, bfslot);
-}
+using FxFluxKernel = void (*)(FxDev, const int *, int, int);
+struct FxFluxLaunch {
+    FxFluxKernel fn;
+    int tpb;
+};
 
 /* the autotuner's launch shapes (threads per CTA, minimum CTAs per SM).
  * Microseconds per launch, MC / WENO-Z3 / hydro MC (512, 216, 216 blocks):
@@ -1872,17 +1874,22 @@ static void launch_flux_shape(const FxDev &D, const int *blist, int nlist, int n
  * 18 warps per SM at 96 registers suit MC; WENO-Z3 with its 54 divisions per
  * face wants the 24 warps of 80 registers; small CTAs leave no half-empty
  * SM behind a slow warp. */
-template <bool MHD, bool FULL, int RECON>
-static void launch_flux_shapes(const FxDev &D, const int *blist, int nlist, int ndir, int wslot,
-    int bfslot, int variant, cudaStream_t s)
+template <bool MHD, bool FULL, bool RING, int RECON>
+static FxFluxLaunch flux_shape(int variant)
 {
-    switch (variant) {
-    case 1: launch_flux_shape<MHD, FULL, 64, 8, RECON>(D, blist, nlist, ndir, wslot, bfslot, s); break;
-    case 2: launch_flux_shape<MHD, FULL, 32, 18, RECON>(D, blist, nlist, ndir, wslot, bfslot, s); break;
-    case 3: launch_flux_shape<MHD, FULL, 128, 5, RECON>(D, blist, nlist, ndir, wslot, bfslot, s); break;
-    case 4: launch_flux_shape<MHD, FULL, 64, 12, RECON>(D, blist, nlist, ndir, wslot, bfslot, s); break;
-    case 5: launch_flux_shape<MHD, FULL, 256, 3, RECON>(D, blist, nlist, ndir, wslot, bfslot, s); break;
-    default: launch_flux_shape<MHD, FULL, 64, 9, RECON>(D, blist, nlist, ndir, wslot, bfslot, s); break;
+    if constexpr (FULL) {
+        /* the plain form's launches hold one block, 258 CTAs of 64: two per
+         * SM whatever the shape allows, so the one that does not spill */
+        return {k_flux<MHD, true, true, 64, 8, RECON>, 64};
+    } else {
+        switch (variant) {
+        case 1: return {k_flux<MHD, false, RING, 64, 8, RECON>, 64};
+        case 2: return {k_flux<MHD, false, RING, 32, 18, RECON>, 32};
+        case 3: return {k_flux<MHD, false, RING, 128, 5, RECON>, 128};
+        case 4: return {k_flux<MHD, false, RING, 64, 12, RECON>, 64};
+        case 5: return {k_flux<MHD, false, RING, 256, 3, RECON>, 256};
+        default: return {k_flux<MHD, false, RING, 64, 9, RECON>, 64};
+        }
     }
 }
 
@@ -1890,62 +1897,38 @@ static void launch_flux_shapes(const FxDev &D, const int *blist, int nlist, int 
  * three cells beyond each face's neighbours and exists in the
  * four-ghost-layer build only (the context rejects it elsewhere); its
  * register demand (about 180 per thread unbounded) makes the shape matter. */
-template <bool MHD, bool FULL>
-static void launch_flux_variant(const FxDev &D, const int *blist, int nlist, int ndir, int wslot,
-    int bfslot, int variant, cudaStream_t s)
+template <bool MHD, bool FULL, bool RING>
+static FxFluxLaunch flux_kernel(const FxDev &D)
 {
-    if constexpr (FULL) {
-        /* the plain form's launches hold one block, 258 CTAs of 64: two per
-         * SM whatever the shape allows, so the one that does not spill */
-        if (D.recon == FX_RECON_WENO3) {
-            launch_flux_shape<MHD, true, 64, 8, FX_RECON_WENO3>(D, blist, nlist, ndir, wslot, bfslot, s);
-            return;
-        }
+    if (D.recon == FX_RECON_WENO3) return flux_shape<MHD, FULL, RING, FX_RECON_WENO3>(D.flux_variant);
 #if FX_NG >= 4
-        if (D.recon == FX_RECON_WENO7) {
-            launch_flux_shape<MHD, true, 64, 8, FX_RECON_WENO7>(D, blist, nlist, ndir, wslot, bfslot, s);
-            return;
-        }
+    if (D.recon == FX_RECON_WENO7) return flux_shape<MHD, FULL, RING, FX_RECON_WENO7>(D.flux_variant);
 #endif
-        launch_flux_shape<MHD, true, 64, 8, FX_RECON_MC>(D, blist, nlist, ndir, wslot, bfslot, s);
-        return;
-    }
-    if (D.recon == FX_RECON_WENO3) {
-        launch_flux_shapes<MHD, FULL, FX_RECON_WENO3>(D, blist, nlist, ndir, wslot, bfslot, variant, s);
-        return;
-    }
-#if FX_NG >= 4
-    if (D.recon == FX_RECON_WENO7) {
-        launch_flux_shapes<MHD, FULL, FX_RECON_WENO7>(D, blist, nlist, ndir, wslot, bfslot, variant, s);
-        return;
-    }
-#endif
-    launch_flux_shapes<MHD, FULL, FX_RECON_MC>(D, blist, nlist, ndir, wslot, bfslot, variant, s);
+    return flux_shape<MHD, FULL, RING, FX_RECON_MC>(D.flux_variant);
 }
+
+static FxFluxLaunch flux_kernel(const FxDev &D, int full, int inner)
+{
+    if (D.nv != 9) return full ? flux_kernel<false, true, false>(D) : flux_kernel<false, false, false>(D);
+    if (full) return flux_kernel<true, true, true>(D);
+    return inner ? flux_kernel<true, false, false>(D) : flux_kernel<true, false, true>(D);
+}
+
+void *fx_flux_function(const FxDev &D, int inner) { return (void *)flux_kernel(D, 0, inner).fn; }
 
 void fx_launch_flux(const FxDev &D, const int *blist, int nlist, int ndir, int wslot, int bfslot,
     int full, cudaStream_t s)
 {
     if (nlist <= 0) return;
+    FxFluxLaunch f = flux_kernel(D, full, D.inner);
     if (D.br_mode != 0 && full && D.nv == 9 && D.recon == FX_RECON_MC) {
         /* the plain form recording or replaying its decisions */
-        constexpr int nf = (FX_BS + 1) * (FX_BS + 2) * (FX_BS + 2);
-        const dim3 g(fx_blocks(nf, 128), ndir, nlist);
-        if (D.br_mode == 1) {
-            k_flux<true, true, 128, 4, FX_RECON_MC, 1><<<g, 128, 0, s>>>(D, blist, wslot, bfslot);
-        } else {
-            k_flux<true, true, 128, 4, FX_RECON_MC, 2><<<g, 128, 0, s>>>(D, blist, wslot, bfslot);
-        }
-        return;
+        f.fn = D.br_mode == 1 ? k_flux<true, true, true, 128, 4, FX_RECON_MC, 1>
+                              : k_flux<true, true, true, 128, 4, FX_RECON_MC, 2>;
+        f.tpb = 128;
     }
-    const int v = D.flux_variant;
-    if (D.nv == 9) {
-        if (full) launch_flux_variant<true, true>(D, blist, nlist, ndir, wslot, bfslot, v, s);
-        else launch_flux_variant<true, false>(D, blist, nlist, ndir, wslot, bfslot, v, s);
-    } else {
-        if (full) launch_flux_variant<false, true>(D, blist, nlist, ndir, wslot, bfslot, v, s);
-        else launch_flux_variant<false, false>(D, blist, nlist, ndir, wslot, bfslot, v, s);
-    }
+    const int nf = D.nv == 9 ? (FX_BS + 1) * (FX_BS + 2) * (FX_BS + 2) : (FX_BS + 1) * FX_BS * FX_BS;
+    f.fn<<<dim3(fx_blocks(nf, f.tpb), ndir, nlist), f.tpb, 0, s>>>(D, blist, wslot, bfslot);
 }
 
 void fx_flux_shape(int variant, int *tpb, int *minb)

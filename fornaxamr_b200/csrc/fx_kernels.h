@@ -71,6 +71,9 @@ struct FxDev {
      * br_edges (likewise per edge, br_eoff); replays count the decisions
      * whose comparison differs from the recorded one in br_flips */
     int br_mode;
+    /* set: a later launch of the same call replaces this one's fluxes, so the
+     * batched form leaves out the ghost layer's (k_flux, RING) */
+    int inner;
     size_t br_off, br_eoff;
     unsigned long long *br_words, *br_edges, *br_flips;
     double *W2;   /* eSSPRK10_4 stage slot 2 of W: [b][v][cell] (null for RK2) */
@@ -206,6 +209,9 @@ cudaError_t fx_prepare_kernels();
 /* launchers (fx_kernels.cu); all asynchronous on `s` */
 void fx_launch_flux(const FxDev &D, const int *blist, int nlist, int ndir, int wslot, int bfslot,
     int full, cudaStream_t s);
+/* the batched form's face kernel for D, with or without `inner`: what a node
+ * of a captured graph is given */
+void *fx_flux_function(const FxDev &D, int inner);
 void fx_launch_emf(const FxDev &D, const int *blist, int nlist, int wslot, int bfslot, cudaStream_t s);
 /* one block's fluxes (nv components) or face velocities (3) of one direction
  * in the reference's tiles, zero where the block has no face */

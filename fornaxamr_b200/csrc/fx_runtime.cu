@@ -114,6 +114,9 @@ struct fx_ctx {
 
     cudaGraphExec_t g_step = nullptr; /* batched RK2 step, dt from the control block */
     cudaGraphExec_t g_run = nullptr;  /* batched driver step (calc_dt + step + dt update) */
+    cudaGraph_t run_graph = nullptr;  /* what g_run was made from (kept for flux_node) */
+    cudaGraphNode_t flux_node = nullptr; /* the face kernel of its last stage */
+    bool run_inner = false;           /* g_run's flux_node leaves out the ghost layer's fluxes */
     cudaGraphExec_t g_plain = nullptr; /* plain step, dt from the control block */
     int plain_steps = 0;              /* plain steps taken launch by launch on this mesh */
     int last_slot = 0;                /* W slot written by the last stage */
@@ -258,6 +261,11 @@ void free_graphs(fx_ctx *c)
     if (c->g_run) {
         cudaGraphExecDestroy(c->g_run);
         c->g_run = nullptr;
+    }
+    if (c->run_graph) {
+        cudaGraphDestroy(c->run_graph);
+        c->run_graph = nullptr;
+        c->flux_node = nullptr;
     }
     if (c->g_plain) {
         cudaGraphExecDestroy(c->g_plain);
@@ -522,6 +530,19 @@ void refill(fx_ctx *c, int form, int slot)
     }
 }
 
+/* remembers the node that the face kernel just launched into a capture of the
+ * context's stream has become */
+void note_flux_node(fx_ctx *c)
+{
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    const cudaGraphNode_t *dep = nullptr;
+    size_t n = 0;
+    if (cudaStreamGetCaptureInfo(c->stream, &st, nullptr, nullptr, &dep, &n) == cudaSuccess &&
+        st == cudaStreamCaptureStatusActive && n == 1) {
+        c->flux_node = dep[0];
+    }
+}
+
 /* the phases of a stage: fluxes and EMFs of W slot wslot and field slot
  * bfslot, the CT and cell updates of `stage`, the fill of slot dst */
 void stage_phases(fx_ctx *c, int form, int wslot, int bfslot, int stage, int dst)
@@ -529,6 +550,7 @@ void stage_phases(fx_ctx *c, int form, int wslot, int bfslot, int stage, int dst
     const int full = form == FX_FORM_PLAIN ? 1 : 0;
     lanes_open(c, form);
     per_block(c, form, [&](const int *l, int n, cudaStream_t s) { fx_launch_flux(c->D, l, n, 3, wslot, bfslot, full, s); });
+    if (c->next_dt && stage == 2 && c->cfg.mhd) note_flux_node(c);
     shard_exchange(c, FX_XF, wslot);
     if (!c->plan.flux_corr.empty()) {
         lanes_close(c);
@@ -604,10 +626,14 @@ void essprk_seq(fx_ctx *c, int form)
 {
     fx_launch_stage_dt(c->D, 6.0, c->stream);
     essprk_save(c, form, 1);
+    c->D.inner = 1;
     for (int n = 0; n < 5; ++n) essprk_substep(c, form);
     essprk_save(c, form, 2);
     essprk_blend(c, form, 1, 3.0 / 5.0);
-    for (int n = 0; n < 5; ++n) essprk_substep(c, form);
+    for (int n = 0; n < 5; ++n) {
+        c->D.inner = n < 4;
+        essprk_substep(c, form);
+    }
     essprk_blend(c, form, 2, 3.0 / 8.0);
     essprk_blend(c, form, 1, 1.0 / 25.0);
     c->last_slot = 0;
@@ -619,7 +645,9 @@ void step_seq(fx_ctx *c, int form)
     if (c->cfg.integrator == FX_INT_ESSPRK10_4) {
         essprk_seq(c, form);
     } else {
+        c->D.inner = 1;
         stage_seq(c, form, 1);
+        c->D.inner = 0;
         stage_seq(c, form, 2);
     }
 }
@@ -707,13 +735,26 @@ int build_run_graph(fx_ctx *c, double cfl)
     if (c->g_run) {
         return FX_SUCCESS;
     }
-    cudaGraph_t g;
+    c->flux_node = nullptr;
     FX_CUDA(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
     run_seq(c, cfl);
-    FX_CUDA(c, cudaStreamEndCapture(c->stream, &g));
-    cudaError_t e = cudaGraphInstantiate(&c->g_run, g, 0);
-    cudaGraphDestroy(g);
-    FX_CUDA(c, e);
+    FX_CUDA(c, cudaStreamEndCapture(c->stream, &c->run_graph));
+    FX_CUDA(c, cudaGraphInstantiate(&c->g_run, c->run_graph, 0));
+    c->run_inner = false;
+    return FX_SUCCESS;
+}
+
+/* Has the run graph's last face kernel store the ghost layer's fluxes or not:
+ * a call's last step has them.  A run of several steps exchanges the node's
+ * kernel twice; that does not show at 8 blocks (2.2 ms per 32 steps). */
+int set_run_inner(fx_ctx *c, bool inner)
+{
+    if (!c->flux_node || c->run_inner == inner) return FX_SUCCESS;
+    cudaKernelNodeParams p{};
+    FX_CUDA(c, cudaGraphKernelNodeGetParams(c->flux_node, &p));
+    p.func = fx_flux_function(c->D, inner);
+    FX_CUDA(c, cudaGraphExecKernelNodeSetParams(c->g_run, c->flux_node, &p));
+    c->run_inner = inner;
     return FX_SUCCESS;
 }
 
@@ -2129,6 +2170,7 @@ int fx_run(fx_ctx *c, int form, int nsteps, double cfl, double dt_factor, double
     } else {
         if ((rc = build_run_graph(c, cfl))) return rc;
         for (int n = 0; n < nsteps; ++n) {
+            if ((rc = set_run_inner(c, n + 1 < nsteps))) return rc;
             FX_CUDA(c, cudaGraphLaunch(c->g_run, c->stream));
         }
     }
@@ -2136,6 +2178,15 @@ int fx_run(fx_ctx *c, int form, int nsteps, double cfl, double dt_factor, double
     FX_CUDA(c, cudaMemcpyAsync(c->h_ctl, c->d_ctl, sizeof(FxCtl), cudaMemcpyDeviceToHost, c->stream));
     rc = sync_and_check(c);
     if (rc) return rc;
+    const double taken = (double)c->h_ctl->step - state[2];
+    if (c->flux_node && taken > 0 && taken < nsteps) {
+        /* the time ran out before the steps did: the last step's second
+         * stage once more for the ghost layer (it read slot 1, which is as
+         * it was) */
+        fx_launch_set_dt(c->D, 0.0, c->stream);
+        fx_launch_flux(c->D, c->d_active, c->nactive, 3, 1, 1, 0, c->stream);
+        flux_correct(c, 6, c->stream);
+    }
     state[0] = c->h_ctl->time;
     state[1] = c->h_ctl->dt_prev;
     state[2] = (double)c->h_ctl->step;
@@ -2166,15 +2217,19 @@ int fx_time_phase(fx_ctx *c, int phase, int reps, double dt, double *ms)
         }
     };
     fx_launch_set_dt(c->D, dt, s);
-    launch();
     cudaEvent_t e0, e1;
     FX_CUDA(c, cudaEventCreate(&e0));
     FX_CUDA(c, cudaEventCreate(&e1));
-    FX_CUDA(c, cudaEventRecord(e0, s));
+    const bool faces = phase == FX_PHASE_FLUX; /* timed as most launches run, once more for every flux there is */
+    c->D.inner = faces;
+    launch();
+    cudaEventRecord(e0, s);
     for (int r = 0; r < reps; ++r) {
         launch();
     }
-    FX_CUDA(c, cudaEventRecord(e1, s));
+    cudaEventRecord(e1, s);
+    c->D.inner = 0;
+    if (faces) launch();
     FX_CUDA(c, cudaEventSynchronize(e1));
     float t = 0.0f;
     FX_CUDA(c, cudaEventElapsedTime(&t, e0, e1));
@@ -2197,12 +2252,14 @@ int fx_autotune(fx_ctx *c, double *times_ms, int n, int *choice)
     double best_ms = 1.0e30;
     for (int v = 0; v < FX_FLUX_VARIANTS; ++v) {
         c->D.flux_variant = v;
+        c->D.inner = 1; /* timed as most launches run */
         fx_launch_flux(c->D, c->d_active, c->nactive, 3, 0, 0, 0, s);
-        FX_CUDA(c, cudaEventRecord(e0, s));
+        cudaEventRecord(e0, s);
         for (int r = 0; r < 3; ++r) {
             fx_launch_flux(c->D, c->d_active, c->nactive, 3, 0, 0, 0, s);
         }
-        FX_CUDA(c, cudaEventRecord(e1, s));
+        cudaEventRecord(e1, s);
+        c->D.inner = 0;
         FX_CUDA(c, cudaEventSynchronize(e1));
         float t = 0.0f;
         FX_CUDA(c, cudaEventElapsedTime(&t, e0, e1));
@@ -2216,6 +2273,7 @@ int fx_autotune(fx_ctx *c, double *times_ms, int n, int *choice)
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     c->D.flux_variant = best;
+    fx_launch_flux(c->D, c->d_active, c->nactive, 3, 0, 0, 0, s); /* every flux there is */
     free_graphs(c); /* captured graphs hold the previous launch shape */
     *choice = best;
     return check_device_error(c);
@@ -2796,7 +2854,9 @@ int fx_adjoint_forward(fx_ctx *c, int nsteps, double dt)
     for (int n = 0; n < nsteps; ++n) {
         for (int stage = 1; stage <= 2; ++stage) {
             fx_launch_set_dt(c->D, dt, s);
+            c->D.inner = n + 1 < nsteps || stage == 1;
             stage_seq(c, FX_FORM_BATCHED, stage);
+            c->D.inner = 0;
             const size_t k = 2 * (size_t)n + stage;
             FX_CUDA(c, cudaMemcpyAsync(c->d_ckW + k * wn, c->d_W, wn * sizeof(double), d2d, s));
             FX_CUDA(c, cudaMemcpyAsync(c->d_ckBf + k * bn, c->d_Bf, bn * sizeof(double), d2d, s));

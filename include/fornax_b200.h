@@ -70,6 +70,9 @@ extern "C" {
 /* block-level array selectors for fx_download_array */
 #define FX_ARR_W 0        /* NHYDRO * 2 * 8000, WIDX */
 #define FX_ARR_EOSVAR 1   /* 3 * 8000, EIDX (AoSoA) */
+/* FLUX: the faces of the block and, MHD, of one transverse ghost layer, zero
+ * elsewhere.  The batched form computes variables 0-5 and the velocity along
+ * dir; the others keep what the last plain step or fx_flux_update left. */
 #define FX_ARR_FLUX 4     /* per dir: NHYDRO * 8000, VIDX (AoSoA) */
 #define FX_ARR_VRIEMANN 5 /* per dir: 3 * 8000, VRIDX (AoSoA) */
 #define FX_ARR_GRAV 6     /* per dir: 8000, IDX */

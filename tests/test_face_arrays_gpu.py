@@ -13,9 +13,13 @@ COORD = (0.0, 1.0, 0.0, 1.0, 0.0, 1.0)
 P, NG, BS = 20, 2, 16
 
 
+def _initial(root):
+    return [np.ascontiguousarray(a) for a in problems.fourier_mhd(mesh.uniform_mesh(root, COORD), nmodes=4, kmax=3)]
+
+
 def _context(root=(2, 2, 4), mhd=True, **kw):
     blocks = mesh.uniform_mesh(root, COORD)
-    W, Bf = problems.fourier_mhd(blocks, nmodes=4, kmax=3)
+    W, Bf = _initial(root)
     if not mhd:
         W, Bf = np.ascontiguousarray(W[:, :6]), None
     ctx = fx.Context(mhd, 5.0 / 3.0, COORD, **kw)
@@ -159,3 +163,103 @@ def test_timed_phases_run_on_the_last_faces(phase, array):
         assert np.array_equal(a, b)
 
 
+def _advance(ctx, form, how):
+    """Ways to the last face fluxes of a call."""
+    dt = 0.2 * ctx.calc_dt(0.4)
+    if how == "step":
+        ctx.step(form, dt)
+        ctx.step(form, dt)
+    elif how == "stage":
+        ctx.stage(form, 1, dt)
+    elif how == "run":
+        a = ctx.run(form, 3, 0.1, 1.2, 1.0e30, (0.0, 0.0, 0))
+        a = ctx.run(form, 1, 0.1, 1.2, 1.0e30, a)
+        ctx.run(form, 2, 0.1, 1.2, 1.0e30, a)
+    else:  # the run ends before its steps are used up
+        a = ctx.run(form, 9, 0.1, 1.2, 5.0 * dt / 2.0, (0.0, 0.0, 0))
+        assert a[0] == 5.0 * dt / 2.0 and a[2] < 9
+
+
+@pytest.mark.parametrize("mhd,integ,how", [(m, i, h) for m in (True, False) for i, h in
+                                           [(fx.INT_RK2, "step"), (fx.INT_RK2, "stage"), (fx.INT_RK2, "run"),
+                                            (fx.INT_RK2, "run to t_end"), (fx.INT_ESSPRK10_4, "step"),
+                                            (fx.INT_ESSPRK10_4, "run")]])
+def test_every_face_of_both_forms_is_the_same(mhd, integ, how):
+    """All of a block's faces, the MHD ghost layer of the transverse axes
+    among them: six components and the normal velocity of the batched form,
+    every component of the plain one; nothing elsewhere."""
+    got = []
+    for form in (fx.FORM_PLAIN, fx.FORM_BATCHED):
+        ctx, n = _context((2, 2, 3), mhd, integrator=integ)
+        _advance(ctx, form, how)
+        got.append(_faces(ctx, n))
+        ctx.close()
+    _same_faces(got[0], got[1], variables=6, normal_only=True)
+    r = 1 if mhd else 0
+    for q, (f, v) in enumerate(got[0]):
+        d = q % 3
+        m = np.zeros((P, P, P), bool)
+        m[tuple(slice(NG, NG + BS + 1) if a == d else slice(NG - r, NG + BS + r) for a in range(3))] = True
+        assert (f[0][m] != 0).mean() > 0.99 and (v[d][m] != 0).mean() > 0.99
+        assert not f[:, ~m].any() and not v[:, ~m].any()
+        if mhd:  # the field flux along the sweep is zero
+            assert [bool(c[m].any()) for c in f[6:]] == [c != d for c in range(3)] and all(c[m].any() for c in v)
+
+
+def test_faces_of_a_run_cut_short_on_three_levels():
+    """With coarse/fine corrections of the fluxes: a run that reaches t_end
+    early, in both forms."""
+    coord = (-0.7, 0.7) * 3
+    blocks = mesh.static_amr_mesh((3,) * 3, coord, 2, mesh.ball_refiner((0.1, 0.05, 0.0), (0.4, 0.2)))
+    desc = mesh.to_desc(blocks)
+    W, Bf = problems.amr_blast(blocks, fx.plan_export(fx.make_config(True, 5.0 / 3.0, coord), desc, 3))
+    act = [b for b in range(len(blocks)) if blocks[b].active == 1][::7]
+    got = []
+    for form in (fx.FORM_PLAIN, fx.FORM_BATCHED):
+        ctx = fx.Context(True, 5.0 / 3.0, coord)
+        ctx.set_mesh(desc)
+        ctx.upload_all(W, Bf)
+        ctx.boundary_fill(1, 0)
+        dt = ctx.calc_dt(0.2)
+        assert ctx.run(form, 9, 0.2, 1.2, 2.5 * dt, (0.0, 0.0, 0))[2] < 9
+        got.append([(ctx.download_array(b, fx.ARR_FLUX, d).reshape(P, P, P // 4, 9, 4)[:, :, :, :6],
+                     ctx.download_array(b, fx.ARR_VRIEMANN, d).reshape(P, P, P // 4, 3, 4)[:, :, :, d])
+                    for b in act for d in range(3)])
+        ctx.close()
+    for (fa, va), (fb, vb) in zip(*got):
+        assert np.array_equal(fa, fb) and np.array_equal(va, vb)
+
+
+def test_a_batched_step_keeps_what_only_the_plain_form_has():
+    """Field fluxes and transverse face velocities of an earlier plain step
+    are still there after a batched one, which does not compute them."""
+    ctx, n = _context()
+    dt = 0.2 * ctx.calc_dt(0.4)
+    ctx.step(fx.FORM_PLAIN, dt)
+    a = _faces(ctx, n)
+    ctx.step(fx.FORM_BATCHED, dt)
+    b = _faces(ctx, n)
+    ctx.close()
+    for q, ((fa, va), (fb, vb)) in enumerate(zip(a, b)):
+        assert np.array_equal(fa[6:], fb[6:])
+        for c in range(3):
+            assert np.array_equal(va[c], vb[c]) == (c != q % 3)
+
+
+@pytest.mark.parametrize("how", ["autotune", "time_phase"])
+def test_timed_face_kernels_leave_every_face(how):
+    """As the flux kernel of the plain form leaves them on the same state."""
+    ctx, n = _context()
+    dt = 0.2 * ctx.calc_dt(0.4)
+    for b in range(n):
+        ctx.flux_update(b, 0, 0)
+    want = _faces(ctx, n)
+    ctx.step(fx.FORM_BATCHED, dt)
+    ctx.upload_all(*_initial((2, 2, 4)))
+    ctx.boundary_fill(1, 0)
+    if how == "autotune":
+        ctx.autotune()
+    else:
+        ctx.time_phase(fx.PHASE_FLUX, 2, dt)
+    _same_faces(_faces(ctx, n), want, variables=6, normal_only=True)
+    ctx.close()
