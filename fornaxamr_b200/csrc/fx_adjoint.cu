@@ -385,28 +385,47 @@ __global__ void __launch_bounds__(256) k_adj_gather(FxAdjDev A, const FxAdjSrc *
     }
 }
 
-__global__ void __launch_bounds__(256) k_adj_zero(FxAdjDev A, const FxGop *__restrict__ cops, int nc,
-    const FxGop *__restrict__ fops, int nf, const FxBop *__restrict__ bops, int nb, int slot)
+/* n neighbouring cells from variable v0 to v1 */
+__device__ __forceinline__ void adj_zero_cells(const FxAdjDev &A, int key, int n, int v0, int v1, int slot)
+{
+    double *d = A.Wb + (size_t)FX_CELL_BLOCK(key) * FX_W_COUNT(9) + (size_t)slot * FX_NCELLS + FX_CELL_IDX(key);
+    for (int v = v0; v <= v1; ++v) {
+        for (int h = 0; h < n; ++h) d[(size_t)v * kPlaneA + h] = 0.0;
+    }
+}
+
+/* the destinations of a wave, from the lists that the fill itself runs */
+__global__ void __launch_bounds__(256) k_adj_zero(FxAdjDev A, FxWave w, int slot)
 {
     int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < nc) {
-        const int key = cops[t].dst;
-        double *d = A.Wb + (size_t)FX_CELL_BLOCK(key) * FX_W_COUNT(9) + (size_t)slot * FX_NCELLS + FX_CELL_IDX(key);
-        for (int v = 0; v < 6; ++v) d[(size_t)v * kPlaneA] = 0.0;
+    if (t < w.ncp) {
+        const int dst = w.cp[t].dst;
+        adj_zero_cells(A, dst & 0x7fffffff, dst < 0 ? 1 : 2, 0, FX_B1 - 1, slot);
         return;
     }
-    t -= nc;
-    if (t < nf) {
-        const FxGop op = fops[t];
+    t -= w.ncp;
+    if (t < w.ncg) {
+        adj_zero_cells(A, w.cg[t].dst, 1, 0, FX_B1 - 1, slot);
+        return;
+    }
+    t -= w.ncg;
+    if (t < w.nfp) {
+        const int dst = w.fp[t].dst;
+        double *d = A.Bfb + ((size_t)((dst & 0x7fffffff) >> 14) * FX_NSTAGES + slot) * FX_NFACES + (dst & 16383);
+        d[0] = 0.0;
+        if (dst >= 0) d[1] = 0.0;
+        return;
+    }
+    t -= w.nfp;
+    if (t < w.nfg) {
+        const FxGop op = w.fg[t];
         A.Bfb[(size_t)(op.dst >> 15) * FX_BF_COUNT + ((size_t)(op.aux & 3) * FX_NSTAGES + slot) * FX_NFACES +
             (op.dst & 32767)] = 0.0;
         return;
     }
-    t -= nf;
-    if (t < nb) {
-        const int key = bops[t].dst;
-        double *d = A.Wb + (size_t)FX_CELL_BLOCK(key) * FX_W_COUNT(9) + (size_t)slot * FX_NCELLS + FX_CELL_IDX(key);
-        for (int v = FX_B1; v <= FX_B3; ++v) d[(size_t)v * kPlaneA] = 0.0;
+    t -= w.nfg;
+    if (t < w.nb) {
+        adj_zero_cells(A, w.b[t].dst, w.b[t].pad, FX_B1, FX_B3, slot);
     }
 }
 
@@ -441,10 +460,9 @@ void fx_launch_adj_gather(const FxAdjDev &A, const FxAdjSrc *csrc, int nc, const
     k_adj_gather<<<adj_blocks(nc + nf, 256), 256, 0, s>>>(A, csrc, nc, fsrc, nf, ents, slot);
 }
 
-void fx_launch_adj_zero(const FxAdjDev &A, const FxGop *cops, int nc, const FxGop *fops, int nf,
-    const FxBop *bops, int nb, int slot, cudaStream_t s)
+void fx_launch_adj_zero(const FxAdjDev &A, const FxWave &w, int slot, cudaStream_t s)
 {
-    const int n = nc + nf + nb;
+    const int n = w.ncp + w.ncg + w.nfp + w.nfg + w.nb;
     if (n <= 0) return;
-    k_adj_zero<<<adj_blocks(n, 256), 256, 0, s>>>(A, cops, nc, fops, nf, bops, nb, slot);
+    k_adj_zero<<<adj_blocks(n, 256), 256, 0, s>>>(A, w, slot);
 }

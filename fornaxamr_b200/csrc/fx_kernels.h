@@ -318,8 +318,7 @@ void fx_launch_adj_gather(const FxAdjDev &A, const FxAdjSrc *csrc, int nc, const
     const FxAdjEnt *ents, int slot, cudaStream_t s);
 /* zero the wave's destinations: cell ops (variables 0-5), face ops, and the
  * field components of cell-field ops */
-void fx_launch_adj_zero(const FxAdjDev &A, const FxGop *cops, int nc, const FxGop *fops, int nf,
-    const FxBop *bops, int nb, int slot, cudaStream_t s);
+void fx_launch_adj_zero(const FxAdjDev &A, const FxWave &w, int slot, cudaStream_t s);
 void fx_launch_adj_cells(const FxAdjDev &A, const int *blist, int nlist, int stage, cudaStream_t s);
 void fx_launch_adj_bf(const FxAdjDev &A, const int *blist, int nlist, int stage, cudaStream_t s);
 void fx_launch_adj_emf(const FxAdjDev &A, const int *blist, int nlist, int stage, cudaStream_t s);

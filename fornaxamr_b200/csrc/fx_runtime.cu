@@ -135,8 +135,6 @@ struct fx_ctx {
     std::vector<int> adj_cbeg, adj_fbeg;
     FxAdjSrc *d_adj_csrc = nullptr, *d_adj_fsrc = nullptr;
     FxAdjEnt *d_adj_ents = nullptr;
-    FxGop *d_adj_cops = nullptr, *d_adj_fops = nullptr; /* the program's operations one by one */
-    FxBop *d_adj_bops = nullptr;
 
     /* decision record / replay of the plain form (fx_branch_trace) */
     unsigned long long *d_br_words = nullptr, *d_br_edges = nullptr;
@@ -321,11 +319,6 @@ void free_mesh(fx_ctx *c)
     cudaFree(c->d_adj_csrc);
     cudaFree(c->d_adj_fsrc);
     cudaFree(c->d_adj_ents);
-    cudaFree(c->d_adj_cops);
-    cudaFree(c->d_adj_fops);
-    cudaFree(c->d_adj_bops);
-    c->d_adj_cops = c->d_adj_fops = nullptr;
-    c->d_adj_bops = nullptr;
     c->d_adj_csrc = c->d_adj_fsrc = nullptr;
     c->d_adj_ents = nullptr;
     c->adj_ghost_ready = false;
@@ -1224,11 +1217,6 @@ void drop_adjoint(fx_ctx *c)
     cudaFree(c->d_adj_csrc);
     cudaFree(c->d_adj_fsrc);
     cudaFree(c->d_adj_ents);
-    cudaFree(c->d_adj_cops);
-    cudaFree(c->d_adj_fops);
-    cudaFree(c->d_adj_bops);
-    c->d_adj_cops = c->d_adj_fops = nullptr;
-    c->d_adj_bops = nullptr;
     cudaFree(c->d_Wb);
     cudaFree(c->d_Bfb);
     cudaFree(c->d_G);
@@ -2684,7 +2672,11 @@ int adj_supported(fx_ctx *c)
     return FX_SUCCESS;
 }
 
-/* the ghost program's waves transposed into gathers (FxAdjSrc / FxAdjEnt) */
+/* The ghost program's waves transposed into gathers (FxAdjSrc / FxAdjEnt):
+ * elements in the order of their keys, each with its readers in program order.
+ * Keys are dense, so readers are counted and put in place (a sort of the 2.5 M
+ * readers of 64 blocks took 105 of the 134 ms of a first adjoint_forward; a
+ * context's first gradient 168 -> 50 ms). */
 int build_adj_ghost(fx_ctx *c)
 {
     if (c->adj_ghost_ready) {
@@ -2695,66 +2687,59 @@ int build_adj_ghost(fx_ctx *c)
     std::vector<FxAdjEnt> ents;
     c->adj_cbeg.assign(1, 0);
     c->adj_fbeg.assign(1, 0);
-    std::vector<std::pair<int64_t, FxAdjEnt>> list;
+    std::vector<int32_t> at; /* per key: its readers' count, then where the next one goes */
+    /* each(f) calls f(key, reader); source(key) names the element */
+    auto transpose = [&](size_t keys, auto each, auto source, std::vector<FxAdjSrc> &out) {
+        at.assign(keys, 0);
+        each([&](size_t key, FxAdjEnt) { ++at[key]; });
+        int32_t n = (int32_t)ents.size();
+        for (size_t key = 0; key < keys; ++key) {
+            const int32_t count = at[key];
+            at[key] = n;
+            if (count == 0) continue;
+            FxAdjSrc sr = source((int32_t)key);
+            sr.begin = n;
+            n += count;
+            sr.end = n;
+            out.push_back(sr);
+        }
+        ents.resize((size_t)n);
+        each([&](size_t key, FxAdjEnt e) { ents[at[key]++] = e; });
+    };
+    const size_t cell_keys = (size_t)c->nblocks << FX_CELL_BITS;
+    const size_t face_keys = (size_t)c->nblocks * 3 * FX_NFACES;
+    auto face_key = [](int32_t key, int d) { return ((size_t)(key >> 15) * 3 + d) * FX_NFACES + (key & 32767); };
     for (int w = 0; w < g.nwaves(); ++w) {
-        list.clear();
-        for (int q = g.cell_begin[w]; q < g.cell_begin[w + 1]; ++q) {
-            const FxGop &op = g.cell_ops[q];
-            int kind = 0;
-            if (op.type == FX_GOP_COPY_NEG) kind = 1 + op.aux;
-            if (op.type == FX_GOP_COPY_USER && op.aux) kind = 16;
-            list.push_back({(int64_t)op.src, FxAdjEnt{op.dst, kind}});
-        }
-        std::stable_sort(list.begin(), list.end(),
-            [](const std::pair<int64_t, FxAdjEnt> &a, const std::pair<int64_t, FxAdjEnt> &b) { return a.first < b.first; });
-        for (size_t q = 0; q < list.size();) {
-            FxAdjSrc sr{(int32_t)list[q].first, 0, (int32_t)ents.size(), 0};
-            while (q < list.size() && list[q].first == sr.key) {
-                ents.push_back(list[q].second);
-                ++q;
+        transpose(cell_keys, [&](auto put) {
+            for (int q = g.cell_begin[w]; q < g.cell_begin[w + 1]; ++q) {
+                const FxGop &op = g.cell_ops[q];
+                int kind = 0;
+                if (op.type == FX_GOP_COPY_NEG) kind = 1 + op.aux;
+                if (op.type == FX_GOP_COPY_USER && op.aux) kind = 16;
+                put((size_t)op.src, FxAdjEnt{op.dst, kind});
             }
-            sr.end = (int32_t)ents.size();
-            cs.push_back(sr);
-        }
+        }, [](int32_t key) { return FxAdjSrc{key, 0, 0, 0}; }, cs);
         c->adj_cbeg.push_back((int)cs.size());
-        list.clear();
-        for (int q = g.face_begin[w]; q < g.face_begin[w + 1]; ++q) {
-            const FxGop &op = g.face_ops[q];
-            list.push_back({((int64_t)op.src << 2) | (op.aux & 3), FxAdjEnt{op.dst, 0}});
-        }
-        for (int q = g.b_begin[w]; q < g.b_begin[w + 1]; ++q) {
-            const FxBop &op = g.b_ops[q];
-            for (int d = 0; d < 3; ++d) {
-                for (int h = 0; h < 2; ++h) {
-                    list.push_back({((int64_t)op.f[2 * d + h] << 2) | d, FxAdjEnt{op.dst, 1 + d}});
-                }
+        transpose(face_keys, [&](auto put) {
+            for (int q = g.face_begin[w]; q < g.face_begin[w + 1]; ++q) {
+                const FxGop &op = g.face_ops[q];
+                put(face_key(op.src, op.aux & 3), FxAdjEnt{op.dst, 0});
             }
-        }
-        std::stable_sort(list.begin(), list.end(),
-            [](const std::pair<int64_t, FxAdjEnt> &a, const std::pair<int64_t, FxAdjEnt> &b) { return a.first < b.first; });
-        for (size_t q = 0; q < list.size();) {
-            const int64_t key = list[q].first;
-            FxAdjSrc sr{(int32_t)(key >> 2), (int32_t)(key & 3), (int32_t)ents.size(), 0};
-            while (q < list.size() && list[q].first == key) {
-                ents.push_back(list[q].second);
-                ++q;
+            for (int q = g.b_begin[w]; q < g.b_begin[w + 1]; ++q) {
+                const FxBop &op = g.b_ops[q];
+                for (int n = 0; n < 6; ++n) put(face_key(op.f[n], n / 2), FxAdjEnt{op.dst, 1 + n / 2});
             }
-            sr.end = (int32_t)ents.size();
-            fs.push_back(sr);
-        }
+        }, [](int32_t key) {
+            const int32_t bd = key / FX_NFACES;
+            return FxAdjSrc{((bd / 3) << 15) | (key % FX_NFACES), bd % 3, 0, 0};
+        }, fs);
         c->adj_fbeg.push_back((int)fs.size());
     }
     int rc;
     if ((rc = dev_alloc(c, &c->d_adj_csrc, cs.size()))) return rc;
     if ((rc = dev_alloc(c, &c->d_adj_fsrc, fs.size()))) return rc;
     if ((rc = dev_alloc(c, &c->d_adj_ents, ents.size()))) return rc;
-    if ((rc = dev_alloc(c, &c->d_adj_cops, g.cell_ops.size()))) return rc;
-    if ((rc = dev_alloc(c, &c->d_adj_fops, g.face_ops.size()))) return rc;
-    if ((rc = dev_alloc(c, &c->d_adj_bops, g.b_ops.size()))) return rc;
     const cudaMemcpyKind h2d = cudaMemcpyHostToDevice;
-    if (!g.cell_ops.empty()) FX_CUDA(c, cudaMemcpyAsync(c->d_adj_cops, g.cell_ops.data(), g.cell_ops.size() * sizeof(FxGop), h2d, c->stream));
-    if (!g.face_ops.empty()) FX_CUDA(c, cudaMemcpyAsync(c->d_adj_fops, g.face_ops.data(), g.face_ops.size() * sizeof(FxGop), h2d, c->stream));
-    if (!g.b_ops.empty()) FX_CUDA(c, cudaMemcpyAsync(c->d_adj_bops, g.b_ops.data(), g.b_ops.size() * sizeof(FxBop), h2d, c->stream));
     if (!cs.empty()) FX_CUDA(c, cudaMemcpyAsync(c->d_adj_csrc, cs.data(), cs.size() * sizeof(FxAdjSrc), h2d, c->stream));
     if (!fs.empty()) FX_CUDA(c, cudaMemcpyAsync(c->d_adj_fsrc, fs.data(), fs.size() * sizeof(FxAdjSrc), h2d, c->stream));
     if (!ents.empty()) FX_CUDA(c, cudaMemcpyAsync(c->d_adj_ents, ents.data(), ents.size() * sizeof(FxAdjEnt), h2d, c->stream));
@@ -2771,9 +2756,7 @@ void adj_ghost(fx_ctx *c, const FxAdjDev &A, int slot)
     for (int w = g.nwaves() - 1; w >= 0; --w) {
         fx_launch_adj_gather(A, c->d_adj_csrc + c->adj_cbeg[w], c->adj_cbeg[w + 1] - c->adj_cbeg[w],
             c->d_adj_fsrc + c->adj_fbeg[w], c->adj_fbeg[w + 1] - c->adj_fbeg[w], c->d_adj_ents, slot, c->stream);
-        fx_launch_adj_zero(A, c->d_adj_cops + g.cell_begin[w], g.cell_begin[w + 1] - g.cell_begin[w],
-            c->d_adj_fops + g.face_begin[w], g.face_begin[w + 1] - g.face_begin[w],
-            c->d_adj_bops + g.b_begin[w], g.b_begin[w + 1] - g.b_begin[w], slot, c->stream);
+        fx_launch_adj_zero(A, c->waves[w], slot, c->stream);
     }
 }
 
