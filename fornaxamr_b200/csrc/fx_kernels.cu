@@ -60,61 +60,6 @@ __device__ __forceinline__ unsigned long long fx_double_key(double d)
 /* ------------------------------------------------------------------------ */
 /* Face fluxes                                                               */
 /* ------------------------------------------------------------------------ */
-/* FULL: store every component the reference stores (the drop-in form);
- * otherwise only what later phases read (hydro flux components, the normal
- * face velocity, Bv1/Bv2).  blockIdx.z is the sweep direction.  TPB/MINB
- * set the launch shape (threads per CTA, resident CTAs per SM the register
- * allocation must allow); the autotuner picks among the compiled shapes. */
-/* left state of the face from cells (qm, q0, q1), right state from (q0,
- * q1, q2): MC slopes (the reference's fast path, prj_flux_recon_var_mc:
- * q +- 0.5 slope) or WENO-Z3 face values (its per-face path,
- * src/prj_flux.c:440-475) */
-/* cells of a face's stencil along the sweep: 4 (cL - 1 .. cR + 1) for MC
- * and WENO-Z3, 8 (cL - 3 .. cR + 3) for WENO-Z7; q[n] is cell cL + n - NS/2 + 1 */
-template <int RECON>
-struct FxStencil {
-    static constexpr int NS = RECON == FX_RECON_WENO7 ? 8 : 4;
-};
-
-template <int RECON>
-__device__ __forceinline__ void fx_recon_pair(const double (&q)[FxStencil<RECON>::NS], double &wl, double &wr)
-{
-    if constexpr (RECON == FX_RECON_WENO7) {
-        /* left state: cells cL-3 .. cL+3 at +1/2; right state: cells cR-3 ..
-         * cR+3 at -1/2, i.e. the mirrored stencil cR+3 .. cR-3 at +1/2 */
-        wl = fx_weno7_plus(q[0], q[1], q[2], q[3], q[4], q[5], q[6]);
-        wr = fx_weno7_plus(q[7], q[6], q[5], q[4], q[3], q[2], q[1]);
-    } else if constexpr (RECON == FX_RECON_WENO3) {
-        wl = fx_weno3_face(q[0], q[1], q[2], 0.5);
-        wr = fx_weno3_face(q[1], q[2], q[3], -0.5);
-    } else {
-        const double d0 = q[1] - q[0], d1 = q[2] - q[1], d2 = q[3] - q[2];
-        wl = q[1] + fx_mc_half(d0, d1);
-        wr = q[2] - fx_mc_half(d1, d2);
-    }
-}
-
-/* the value on one side of a face: the left state's (left) or the right's,
- * read from the stencil's cells at q (first cell) with stride s */
-template <int RECON>
-__device__ __forceinline__ double fx_recon_one(const double *q, int s, bool left)
-{
-    if constexpr (RECON == FX_RECON_WENO7) {
-        const double *p = left ? q : q + 7 * s;
-        const int d = left ? s : -s;
-        return fx_weno7_plus(p[0], p[d], p[2 * d], p[3 * d], p[4 * d], p[5 * d], p[6 * d]);
-    } else {
-        const double *p = left ? q : q + s;
-        const double a = __ldg(p), b = __ldg(p + s), c = __ldg(p + 2 * s);
-        if constexpr (RECON == FX_RECON_WENO3) {
-            return fx_weno3_face(a, b, c, left ? 0.5 : -0.5);
-        } else {
-            const double h = fx_mc_half(b - a, c - b);
-            return left ? b + h : b - h;
-        }
-    }
-}
-
 /* MC face values of a 4-cell stencil with the limiter's selections through
  * a branch policy: bits 4 q + 0 and 4 q + 2 of the face's word */
 template <class BR>
@@ -364,7 +309,12 @@ __device__ __forceinline__ void fx_flux_dir(const FxDev &D, const int *__restric
     }
 }
 
-/* BRM: 0 the solver as it stands; 1 record / 2 replay every face's
+/* FULL: store every component the reference stores (the drop-in form);
+ * otherwise only what later phases read (hydro flux components, the normal
+ * face velocity, Bv1/Bv2).  TPB/MINB set the launch shape (threads per CTA,
+ * resident CTAs per SM the register allocation must allow); the autotuner
+ * picks among the compiled shapes.
+ * BRM: 0 the solver as it stands; 1 record / 2 replay every face's
  * decisions in D.br_words (FxBrRecord / FxBrReplay; MHD, MC and the plain
  * form only), the branch-frozen map the adjoint checks use.
  * RING (MHD): the fluxes of the transverse ghost layer are stored too.
@@ -841,9 +791,6 @@ __global__ void __launch_bounds__(128) k_bf_update(FxDev D, const int *__restric
 /* ------------------------------------------------------------------------ */
 /* Cell update (flux divergence + sources + RK2 combine + cons2prim)         */
 /* ------------------------------------------------------------------------ */
-/* STAGE 1 / 2: the RK2 stages; STAGE 0: the stage-1 arithmetic written in
- * place to slot 0 with the field of Bf slot 0 (an eSSPRK substep,
- * prj_timeint_eSSPRK_step, src/prj_timeint.c:2484-2508) */
 /* a cell's timestep, prj_timeint_calc_dt (src/prj_timeint.c:2144-2256) */
 __device__ __forceinline__ double fx_cell_dt(double cfl, double g, double rho, double eint, double v1, double v2,
     double v3, const FxBlockDev &B)
@@ -854,10 +801,14 @@ __device__ __forceinline__ double fx_cell_dt(double cfl, double g, double rho, d
     return cfl / denom;
 }
 
-/* FULL: the plain form (rhs stored), else the batched one.  DT (the RK2 driver loop): the new state's timestep minimum goes to
- * D.red[0] for the next step, which then needs no pass over the state for it
- * (the ghost fill leaves active cells alone): a step of 8 blocks 68.1 -> 65.1
- * us, of 512 blocks 2025 -> 1983. */
+/* STAGE 1 / 2: the RK2 stages; STAGE 0: the stage-1 arithmetic written in
+ * place to slot 0 with the field of Bf slot 0 (an eSSPRK substep,
+ * prj_timeint_eSSPRK_step, src/prj_timeint.c:2484-2508).
+ * FULL: the plain form (rhs stored), else the batched one.
+ * DT (the RK2 driver loop): the new state's timestep minimum goes to D.red[0]
+ * for the next step, which then needs no pass over the state for it (the ghost
+ * fill leaves active cells alone): a step of 8 blocks 68.1 -> 65.1 us, of 512
+ * blocks 2025 -> 1983. */
 template <bool MHD, int STAGE, bool FULL, bool DT = false>
 __global__ void __launch_bounds__(128) k_cell_update(FxDev D, const int *__restrict__ blist, int gravity)
 {

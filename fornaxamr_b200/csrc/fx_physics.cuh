@@ -22,6 +22,7 @@
 
 #include <cmath>
 
+#include "../../include/fornax_b200.h"
 #include "fx_layout.h"
 
 /* error codes (first error wins); the host maps them to the reference's
@@ -417,6 +418,61 @@ FX_HD double fx_weno7_plus(double q0, double q1, double q2, double q3, double q4
     const double a3 = (4.0 / 35.0) * (1.0 + r3 * r3);
     const double sum = a0 + a1 + a2 + a3;
     return (a0 * p0 + a1 * p1 + a2 * p2 + a3 * p3) / sum;
+}
+
+/* cells of a face's stencil along the sweep: 4 (cL - 1 .. cR + 1) for MC
+ * and WENO-Z3, 8 (cL - 3 .. cR + 3) for WENO-Z7; q[n] is cell cL + n - NS/2 + 1 */
+template <int RECON>
+struct FxStencil {
+    static constexpr int NS = RECON == FX_RECON_WENO7 ? 8 : 4;
+};
+
+/* Both sides of a face: the left state from cells (qm, q0, q1), the right from
+ * (q0, q1, q2): MC slopes (the reference's fast path, prj_flux_recon_var_mc:
+ * q +- 0.5 slope) or WENO-Z3 face values (its per-face path,
+ * src/prj_flux.c:440-475) */
+template <int RECON>
+FX_HD void fx_recon_pair(const double (&q)[FxStencil<RECON>::NS], double &wl, double &wr)
+{
+    if constexpr (RECON == FX_RECON_WENO7) {
+        /* left state: cells cL-3 .. cL+3 at +1/2; right state: cells cR-3 ..
+         * cR+3 at -1/2, i.e. the mirrored stencil cR+3 .. cR-3 at +1/2 */
+        wl = fx_weno7_plus(q[0], q[1], q[2], q[3], q[4], q[5], q[6]);
+        wr = fx_weno7_plus(q[7], q[6], q[5], q[4], q[3], q[2], q[1]);
+    } else if constexpr (RECON == FX_RECON_WENO3) {
+        wl = fx_weno3_face(q[0], q[1], q[2], 0.5);
+        wr = fx_weno3_face(q[1], q[2], q[3], -0.5);
+    } else {
+        const double d0 = q[1] - q[0], d1 = q[2] - q[1], d2 = q[3] - q[2];
+        wl = q[1] + fx_mc_half(d0, d1);
+        wr = q[2] - fx_mc_half(d1, d2);
+    }
+}
+
+/* a load through the read-only data path (device) */
+FX_HD double fx_ldg(const double *p)
+{
+#ifdef __CUDA_ARCH__
+    return __ldg(p);
+#else
+    return *p;
+#endif
+}
+
+/* the WENO value on one side of a face: the left state's (left) or the
+ * right's, read from the stencil's cells at q (first cell) with stride s */
+template <int RECON>
+FX_HD double fx_recon_one(const double *q, int s, bool left)
+{
+    static_assert(RECON == FX_RECON_WENO3 || RECON == FX_RECON_WENO7, "MC takes both sides at once");
+    if constexpr (RECON == FX_RECON_WENO7) {
+        const double *p = left ? q : q + 7 * s;
+        const int d = left ? s : -s;
+        return fx_weno7_plus(p[0], p[d], p[2 * d], p[3 * d], p[4 * d], p[5 * d], p[6 * d]);
+    } else {
+        const double *p = left ? q : q + s;
+        return fx_weno3_face(fx_ldg(p), fx_ldg(p + s), fx_ldg(p + 2 * s), left ? 0.5 : -0.5);
+    }
 }
 
 /* minmod slope of prj_reconstruct_minmod_slope (src/prj_reconstruct.h:46-62) */

@@ -1,6 +1,7 @@
 """The face kernel's solver compiled for the host (tests/face_solver_check.cpp)
 against the plain-C restatement (oracle/fx_oracle.c), bit for bit: halved MC
-slope, HLLD (cheap checks and the checks themselves), HLLC.  No tolerance: the
+slope, one-sided WENO values, HLLD (cheap checks and the checks themselves, one
+side's energy and composition), HLLC.  No tolerance: the
 same IEEE operations on selected operands."""
 import os
 import shutil
