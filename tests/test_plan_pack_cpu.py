@@ -1,6 +1,6 @@
 """The ghost fill's operations as packed for the device (neighbouring copies
-joined to pairs) are the compiled program's, wave by wave: built with the host
-compiler from fornaxamr_b200/csrc/fx_plan.cpp (tests/plan_pack_check.cpp)."""
+joined to pairs) are the compiled program's, wave by wave and in order, and most
+are joined: built with the host compiler from fornaxamr_b200/csrc/fx_plan.cpp (tests/plan_pack_check.cpp)."""
 import os
 import shutil
 import subprocess
@@ -29,14 +29,14 @@ def test_packed_program_holds_the_same_operations(tmp_path):
         "amr": (mesh.static_amr_mesh((2,) * 3, c, 2, mesh.ball_refiner((0.1, 0.05, 0.0), (0.4, 0.2))), True, (0,) * 6),
         "hydro": (mesh.uniform_mesh((5, 1, 2), c), False, (1, 1, 2, 2, 3, 0)),
     }
-    names = []
+    names, joined = [], []
     for name, (blocks, mhd, bc) in meshes.items():
         prefix = str(tmp_path / name)
         with open(prefix + ".cfg", "wb") as f:
             f.write(bytes(fx.make_config(mhd, 5.0 / 3.0, c, bc)))
         with open(prefix + ".desc", "wb") as f:
             f.write(bytes(mesh.to_desc(blocks)))
-        names.append(prefix)
-    r = subprocess.run([exe] + names, capture_output=True, text=True, timeout=600)
+        (joined if name in ("uniform", "amr") else names).append(prefix)
+    r = subprocess.run([exe] + names + ["--"] + joined, capture_output=True, text=True, timeout=600)
     assert r.returncode == 0, r.stdout + r.stderr
     print(r.stdout)
