@@ -11,7 +11,7 @@ One step = one pass of the driver loop: calc_dt, dt limiting, both RK2
 stages with ghost fills, dt_src clamp.  `value` is device time (CUDA events on
 the library's stream, state resident in HBM) for the batched form (every
 phase swept over all blocks, whole step replayed as one CUDA graph).  The
-working set (~2.7 GB) is far larger than L2, so no explicit flush is needed.
+working set (~2.4 GB) is far larger than L2, so no explicit flush is needed.
 `e2e` is the same metric through the C ABI with host buffers: each step
 uploads the state (W and Bf, stage slot 0) from pinned host memory, steps,
 and downloads it again.
@@ -807,11 +807,12 @@ def run_fx(args, rank, world, local_rank):
     alg_bytes = ZONES * BYTES_PER_ZONE_STEP / 2.0
     achieved = alg_bytes / (ms_flux * 1e-3) / 1e9
     # the kernel's own input and output bytes: per direction and block the 8
-    # primitive inputs of the 20 x 18 x 18 stencil cells, and per face the
-    # face field (8 B) plus the outputs later phases read (6 hydro fluxes, the
-    # normal velocity, Bv1, Bv2: 9 doubles)
-    faces = nb * 3 * 17 * 18 * 18
-    kernel_bytes = nb * 3 * 20 * 18 * 18 * 8 * 8 + faces * 8 + faces * 9 * 8
+    # primitive inputs of the 20 x 18 x 18 stencil cells; per face the face
+    # field and the outputs later phases read (normal velocity, Bv1, Bv2: 3
+    # doubles), and per face of the block itself its 6 hydro fluxes (a call's
+    # last launch stores the ghost layer's too)
+    faces, own_faces = nb * 3 * 17 * 18 * 18, nb * 3 * 17 * 16 * 16
+    kernel_bytes = nb * 3 * 20 * 18 * 18 * 8 * 8 + faces * (1 + 3) * 8 + own_faces * 6 * 8
     prof = flux_profile_figures()
     traffic = prof["dram_bytes_per_launch"]
     launches_per_step = ctx.info(0) + 1
@@ -831,7 +832,7 @@ def run_fx(args, rank, world, local_rank):
         "config": {
             "workload": "3D ideal MHD 128^3, 512 blocks of 16^3 + 2 ghosts, gamma 5/3, 32 seeded modes k<=4, "
                         "MC+HLLD+CT RK2, batched form (one CUDA graph per step)",
-            "blocks": nb, "zones": ZONES, "form": "batched", "l2": "working set 2.7 GB >> 126 MB L2 (no flush)",
+            "blocks": nb, "zones": ZONES, "form": "batched", "l2": "working set 2.4 GB >> 126 MB L2 (no flush)",
             "parallelism": f"replicas x{world}",
         },
         "hbm_gbs_step": ZONES * BYTES_PER_ZONE_STEP / (ms_step * 1e-3) / 1e9,
@@ -883,6 +884,11 @@ def main():
 
     if args.impl == "reference":
         if rank != 0:
+            return 0
+        from oracle import ref
+        if not ref.available(True):
+            print(json.dumps({"impl": "reference",
+                              "unavailable": "oracle/_ref holds no reference library and the reference's sources are absent"}))
             return 0
         t0 = time.time()
         cb = cpu_reference(args.steps, args.warmup, args.cpu_seconds)
