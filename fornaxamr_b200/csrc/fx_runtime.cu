@@ -263,8 +263,8 @@ void free_graphs(fx_ctx *c)
     if (c->run_graph) {
         cudaGraphDestroy(c->run_graph);
         c->run_graph = nullptr;
-        c->flux_node = nullptr;
     }
+    c->flux_node = nullptr;
     if (c->g_plain) {
         cudaGraphExecDestroy(c->g_plain);
         c->g_plain = nullptr;
@@ -728,11 +728,12 @@ int build_run_graph(fx_ctx *c, double cfl)
     if (c->g_run) {
         return FX_SUCCESS;
     }
-    c->flux_node = nullptr;
     FX_CUDA(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
     run_seq(c, cfl);
-    FX_CUDA(c, cudaStreamEndCapture(c->stream, &c->run_graph));
-    FX_CUDA(c, cudaGraphInstantiate(&c->g_run, c->run_graph, 0));
+    cudaError_t e = cudaStreamEndCapture(c->stream, &c->run_graph);
+    if (e == cudaSuccess) e = cudaGraphInstantiate(&c->g_run, c->run_graph, 0);
+    if (e != cudaSuccess) free_graphs(c);
+    FX_CUDA(c, e);
     c->run_inner = false;
     return FX_SUCCESS;
 }
