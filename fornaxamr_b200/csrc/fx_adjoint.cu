@@ -385,13 +385,23 @@ __global__ void __launch_bounds__(256) k_adj_gather(FxAdjDev A, const FxAdjSrc *
     }
 }
 
-/* n neighbouring cells from variable v0 to v1 */
-__device__ __forceinline__ void adj_zero_cells(const FxAdjDev &A, int key, int n, int v0, int v1, int slot)
+/* one element or two neighbours; two from an even index in one 16-byte store
+ * (blocks, planes and slots hold even numbers of elements) */
+__device__ __forceinline__ void adj_zero(double *p, int i, bool two)
 {
-    double *d = A.Wb + (size_t)FX_CELL_BLOCK(key) * FX_W_COUNT(9) + (size_t)slot * FX_NCELLS + FX_CELL_IDX(key);
-    for (int v = v0; v <= v1; ++v) {
-        for (int h = 0; h < n; ++h) d[(size_t)v * kPlaneA + h] = 0.0;
+    if (two && (i & 1) == 0) {
+        *reinterpret_cast<double2 *>(p + i) = make_double2(0.0, 0.0);
+    } else {
+        p[i] = 0.0;
+        if (two) p[i + 1] = 0.0;
     }
+}
+
+/* one cell or two neighbours, variables v0 to v1 */
+__device__ __forceinline__ void adj_zero_cells(const FxAdjDev &A, int key, bool two, int v0, int v1, int slot)
+{
+    double *d = A.Wb + (size_t)FX_CELL_BLOCK(key) * FX_W_COUNT(9) + (size_t)slot * FX_NCELLS;
+    for (int v = v0; v <= v1; ++v) adj_zero(d + (size_t)v * kPlaneA, FX_CELL_IDX(key), two);
 }
 
 /* the destinations of a wave, from the lists that the fill itself runs */
@@ -400,20 +410,18 @@ __global__ void __launch_bounds__(256) k_adj_zero(FxAdjDev A, FxWave w, int slot
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < w.ncp) {
         const int dst = w.cp[t].dst;
-        adj_zero_cells(A, dst & 0x7fffffff, dst < 0 ? 1 : 2, 0, FX_B1 - 1, slot);
+        adj_zero_cells(A, dst & 0x7fffffff, dst >= 0, 0, FX_B1 - 1, slot);
         return;
     }
     t -= w.ncp;
     if (t < w.ncg) {
-        adj_zero_cells(A, w.cg[t].dst, 1, 0, FX_B1 - 1, slot);
+        adj_zero_cells(A, w.cg[t].dst, false, 0, FX_B1 - 1, slot);
         return;
     }
     t -= w.ncg;
     if (t < w.nfp) {
         const int dst = w.fp[t].dst;
-        double *d = A.Bfb + ((size_t)((dst & 0x7fffffff) >> 14) * FX_NSTAGES + slot) * FX_NFACES + (dst & 16383);
-        d[0] = 0.0;
-        if (dst >= 0) d[1] = 0.0;
+        adj_zero(A.Bfb + ((size_t)((dst & 0x7fffffff) >> 14) * FX_NSTAGES + slot) * FX_NFACES, dst & 16383, dst >= 0);
         return;
     }
     t -= w.nfp;
@@ -425,7 +433,7 @@ __global__ void __launch_bounds__(256) k_adj_zero(FxAdjDev A, FxWave w, int slot
     }
     t -= w.nfg;
     if (t < w.nb) {
-        adj_zero_cells(A, w.b[t].dst, w.b[t].pad, FX_B1, FX_B3, slot);
+        adj_zero_cells(A, w.b[t].dst, w.b[t].pad == 2, FX_B1, FX_B3, slot);
     }
 }
 
