@@ -1868,10 +1868,10 @@ static FxFluxLaunch flux_kernel(const FxDev &D, int full, int inner)
 void *fx_flux_function(const FxDev &D, int inner) { return (void *)flux_kernel(D, 0, inner).fn; }
 
 void fx_launch_flux(const FxDev &D, const int *blist, int nlist, int ndir, int wslot, int bfslot,
-    int full, cudaStream_t s)
+    int full, int inner, cudaStream_t s)
 {
     if (nlist <= 0) return;
-    FxFluxLaunch f = flux_kernel(D, full, D.inner);
+    FxFluxLaunch f = flux_kernel(D, full, inner);
     if (D.br_mode != 0 && full && D.nv == 9 && D.recon == FX_RECON_MC) {
         /* the plain form recording or replaying its decisions */
         f.fn = D.br_mode == 1 ? k_flux<true, true, true, 128, 4, FX_RECON_MC, 1>

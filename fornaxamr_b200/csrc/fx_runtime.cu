@@ -120,6 +120,7 @@ struct fx_ctx {
     cudaGraphExec_t g_plain = nullptr; /* plain step, dt from the control block */
     int plain_steps = 0;              /* plain steps taken launch by launch on this mesh */
     int last_slot = 0;                /* W slot written by the last stage */
+    int inner = 0;                    /* a later stage of the call replaces the fluxes of the one being issued */
     bool next_dt = false;             /* stage 2 being issued takes the next step's timestep too */
 
     /* discrete adjoint: states after every stage of the last
@@ -542,7 +543,7 @@ void stage_phases(fx_ctx *c, int form, int wslot, int bfslot, int stage, int dst
 {
     const int full = form == FX_FORM_PLAIN ? 1 : 0;
     lanes_open(c, form);
-    per_block(c, form, [&](const int *l, int n, cudaStream_t s) { fx_launch_flux(c->D, l, n, 3, wslot, bfslot, full, s); });
+    per_block(c, form, [&](const int *l, int n, cudaStream_t s) { fx_launch_flux(c->D, l, n, 3, wslot, bfslot, full, c->inner, s); });
     if (c->next_dt && stage == 2 && c->cfg.mhd) note_flux_node(c);
     shard_exchange(c, FX_XF, wslot);
     if (!c->plan.flux_corr.empty()) {
@@ -619,12 +620,12 @@ void essprk_seq(fx_ctx *c, int form)
 {
     fx_launch_stage_dt(c->D, 6.0, c->stream);
     essprk_save(c, form, 1);
-    c->D.inner = 1;
+    c->inner = 1;
     for (int n = 0; n < 5; ++n) essprk_substep(c, form);
     essprk_save(c, form, 2);
     essprk_blend(c, form, 1, 3.0 / 5.0);
     for (int n = 0; n < 5; ++n) {
-        c->D.inner = n < 4;
+        c->inner = n < 4;
         essprk_substep(c, form);
     }
     essprk_blend(c, form, 2, 3.0 / 8.0);
@@ -638,9 +639,9 @@ void step_seq(fx_ctx *c, int form)
     if (c->cfg.integrator == FX_INT_ESSPRK10_4) {
         essprk_seq(c, form);
     } else {
-        c->D.inner = 1;
+        c->inner = 1;
         stage_seq(c, form, 1);
-        c->D.inner = 0;
+        c->inner = 0;
         stage_seq(c, form, 2);
     }
 }
@@ -1933,7 +1934,7 @@ int fx_flux_update(fx_ctx *c, int b, int w_slot, int use_bf1)
     if (rc) return rc;
     if (w_slot < 0 || w_slot > 1 || use_bf1 < 0 || use_bf1 > 1) return set_err(c, FX_EINVAL, "bad slot");
     fx_launch_set_dt(c->D, 0.0, c->stream);
-    fx_launch_flux(c->D, c->d_ids + b, 1, 3, w_slot, use_bf1, 1, c->stream);
+    fx_launch_flux(c->D, c->d_ids + b, 1, 3, w_slot, use_bf1, 1, 0, c->stream);
     return FX_SUCCESS;
 }
 
@@ -2173,7 +2174,7 @@ int fx_run(fx_ctx *c, int form, int nsteps, double cfl, double dt_factor, double
          * stage once more for the ghost layer (it read slot 1, which is as
          * it was) */
         fx_launch_set_dt(c->D, 0.0, c->stream);
-        fx_launch_flux(c->D, c->d_active, c->nactive, 3, 1, 1, 0, c->stream);
+        fx_launch_flux(c->D, c->d_active, c->nactive, 3, 1, 1, 0, 0, c->stream);
         flux_correct(c, 6, c->stream);
     }
     state[0] = c->h_ctl->time;
@@ -2195,9 +2196,10 @@ int fx_time_phase(fx_ctx *c, int phase, int reps, double dt, double *ms)
         if (rc) return rc;
     }
     cudaStream_t s = c->stream;
+    int inner = 0;
     auto launch = [&]() {
         switch (phase) {
-        case FX_PHASE_FLUX: fx_launch_flux(c->D, c->d_active, c->nactive, 3, 0, 0, 0, s); break;
+        case FX_PHASE_FLUX: fx_launch_flux(c->D, c->d_active, c->nactive, 3, 0, 0, 0, inner, s); break;
         case FX_PHASE_EMF: fx_launch_emf(c->D, c->d_active, c->nactive, 0, 0, s); break;
         case FX_PHASE_CT: fx_launch_bf_update(c->D, c->d_active, c->nactive, 1, s); break;
         case FX_PHASE_CELLS: fx_launch_cell_update(c->D, c->d_active, c->nactive, 1, c->cfg.gravity, 0, 0, s); break;
@@ -2210,14 +2212,14 @@ int fx_time_phase(fx_ctx *c, int phase, int reps, double dt, double *ms)
     FX_CUDA(c, cudaEventCreate(&e0));
     FX_CUDA(c, cudaEventCreate(&e1));
     const bool faces = phase == FX_PHASE_FLUX; /* timed as most launches run, once more for every flux there is */
-    c->D.inner = faces;
+    inner = faces;
     launch();
     cudaEventRecord(e0, s);
     for (int r = 0; r < reps; ++r) {
         launch();
     }
     cudaEventRecord(e1, s);
-    c->D.inner = 0;
+    inner = 0;
     if (faces) launch();
     FX_CUDA(c, cudaEventSynchronize(e1));
     float t = 0.0f;
@@ -2241,14 +2243,13 @@ int fx_autotune(fx_ctx *c, double *times_ms, int n, int *choice)
     double best_ms = 1.0e30;
     for (int v = 0; v < FX_FLUX_VARIANTS; ++v) {
         c->D.flux_variant = v;
-        c->D.inner = 1; /* timed as most launches run */
-        fx_launch_flux(c->D, c->d_active, c->nactive, 3, 0, 0, 0, s);
+        /* timed as most launches run */
+        fx_launch_flux(c->D, c->d_active, c->nactive, 3, 0, 0, 0, 1, s);
         cudaEventRecord(e0, s);
         for (int r = 0; r < 3; ++r) {
-            fx_launch_flux(c->D, c->d_active, c->nactive, 3, 0, 0, 0, s);
+            fx_launch_flux(c->D, c->d_active, c->nactive, 3, 0, 0, 0, 1, s);
         }
         cudaEventRecord(e1, s);
-        c->D.inner = 0;
         FX_CUDA(c, cudaEventSynchronize(e1));
         float t = 0.0f;
         FX_CUDA(c, cudaEventElapsedTime(&t, e0, e1));
@@ -2262,7 +2263,7 @@ int fx_autotune(fx_ctx *c, double *times_ms, int n, int *choice)
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     c->D.flux_variant = best;
-    fx_launch_flux(c->D, c->d_active, c->nactive, 3, 0, 0, 0, s); /* every flux there is */
+    fx_launch_flux(c->D, c->d_active, c->nactive, 3, 0, 0, 0, 0, s); /* every flux there is */
     free_graphs(c); /* captured graphs hold the previous launch shape */
     *choice = best;
     return check_device_error(c);
@@ -2838,9 +2839,9 @@ int fx_adjoint_forward(fx_ctx *c, int nsteps, double dt)
     for (int n = 0; n < nsteps; ++n) {
         for (int stage = 1; stage <= 2; ++stage) {
             fx_launch_set_dt(c->D, dt, s);
-            c->D.inner = n + 1 < nsteps || stage == 1;
+            c->inner = n + 1 < nsteps || stage == 1;
             stage_seq(c, FX_FORM_BATCHED, stage);
-            c->D.inner = 0;
+            c->inner = 0;
             const size_t k = 2 * (size_t)n + stage;
             FX_CUDA(c, cudaMemcpyAsync(c->d_ckW + k * wn, c->d_W, wn * sizeof(double), d2d, s));
             FX_CUDA(c, cudaMemcpyAsync(c->d_ckBf + k * bn, c->d_Bf, bn * sizeof(double), d2d, s));
