@@ -1820,11 +1820,11 @@ struct FxFluxLaunch {
 
 /* the autotuner's launch shapes (threads per CTA, minimum CTAs per SM).
  * Microseconds per launch, MC / WENO-Z3 / hydro MC (512, 216, 216 blocks):
- * 64 x 9  521 / 538 / 146    32 x 18  519 / 542 / 144    64 x 8  562 / 602 / 156
- * 128 x 5 553 / 558 / 150    64 x 12  551 / 513 / 150    256 x 3 584 / 503 / 165
- * 18 warps per SM at 96 registers suit MC; WENO-Z3 with its 54 divisions per
- * face wants the 24 warps of 80 registers; small CTAs leave no half-empty
- * SM behind a slow warp. */
+ * 64 x 9  505 / 607 / 101    32 x 18  503 / 612 / 101    64 x 8  535 / 622 / 108
+ * 128 x 5 550 / 592 / 103    64 x 12  534 / 557 / 93     256 x 3 563 / 536 / 97
+ * 18 warps per SM at 96 registers suit MC; WENO-Z3 with 48 divisions per face
+ * in its reconstruction wants the 24 warps of 80 registers; small CTAs leave
+ * no half-empty SM behind a slow warp. */
 template <bool MHD, bool FULL, bool RING, int RECON>
 static FxFluxLaunch flux_shape(int variant)
 {
