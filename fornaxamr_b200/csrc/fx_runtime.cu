@@ -542,8 +542,9 @@ void note_flux_node(fx_ctx *c)
 void stage_phases(fx_ctx *c, int form, int wslot, int bfslot, int stage, int dst)
 {
     const int full = form == FX_FORM_PLAIN ? 1 : 0;
+    const int inner = c->inner || c->nranks > 1; /* a sharded mesh hands out no face arrays */
     lanes_open(c, form);
-    per_block(c, form, [&](const int *l, int n, cudaStream_t s) { fx_launch_flux(c->D, l, n, 3, wslot, bfslot, full, c->inner, s); });
+    per_block(c, form, [&](const int *l, int n, cudaStream_t s) { fx_launch_flux(c->D, l, n, 3, wslot, bfslot, full, inner, s); });
     if (c->next_dt && stage == 2 && c->cfg.mhd) note_flux_node(c);
     shard_exchange(c, FX_XF, wslot);
     if (!c->plan.flux_corr.empty()) {
